@@ -30,14 +30,13 @@ struct FlatNode {
 // Device status bits (DocStats::error and friends).
 constexpr uint32_t OL_DEVERR_TIMEOUT = 1u << 0;   // a bounded wait ran out
 constexpr uint32_t OL_DEVERR_CAPACITY = 1u << 1;  // an output buffer was too small
-constexpr uint32_t OL_DEVERR_FIXUP = 1u << 2;     // fix-up list overflow (cannot happen by construction)
 constexpr uint32_t OL_DEVERR_DEEP = 1u << 3;      // a content line deeper than the fast tree path handles
 
 // Per-launch counters that live in device memory next to a document.
 struct DocStats {
     uint32_t line_count;        // lines in the document
     uint32_t max_content_depth; // deepest non-blank line (saturates at 0xFFFFFFFF)
-    uint32_t fixup_count;       // lines classified by the fix-up kernel
+    uint32_t reserved;
     uint32_t error;             // OL_DEVERR_* bits
     uint32_t pad[12];
 };

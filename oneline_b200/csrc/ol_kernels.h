@@ -20,38 +20,35 @@ constexpr uint32_t kParseHalo = 256;    // bytes staged past a tile
 constexpr uint32_t kTreeTile = 4096;    // lines per tree tile (256 threads x 16)
 constexpr uint32_t kTreeLevels = 32;    // depth levels of the fast tree path
 
+constexpr uint32_t kParseSlotCap = 1024;      // staged lines per tile
+constexpr uint32_t kParseFinishTiles = 1024;  // texts up to this size are finished in one launch (parse_finish_kernel)
+
 struct ParseArgs {
     const uint8_t *text;  // padded: n_tiles * kParseTile + kParseHalo readable bytes
     uint64_t text_len;
     uint32_t n_tiles;
     uint32_t *tile_count;   // n_tiles newline counts (pass 1)
-    uint32_t *tile_base;    // n_tiles exclusive prefix sums (pass 2)
-    DocStats *stats;        // fixup_count/error zeroed before the launch
+    uint32_t *tile_base;    // n_tiles exclusive prefix sums (larger texts)
+    uint32_t *tile_first;   // n_tiles: first newline of the tile (tile-local), or NONE (pass 1)
+    uint16_t *tile_depth;   // 8 per tile: deepest staged content line of each warp (pass 1; unset for a tile that
+                            // did not fit its slot)
+    DocStats *stats;        // reset by pass 1
     uint32_t *offsets;      // line_cap entries
     uint8_t *kinds;
     uint8_t *depth8;        // min(depth, 255)
     uint32_t line_cap;
-    uint2 *fixup;           // (line index, start) of lines longer than the halo
-    uint32_t fixup_cap;
-    // Staged form (nullptr: count pass + recomputing pass): per tile a slot of
-    // slot_cap line words, a flag per tile whose lines did not fit, and the
-    // count and list of those tiles.
-    uint32_t *slot;
-    uint8_t *slot_over;
-    uint32_t *redo_n;
-    uint32_t *redo_list;
-    uint32_t slot_cap;
-    uint32_t first_tile;  // staged pass 1: block b takes tile first_tile + b (launches over tile ranges)
+    uint32_t *slot;         // per tile a slot of slot_cap line words
+    uint8_t *slot_over;     // per tile: more lines than the slot holds
+    uint32_t slot_cap;      // kParseSlotCap
+    uint32_t first_tile;    // pass 1: block b takes tile first_tile + b (launches over tile ranges)
 };
-constexpr uint32_t kParseSlotCap = 1024;  // staged lines per tile
 
 cudaError_t launch_parse(const ParseArgs &a, cudaStream_t st);
-// The staged form in three parts, for a parse that starts while the text is
-// still arriving: begin (reset the redo list), the stage pass over tiles
-// [t0, t1) (any ranges that together cover every tile once, each launched once
-// its tiles and their 256-byte halo are in device memory), then end (the scan,
-// the copy pass, the redo and fix-up passes).
-cudaError_t launch_parse_begin(const ParseArgs &a, cudaStream_t st);
+// The same in two parts, for a parse that starts while the text is still
+// arriving: the stage pass over tiles [t0, t1) (any ranges that together cover
+// every tile once, each launched once its tiles and their 256-byte halo are in
+// device memory), then the passes that write the line arrays. The second part
+// alone, with stats reset, writes them again (into larger arrays).
 cudaError_t launch_parse_tiles(const ParseArgs &a, uint32_t t0, uint32_t t1, cudaStream_t st);
 cudaError_t launch_parse_end(const ParseArgs &a, cudaStream_t st);
 

@@ -1,22 +1,22 @@
 // Kernel (a)+(b): newline scan fused with per-line classification.
 //
-// Staged form (the default), no block ever waits on another:
+// The text is read once and no block ever waits on another:
 //   1. parse_stage_kernel: per 16 KiB tile, the newline count (16-byte
 //      coalesced vector loads, exact byte SWAR, popc, warp scans), the
 //      newline positions in order, and the classification of every line
 //      starting in the tile from shared memory, staged as one word per line
-//      in the tile's slot;
-//   2. scan_columns_kernel: exclusive scan of the tile counts = every tile's
-//      first line index;
-//   3. parse_copy_kernel: one warp per tile writes the staged lines at their
-//      line indices; parse_redo_kernel parses the tiles with more lines than
-//      a slot holds again, in place.
-// The text is read once. The recomputing form (newline_count_kernel, the
-// scan, parse_tiles_kernel) reads it twice and needs no slots. A single pass
-// with a decoupled look-back was measured slower here: the look-back chain
-// fell behind the tile rate. A line that runs past the tile plus a 256-byte
-// halo is queued for a small fix-up kernel, which reads it from global memory
-// once the offsets array is complete.
+//      in the tile's slot; also the tile's first newline and deepest line;
+//   2. the staged lines are written at their line indices:
+//      * up to kParseFinishTiles tiles, parse_finish_kernel, one block per
+//        tile: it sums the counts of the tiles before its own itself and
+//        parses a tile with more lines than a slot holds again, in place;
+//      * larger texts: scan_columns_kernel (every tile's first line index),
+//        parse_copy_kernel (one warp per tile) and parse_redo_kernel (the
+//        tiles with more lines than a slot holds).
+// A single pass with a decoupled look-back was measured slower here: the
+// look-back chain fell behind the tile rate. A line that runs past the tile
+// plus a 256-byte halo (at most one per tile) is classified in step 2 from
+// global memory; it ends at the first newline of the tiles after its own.
 //
 // Replaces crates/oneline-gpu/src/scan.wgsl:20-237 (three passes + a host read
 // of the line count) and shader.wgsl:34-134 (one thread per line, byte loads
@@ -38,6 +38,7 @@ constexpr uint32_t PT_HALO = 256;
 constexpr uint32_t PT_LIST = 1024;                        // newline positions listed per round
 
 static_assert(PT_TILE == kParseTile && PT_HALO == kParseHalo, "tile geometry");
+static_assert(PT_LIST == kParseSlotCap && kParseFinishTiles % PT_THREADS == 0, "slot and finish geometry");
 
 struct ParseSmem {
     alignas(16) uint8_t text[PT_TILE + PT_HALO + 16];  // +16: word reads may run 3 bytes past
@@ -46,12 +47,14 @@ struct ParseSmem {
     uint32_t warp_base[PT_STEPS][8];
     uint32_t halo_first;             // first newline in the halo (local), or NONE
     uint32_t tile_nl;                // newlines in the tile
+    uint32_t long_idx, long_start;   // the line left to classify_long (long_start: tile-local), or NONE
 };
 
 // Staged form: a tile's lines as one word each, (start, kind, depth8) or a
 // marker, in its slot of PT_LIST words.
 constexpr uint32_t kSlotNone = 0xFFFFFFFFu;  // a final '\n' that starts no line
-constexpr uint32_t kSlotFixup = 1u << 26;    // the line runs past the halo: the fix-up kernel classifies it
+constexpr uint32_t kSlotLong = 1u << 26;     // the line runs past the halo: classify_long
+constexpr uint32_t kFirstUnlisted = PT_TILE;  // tile_first of a tile with newlines that were not listed
 __device__ __forceinline__ uint32_t slot_word(uint32_t s, uint32_t kind, uint32_t depth) {
     return s | (kind << 15) | (min(depth, 255u) << 18);  // s <= 16384: 15 bits
 }
@@ -125,46 +128,58 @@ __device__ __forceinline__ void newline_bits(const uint4 &v, uint32_t lo, uint32
     }
 }
 
-// Pass 1: newlines per 16 KiB tile (positions < N).
-__global__ void __launch_bounds__(PT_THREADS) newline_count_kernel(const uint8_t *__restrict__ text, uint64_t N,
-                                                                    uint32_t *__restrict__ counts) {
-    __shared__ uint32_t warp_sum[PT_THREADS / 32];
-    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint64_t t0 = (uint64_t)blockIdx.x * PT_TILE;
-    const uint32_t valid = N - t0 >= PT_TILE ? PT_TILE : (uint32_t)(N - t0);
-    uint4 v[PT_STEPS];
+// The first newline at or past tile t0, or N: the whole warp scans the tiles'
+// first newlines, 256 tiles per round trip.
+__device__ __forceinline__ uint32_t next_newline(const ParseArgs &a, uint32_t t0) {
+    const uint32_t lane = threadIdx.x & 31;
+    for (; t0 < a.n_tiles; t0 += 256) {
+        uint32_t v[8];
 #pragma unroll
-    for (uint32_t k = 0; k < PT_STEPS; k++) v[k] = ld_stream16(text + t0 + k * 4096 + tid * 16);
-    uint32_t c = 0;
+        for (uint32_t i = 0; i < 8; i++) {
+            const uint32_t t = t0 + i * 32 + lane;
+            v[i] = t < a.n_tiles ? a.tile_first[t] : NONE;
+        }
 #pragma unroll
-    for (uint32_t k = 0; k < PT_STEPS; k++) {
-        uint32_t z[4];
-        newline_bits(v[k], k * 4096 + tid * 16, valid, z);
-        c += __popc(z[0]) + __popc(z[1]) + __popc(z[2]) + __popc(z[3]);
+        for (uint32_t i = 0; i < 8; i++) {
+            const uint32_t m = __ballot_sync(0xFFFFFFFFu, v[i] != NONE);
+            if (m) {
+                const uint32_t l = __ffs(m) - 1, first = __shfl_sync(0xFFFFFFFFu, v[i], l);
+                uint32_t at = (t0 + i * 32 + l) * PT_TILE;
+                if (first != kFirstUnlisted) return at + first;
+                for (;; at += 32) {  // ends: the tile has a newline
+                    const uint32_t nl = __ballot_sync(0xFFFFFFFFu, __ldg(a.text + at + lane) == '\n');
+                    if (nl) return at + __ffs(nl) - 1;
+                }
+            }
+        }
     }
-    c = __reduce_add_sync(0xFFFFFFFFu, c);
-    if (lane == 0) warp_sum[warp] = c;
-    __syncthreads();
-    if (tid == 0) {
-        uint32_t t = 0;
-#pragma unroll
-        for (uint32_t w = 0; w < PT_THREADS / 32; w++) t += warp_sum[w];
-        counts[blockIdx.x] = t;
-    }
+    return (uint32_t)a.text_len;
+}
+
+// Line idx, which starts at s in `tile` and runs past the tile's halo: its
+// bytes come from global memory. The whole warp calls; lane 0 classifies.
+__device__ __forceinline__ void classify_long(const ParseArgs &a, uint32_t tile, uint32_t idx, uint32_t s) {
+    const uint32_t e = next_newline(a, tile + 1);
+    if ((threadIdx.x & 31) != 0 || idx >= a.line_cap) return;
+    const uint8_t *t = a.text;
+    const FlatNode nd = classify_line(s, e, [t](uint32_t p) -> uint8_t { return __ldg(t + p); });
+    a.kinds[idx] = (uint8_t)nd.kind;
+    a.depth8[idx] = (uint8_t)min(nd.depth, 255u);
+    if (nd.kind != KIND_BLANK) atomicMax(&a.stats->max_content_depth, nd.depth);
 }
 
 // One tile: the block loads tile b, lists its newlines in position order
 // (warp popc scans) and classifies every line that starts after one of them
 // (plus line 0 for tile 0) from shared memory. Consecutive threads take
 // consecutive lines. A line that runs past the tile plus a 256-byte halo is
-// left to the fix-up kernel.
+// left to classify_long.
 //   STAGE: the tile's newline count goes to tile_count and its lines, by
 //     tile-local rank, to its slot (a tile with more lines than a slot holds
-//     is listed for the recomputing form instead);
-//   else: the tile's first line index comes from tile_base (the scan of the
-//     counts), and offsets, kinds and depth8 are written in place.
+//     is flagged for the other form instead);
+//   else: nl_base newlines come before the tile, and offsets, kinds and
+//     depth8 are written in place.
 template <bool STAGE>
-__device__ __forceinline__ void parse_tile(const ParseArgs &a, ParseSmem &sm, uint32_t tile) {
+__device__ __forceinline__ void parse_tile(const ParseArgs &a, ParseSmem &sm, uint32_t tile, uint32_t nl_base) {
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint64_t t0 = (uint64_t)tile * PT_TILE;
     const uint64_t N = a.text_len;
@@ -179,6 +194,7 @@ __device__ __forceinline__ void parse_tile(const ParseArgs &a, ParseSmem &sm, ui
     if (tid < PT_HALO / 16) vh = ld_stream16(a.text + t0 + PT_TILE + tid * 16);
     if (tid == 0) {
         sm.halo_first = NONE;
+        sm.long_idx = NONE;
         *reinterpret_cast<uint4 *>(&sm.text[PT_TILE + PT_HALO]) = make_uint4(0, 0, 0, 0);
     }
 #pragma unroll
@@ -240,24 +256,17 @@ __device__ __forceinline__ void parse_tile(const ParseArgs &a, ParseSmem &sm, ui
     __syncthreads();  // (b) bases and halo_first visible
 
     const uint32_t off = tile == 0 ? 1u : 0u;
-    uint32_t nl_base, n_nl;
+    const uint32_t n_nl = sm.tile_nl;
+    const uint32_t n_lines = n_nl + off;
     if (STAGE) {
-        n_nl = sm.tile_nl;
-        nl_base = 0;
-        const bool over = n_nl + off > a.slot_cap;
+        const bool over = n_lines > a.slot_cap;
         if (tid == 0) {
             a.tile_count[tile] = n_nl;
             a.slot_over[tile] = over ? 1 : 0;
-            if (over) a.redo_list[atomicAdd(a.redo_n, 1u)] = tile;
+            if (over || n_lines == 0) a.tile_first[tile] = over ? kFirstUnlisted : NONE;
         }
         if (over) return;  // uniform
-    } else {
-        nl_base = a.tile_base[tile];  // newlines before this tile
-        n_nl = a.tile_count[tile];
-        if (tile == a.n_tiles - 1 && tid == 0)  // L = 1 + newlines before the last byte
-            a.stats->line_count = 1u + nl_base + n_nl - (a.text[N - 1] == '\n');
     }
-    const uint32_t n_lines = n_nl + off;
     const uint32_t halo_first = sm.halo_first;
     uint32_t *slot = STAGE ? a.slot + (size_t)tile * a.slot_cap : nullptr;
     uint32_t my_max = 0;
@@ -283,6 +292,7 @@ __device__ __forceinline__ void parse_tile(const ParseArgs &a, ParseSmem &sm, ui
             }
         }
         __syncthreads();  // (c) list ready
+        if (STAGE && tid == 0) a.tile_first[tile] = n_nl ? sm.nl[0] : NONE;
 
         const uint32_t r_end = min(n_lines, r0 + PT_LIST);
         for (uint32_t j = r0 + tid; j < r_end; j += PT_THREADS) {
@@ -305,13 +315,12 @@ __device__ __forceinline__ void parse_tile(const ParseArgs &a, ParseSmem &sm, ui
             else if (halo_first != NONE) e = halo_first;
             else if (valid < PT_TILE + PT_HALO) e = valid;  // the text ends in the staged bytes
             else {
-                // runs past the halo: classified by the fix-up kernel
+                // runs past the halo (the tile's last line)
                 if (STAGE) {
-                    slot[j] = s | kSlotFixup;
+                    slot[j] = s | kSlotLong;
                 } else {
-                    uint32_t fx = atomicAdd(&a.stats->fixup_count, 1u);
-                    if (fx < a.fixup_cap) a.fixup[fx] = make_uint2(idx, (uint32_t)t0 + s);
-                    else atomicOr(&a.stats->error, OL_DEVERR_FIXUP);
+                    sm.long_idx = idx;
+                    sm.long_start = s;
                 }
                 continue;
             }
@@ -327,106 +336,169 @@ __device__ __forceinline__ void parse_tile(const ParseArgs &a, ParseSmem &sm, ui
         }
         __syncthreads();  // (d) the next round may overwrite the list
     }
-    for (int o = 16; o > 0; o >>= 1) my_max = max(my_max, __shfl_xor_sync(0xFFFFFFFFu, my_max, o));
-    if (lane == 0 && my_max) atomicMax(&a.stats->max_content_depth, my_max);
-}
-
-// Recomputing form, every tile (pass 3 after newline_count_kernel and the scan).
-__global__ void __launch_bounds__(PT_THREADS, 6) parse_tiles_kernel(ParseArgs a) {
-    __shared__ ParseSmem sm;
-    parse_tile<false>(a, sm, blockIdx.x);
-}
-
-// Staged form, pass 1: every tile counts its newlines and stages its lines.
-// Block b first asks L2 to prefetch the tile kPrefetchTilesAhead further on
-// (when this launch covers it), which a block that starts soon will read.
-__global__ void __launch_bounds__(PT_THREADS, 6) parse_stage_kernel(ParseArgs a) {
-    __shared__ ParseSmem sm;
-    if (threadIdx.x == 0 && blockIdx.x + kPrefetchTilesAhead < gridDim.x)  // inside this launch's tiles
-        prefetch_l2(a.text + (uint64_t)(a.first_tile + blockIdx.x + kPrefetchTilesAhead) * kParseTile, kParseTile);
-    parse_tile<true>(a, sm, a.first_tile + blockIdx.x);
-}
-
-// Staged form, pass 3: the tiles listed by pass 1 (more lines than a slot
-// holds) in the recomputing form, now that their first line index is known.
-__global__ void __launch_bounds__(PT_THREADS, 6) parse_redo_kernel(ParseArgs a) {
-    __shared__ ParseSmem sm;
-    const uint32_t n = *a.redo_n;
-    for (uint32_t i = blockIdx.x; i < n; i += gridDim.x) {
-        parse_tile<false>(a, sm, a.redo_list[i]);
-        __syncthreads();  // shared memory is reused by the next tile
+    my_max = __reduce_max_sync(0xFFFFFFFFu, my_max);
+    if (STAGE) {
+        if (lane == 0) a.tile_depth[tile * 8 + warp] = (uint16_t)my_max;  // at most the staged bytes: below 2^16
+    } else {
+        if (warp == 0 && sm.long_idx != NONE) classify_long(a, tile, sm.long_idx, (uint32_t)t0 + sm.long_start);
+        if (lane == 0 && my_max) atomicMax(&a.stats->max_content_depth, my_max);
     }
 }
 
-// Staged form, pass 2: one warp per tile writes its staged lines at their
-// line indices (the scan of the counts): offsets, kinds and depth8, or a
-// fix-up entry for a line that runs past the halo.
-constexpr uint32_t PC_TILES = 8;  // tiles per block
+// Pass 1: every tile counts its newlines and stages its lines; the block of
+// tile 0 resets the document's counters, which only pass 2 adds to. Block b
+// first asks L2 to prefetch the tile kPrefetchTilesAhead further on (when this
+// launch covers it), which a block that starts soon will read.
+__global__ void __launch_bounds__(PT_THREADS, 6) parse_stage_kernel(ParseArgs a) {
+    __shared__ ParseSmem sm;
+    const uint32_t tile = a.first_tile + blockIdx.x;
+    if (threadIdx.x == 0 && blockIdx.x + kPrefetchTilesAhead < gridDim.x)  // inside this launch's tiles
+        prefetch_l2(a.text + (uint64_t)(tile + kPrefetchTilesAhead) * kParseTile, kParseTile);
+    if (tile == 0 && threadIdx.x < sizeof(DocStats) / 4) reinterpret_cast<uint32_t *>(a.stats)[threadIdx.x] = 0;
+    parse_tile<true>(a, sm, tile, 0);
+}
+
+// A staged line word at line index idx: offsets, kinds and depth8. A long line
+// (kSlotLong) is left to the caller, which gets its start in `at`.
+__device__ __forceinline__ void put_line(const ParseArgs &a, uint32_t t0, uint32_t w, uint32_t idx, uint2 &at) {
+    if (w == kSlotNone) return;
+    if (idx >= a.line_cap) {
+        atomicOr(&a.stats->error, OL_DEVERR_CAPACITY);
+        return;
+    }
+    const uint32_t s = t0 + (w & 0x7FFFu);
+    a.offsets[idx] = s;
+    if (w & kSlotLong) {
+        at = make_uint2(idx, s);
+        return;
+    }
+    a.kinds[idx] = (uint8_t)((w >> 15) & 7u);
+    a.depth8[idx] = (uint8_t)((w >> 18) & 0xFFu);
+}
+
+// The deepest staged line of a tile.
+__device__ __forceinline__ uint32_t tile_depth_of(const ParseArgs &a, uint32_t tile) {
+    const uint4 d = reinterpret_cast<const uint4 *>(a.tile_depth)[tile];
+    const uint32_t m = __vmaxu2(__vmaxu2(d.x, d.y), __vmaxu2(d.z, d.w));
+    return max(m & 0xFFFFu, m >> 16);
+}
+
+// L = 1 + newlines before the last byte, from the last tile's.
+__device__ __forceinline__ void put_line_count(const ParseArgs &a, uint32_t nl_base, uint32_t n_nl) {
+    a.stats->line_count = 1u + nl_base + n_nl - (a.text[a.text_len - 1] == '\n');
+}
+
+// Pass 2 of a text of at most kParseFinishTiles tiles, block b for tile b. The
+// counts before it are at most 4 KiB of L2 reads, all in flight at once, so
+// the scan needs no launch of its own, nor do the dense tiles and long lines:
+// two launches for the whole parse instead of five. At 1 MiB (64 tiles) the
+// passes after the stage pass took 14.6 us of kernels and four launches of
+// 3.9 us each on the host.
+__global__ void __launch_bounds__(PT_THREADS, 6) parse_finish_kernel(ParseArgs a) {
+    __shared__ ParseSmem sm;
+    __shared__ uint32_t warp_sum[PT_THREADS / 32];
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tile = blockIdx.x;
+    uint32_t before = 0;
+#pragma unroll
+    for (uint32_t i = 0; i < kParseFinishTiles / PT_THREADS; i++) {
+        const uint32_t t = i * PT_THREADS + tid;
+        before += t < tile ? a.tile_count[t] : 0u;
+    }
+    const bool over = a.slot_over[tile];
+    const uint32_t depth = tile_depth_of(a, tile);
+    const uint32_t off = tile == 0 ? 1u : 0u, n_nl = a.tile_count[tile], n_lines = n_nl + off;
+    const uint32_t *slot = a.slot + (size_t)tile * a.slot_cap;
+    uint32_t ws[kParseSlotCap / PT_THREADS];
+#pragma unroll
+    for (uint32_t r = 0; r < kParseSlotCap / PT_THREADS; r++) {
+        const uint32_t j = r * PT_THREADS + tid;
+        ws[r] = !over && j < n_lines ? slot[j] : kSlotNone;
+    }
+    before = __reduce_add_sync(0xFFFFFFFFu, before);
+    if (lane == 0) warp_sum[warp] = before;
+    __syncthreads();
+    uint32_t nl_base = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < PT_THREADS / 32; w++) nl_base += warp_sum[w];
+    if (tid == 0 && tile == a.n_tiles - 1) put_line_count(a, nl_base, n_nl);
+    if (over) {  // uniform: more lines than the slot holds
+        parse_tile<false>(a, sm, tile, nl_base);
+        return;
+    }
+    if (tid == 0 && depth) atomicMax(&a.stats->max_content_depth, depth);
+    uint2 at = make_uint2(NONE, 0);
+#pragma unroll
+    for (uint32_t r = 0; r < kParseSlotCap / PT_THREADS; r++)
+        put_line(a, tile * PT_TILE, ws[r], nl_base + r * PT_THREADS + tid + 1 - off, at);
+    const uint32_t m = __ballot_sync(0xFFFFFFFFu, at.x != NONE);
+    if (m) {
+        const uint32_t l = __ffs(m) - 1;
+        classify_long(a, tile, __shfl_sync(0xFFFFFFFFu, at.x, l), __shfl_sync(0xFFFFFFFFu, at.y, l));
+    }
+}
+
+// Pass 2 of a larger text, after the scan of the counts: one warp per tile.
+constexpr uint32_t PC_TILES = 8;    // tiles per block
+constexpr uint32_t PC_FLIGHT = 4;   // 12 (one round trip a tile) measured 62 against 54 us per GiB
 __global__ void __launch_bounds__(256) parse_copy_kernel(ParseArgs a) {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t tile = blockIdx.x * PC_TILES + (threadIdx.x >> 5);
-    if (tile >= a.n_tiles || a.slot_over[tile]) return;
+    if (tile >= a.n_tiles) return;
     const uint32_t off = tile == 0 ? 1u : 0u;
     const uint32_t n_nl = a.tile_count[tile], nl_base = a.tile_base[tile];
     const uint32_t n_lines = n_nl + off;
-    const uint32_t t0 = tile * PT_TILE;
-    if (tile == a.n_tiles - 1 && lane == 0)  // L = 1 + newlines before the last byte
-        a.stats->line_count = 1u + nl_base + n_nl - (a.text[a.text_len - 1] == '\n');
+    if (tile == a.n_tiles - 1 && lane == 0) put_line_count(a, nl_base, n_nl);
+    if (a.slot_over[tile]) return;  // parse_redo_kernel
     const uint32_t *slot = a.slot + (size_t)tile * a.slot_cap;
-    for (uint32_t j0 = 0; j0 < n_lines; j0 += 128) {
-        uint32_t ws[4];  // four independent loads in flight per lane
+    uint2 at = make_uint2(NONE, 0);
+    for (uint32_t j0 = 0; j0 < n_lines; j0 += PC_FLIGHT * 32) {
+        uint32_t ws[PC_FLIGHT];  // independent loads in flight per lane
 #pragma unroll
-        for (uint32_t r = 0; r < 4; r++) {
+        for (uint32_t r = 0; r < PC_FLIGHT; r++) {
             const uint32_t j = j0 + r * 32 + lane;
             ws[r] = j < n_lines ? __ldg(slot + j) : kSlotNone;
         }
 #pragma unroll
-        for (uint32_t r = 0; r < 4; r++) {
-            const uint32_t j = j0 + r * 32 + lane;
-            const uint32_t w = ws[r];
-            if (w == kSlotNone) continue;
-            const uint32_t idx = nl_base + j + 1 - off;
-            if (idx >= a.line_cap) {
-                atomicOr(&a.stats->error, OL_DEVERR_CAPACITY);
-                continue;
-            }
-            const uint32_t s = t0 + (w & 0x7FFFu);
-            a.offsets[idx] = s;
-            if (w & kSlotFixup) {
-                const uint32_t fx = atomicAdd(&a.stats->fixup_count, 1u);
-                if (fx < a.fixup_cap) a.fixup[fx] = make_uint2(idx, s);
-                else atomicOr(&a.stats->error, OL_DEVERR_FIXUP);
-                continue;
-            }
-            a.kinds[idx] = (uint8_t)((w >> 15) & 7u);
-            a.depth8[idx] = (uint8_t)((w >> 18) & 0xFFu);
-        }
+        for (uint32_t r = 0; r < PC_FLIGHT; r++)
+            put_line(a, tile * PT_TILE, ws[r], nl_base + j0 + r * 32 + lane + 1 - off, at);
+    }
+    const uint32_t m = __ballot_sync(0xFFFFFFFFu, at.x != NONE);
+    if (m) {
+        const uint32_t l = __ffs(m) - 1;
+        classify_long(a, tile, __shfl_sync(0xFFFFFFFFu, at.x, l), __shfl_sync(0xFFFFFFFFu, at.y, l));
     }
 }
 
-// Lines queued by the tile kernel: their end comes from the complete offsets
-// array, their bytes from global memory. One warp per line (lane 0 works).
-__global__ void parse_fixup_kernel(ParseArgs a) {
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-    const uint32_t count = min(a.stats->fixup_count, a.fixup_cap);
-    const uint32_t L = a.stats->line_count;
-    if (L > a.line_cap) return;  // outputs overflowed: the host re-runs with room for L lines
-    const uint64_t N = a.text_len;
-    const uint32_t last_end = a.text[N - 1] == '\n' ? (uint32_t)(N - 1) : (uint32_t)N;
-    for (uint32_t i = gw; i < count; i += nw) {
-        if (lane != 0) continue;
-        uint2 f = a.fixup[i];
-        uint32_t idx = f.x, s = f.y;
-        uint32_t e = idx + 1 < L ? a.offsets[idx + 1] - 1 : last_end;
-        const uint8_t *t = a.text;
-        FlatNode nd = classify_line(s, e, [t](uint32_t p) -> uint8_t { return __ldg(t + p); });
-        if (idx >= a.line_cap) continue;
-        a.kinds[idx] = (uint8_t)nd.kind;
-        a.depth8[idx] = (uint8_t)min(nd.depth, 255u);
-        if (nd.kind != KIND_BLANK) atomicMax(&a.stats->max_content_depth, nd.depth);
+// Pass 3 of a larger text: the tiles with more lines than a slot holds, parsed
+// again in place now that their first line index is known, and the document's
+// deepest line. Block b looks through tiles b, b + grid, ...: one atomic a
+// block. (One a warp and tile of the stage pass, all on one address, made that
+// pass 438 us per GiB in some processes and 704 us in others, on one box; it
+// now takes 457 us in all.)
+__global__ void __launch_bounds__(PT_THREADS, 6) parse_redo_kernel(ParseArgs a) {
+    __shared__ ParseSmem sm;
+    __shared__ uint32_t list[PT_THREADS], n_list, deepest;
+    if (threadIdx.x == 0) deepest = 0;
+    uint32_t depth = 0;
+    for (uint32_t i0 = blockIdx.x; i0 < a.n_tiles; i0 += gridDim.x * PT_THREADS) {
+        if (threadIdx.x == 0) n_list = 0;
+        __syncthreads();
+        const uint64_t tile = i0 + (uint64_t)gridDim.x * threadIdx.x;
+        if (tile < a.n_tiles) {
+            if (a.slot_over[tile]) list[atomicAdd(&n_list, 1u)] = (uint32_t)tile;
+            else depth = max(depth, tile_depth_of(a, (uint32_t)tile));
+        }
+        __syncthreads();
+        const uint32_t n = n_list;
+        for (uint32_t i = 0; i < n; i++) {
+            parse_tile<false>(a, sm, list[i], a.tile_base[list[i]]);
+            __syncthreads();  // shared memory is reused by the next tile
+        }
     }
+    depth = __reduce_max_sync(0xFFFFFFFFu, depth);
+    if ((threadIdx.x & 31) == 0) atomicMax(&deepest, depth);
+    __syncthreads();
+    if (threadIdx.x == 0 && deepest) atomicMax(&a.stats->max_content_depth, deepest);
 }
 
 // FlatNode of every line from the text and a complete offsets array (used for
@@ -448,31 +520,12 @@ __global__ void classify_lines_kernel(const uint8_t *__restrict__ text, uint64_t
 
 cudaError_t launch_parse(const ParseArgs &a, cudaStream_t st) {
     if (a.n_tiles == 0) return cudaSuccess;
-    cudaError_t e;
-    if (a.slot) {
-        // staged: the text is read once; tiles with too many lines are redone
-        if ((e = launch_parse_begin(a, st)) != cudaSuccess) return e;
-        if ((e = launch_parse_tiles(a, 0, a.n_tiles, st)) != cudaSuccess) return e;
-        return launch_parse_end(a, st);
-    } else {
-        newline_count_kernel<<<a.n_tiles, PT_THREADS, 0, st>>>(a.text, a.text_len, a.tile_count); OL_LAUNCHED();
-        e = launch_scan_columns(a.tile_count, a.tile_base, nullptr, a.n_tiles, 1, scan_ld(a.n_tiles), st);
-        if (e != cudaSuccess) return e;
-        parse_tiles_kernel<<<a.n_tiles, PT_THREADS, 0, st>>>(a); OL_LAUNCHED();
-    }
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    uint32_t blocks = a.fixup_cap < 64 ? 8 : 64;
-    parse_fixup_kernel<<<blocks, 256, 0, st>>>(a); OL_LAUNCHED();
-    return cudaGetLastError();
-}
-
-cudaError_t launch_parse_begin(const ParseArgs &a, cudaStream_t st) {
-    if (!a.slot || a.slot_cap > PT_LIST) return cudaErrorInvalidValue;  // a slot is listed in one round
-    return cudaMemsetAsync(a.redo_n, 0, sizeof(uint32_t), st);
+    cudaError_t e = launch_parse_tiles(a, 0, a.n_tiles, st);
+    return e == cudaSuccess ? launch_parse_end(a, st) : e;
 }
 
 cudaError_t launch_parse_tiles(const ParseArgs &a, uint32_t t0, uint32_t t1, cudaStream_t st) {
+    if (a.slot_cap != kParseSlotCap) return cudaErrorInvalidValue;  // a slot is listed in one round
     t1 = std::min(t1, a.n_tiles);
     if (t0 >= t1) return cudaSuccess;
     ParseArgs r = a;
@@ -483,14 +536,14 @@ cudaError_t launch_parse_tiles(const ParseArgs &a, uint32_t t0, uint32_t t1, cud
 
 cudaError_t launch_parse_end(const ParseArgs &a, cudaStream_t st) {
     if (a.n_tiles == 0) return cudaSuccess;
+    if (a.n_tiles <= kParseFinishTiles) {
+        parse_finish_kernel<<<a.n_tiles, PT_THREADS, 0, st>>>(a); OL_LAUNCHED();
+        return cudaGetLastError();
+    }
     cudaError_t e = launch_scan_columns(a.tile_count, a.tile_base, nullptr, a.n_tiles, 1, scan_ld(a.n_tiles), st);
     if (e != cudaSuccess) return e;
     parse_copy_kernel<<<(a.n_tiles + PC_TILES - 1) / PC_TILES, 256, 0, st>>>(a); OL_LAUNCHED();
     parse_redo_kernel<<<std::min(a.n_tiles, 512u), PT_THREADS, 0, st>>>(a); OL_LAUNCHED();
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    const uint32_t blocks = a.fixup_cap < 64 ? 8 : 64;
-    parse_fixup_kernel<<<blocks, 256, 0, st>>>(a); OL_LAUNCHED();
     return cudaGetLastError();
 }
 

@@ -219,36 +219,32 @@ cudaError_t h2d(ol_ctx *ctx, uint8_t *dev, const uint8_t *host, uint64_t len) {
     return cudaSuccess;
 }
 
-// The staged parse's arguments for doc, with the context's scratch reserved
-// and the document's counters reset (enqueued on the context stream).
+// The staged parse's arguments for doc, with the context's scratch reserved.
 static cudaError_t parse_args(ol_ctx *ctx, ol_doc *d, ParseArgs &a) {
     cudaStream_t st = ctx->stream;
     cudaError_t e;
     uint32_t n_tiles = parse_tiles(d->text_len);
-    if ((e = ctx->scratch_a.reserve((size_t)scan_ld(n_tiles) * 8, st)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(d->stats, 0, sizeof(DocStats), st)) != cudaSuccess) return e;
+    const size_t ld = scan_ld(n_tiles);  // 16-byte aligned columns
+    if ((e = ctx->scratch_a.reserve(ld * 28, st)) != cudaSuccess) return e;
     a = ParseArgs{};
     a.text = d->text;
     a.text_len = d->text_len;
     a.n_tiles = n_tiles;
     a.tile_count = (uint32_t *)ctx->scratch_a.ptr;
-    a.tile_base = (uint32_t *)ctx->scratch_a.ptr + scan_ld(n_tiles);  // 16-byte aligned
+    a.tile_base = a.tile_count + ld;
+    a.tile_first = a.tile_count + 2 * ld;
+    a.tile_depth = (uint16_t *)(a.tile_count + 3 * ld);
     a.stats = d->stats;
     a.offsets = d->offsets;
     a.kinds = d->kinds;
     a.depth8 = d->depth8;
     a.line_cap = d->line_cap;
-    a.fixup = d->fixup;
-    a.fixup_cap = n_tiles;
-    // staged form: slots, then the per-tile flags, then the redo count and list
+    // slots, then the per-tile flags
     const size_t slot_bytes = (size_t)n_tiles * kParseSlotCap * 4;
-    const size_t list_at = (slot_bytes + n_tiles + 15) & ~size_t(15);
-    if ((e = ctx->parse_slot.reserve(list_at + 16 + (size_t)n_tiles * 4, st)) != cudaSuccess) return e;
+    if ((e = ctx->parse_slot.reserve(slot_bytes + n_tiles, st)) != cudaSuccess) return e;
     uint8_t *ps = (uint8_t *)ctx->parse_slot.ptr;
     a.slot = (uint32_t *)ps;
     a.slot_over = ps + slot_bytes;
-    a.redo_n = (uint32_t *)(ps + list_at);
-    a.redo_list = a.redo_n + 4;
     a.slot_cap = kParseSlotCap;
     return cudaSuccess;
 }
@@ -259,6 +255,16 @@ cudaError_t enqueue_parse(ol_ctx *ctx, ol_doc *d) {
     ParseArgs a;
     cudaError_t e = parse_args(ctx, d, a);
     return e == cudaSuccess ? launch_parse(a, ctx->stream) : e;
+}
+
+// Writes the line arrays of doc again, from the tiles staged by the parse of it
+// that has just run on ctx (the line arrays have grown since).
+static cudaError_t enqueue_parse_end(ol_ctx *ctx, ol_doc *d) {
+    GpuPass pass(ctx, "parse: line arrays");
+    ParseArgs a;
+    cudaError_t e = parse_args(ctx, d, a);
+    if (e == cudaSuccess) e = cudaMemsetAsync(d->stats, 0, sizeof(DocStats), ctx->stream);
+    return e == cudaSuccess ? launch_parse_end(a, ctx->stream) : e;
 }
 
 // The upload chunk after which the stage pass runs on the tiles that have
@@ -277,7 +283,6 @@ cudaError_t upload_parse_overlapped(ol_ctx *ctx, ol_doc *d, const uint8_t *host,
     GpuPass parse_pass(ctx, "parse (overlapped with the upload)");
     ParseArgs a;
     if ((e = parse_args(ctx, d, a)) != cudaSuccess) return e;
-    if ((e = launch_parse_begin(a, st)) != cudaSuccess) return e;
     // the copies start after the document's buffers exist on the main stream
     if ((e = cudaEventRecord(ctx->copy_ready, st)) != cudaSuccess) return e;
     if ((e = cudaStreamWaitEvent(cs, ctx->copy_ready, 0)) != cudaSuccess) return e;
@@ -335,7 +340,8 @@ ol_status alloc_lines(ol_ctx *ctx, ol_doc *d, uint64_t cap_lines) {
     return OL_OK;
 }
 
-// Runs the parse (with one exact-size retry when the estimate was too low),
+// Runs the parse (when the estimate was too low, the line arrays are written
+// once more at the exact size),
 // waits, and records the line count. With nodes_out, the 16-byte nodes are
 // materialised into ctx->scratch_c as well.
 ol_status parse_doc(ol_ctx *ctx, ol_doc *d, uint64_t est_lines, FlatNode **nodes_out, const uint8_t *host_text) {
@@ -343,14 +349,15 @@ ol_status parse_doc(ol_ctx *ctx, ol_doc *d, uint64_t est_lines, FlatNode **nodes
     for (int attempt = 0; attempt < 2; attempt++) {
         ol_status s = alloc_lines(ctx, d, est_lines);
         if (s != OL_OK) return s;
-        // the first attempt uploads the text as it parses; a retry finds it resident
-        cudaError_t e = attempt == 0 && host_text ? upload_parse_overlapped(ctx, d, host_text, d->text_len)
-                                                  : enqueue_parse(ctx, d);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(&d->host_stats, d->stats, sizeof(DocStats), cudaMemcpyDeviceToHost, st);
+        // the first attempt uploads the text as it parses; a retry finds every tile staged
+        cudaError_t e = attempt ? enqueue_parse_end(ctx, d)
+                                : host_text ? upload_parse_overlapped(ctx, d, host_text, d->text_len) : enqueue_parse(ctx, d);
+        DocStats *pinned = &ctx->host_counters->doc;
+        if (e == cudaSuccess) e = cudaMemcpyAsync(pinned, d->stats, sizeof(DocStats), cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) return ctx_cuda(ctx, e, "parse");
+        d->host_stats = *pinned;
         const DocStats &hs = d->host_stats;
-        if (hs.error & OL_DEVERR_FIXUP) return ctx_fail(ctx, OL_ERR_CUDA, "parse: fix-up list overflow");
         if (hs.error & OL_DEVERR_CAPACITY) {
             est_lines = hs.line_count;  // exact now
             continue;
@@ -384,9 +391,8 @@ ol_status new_doc(ol_ctx *ctx, uint64_t len, ol_doc **out) {
     }
     cudaStream_t st = ctx->stream;
     uint64_t alloc = text_alloc_bytes(len);
-    uint32_t n_tiles = parse_tiles(len);
     cudaError_t e = d->text_buf.reserve(alloc, st);
-    if (e == cudaSuccess) e = d->misc_buf.reserve(sizeof(DocStats) + (size_t)n_tiles * sizeof(uint2), st);
+    if (e == cudaSuccess) e = d->misc_buf.reserve(sizeof(DocStats), st);
     if (e == cudaSuccess) e = cudaMemsetAsync((uint8_t *)d->text_buf.ptr + len, 0, alloc - len, st);
     if (e != cudaSuccess) {
         ol_doc_free(d);
@@ -394,7 +400,6 @@ ol_status new_doc(ol_ctx *ctx, uint64_t len, ol_doc **out) {
     }
     d->text = (uint8_t *)d->text_buf.ptr;
     d->stats = (DocStats *)d->misc_buf.ptr;
-    d->fixup = (uint2 *)((uint8_t *)d->misc_buf.ptr + sizeof(DocStats));
     *out = d;
     return OL_OK;
 }

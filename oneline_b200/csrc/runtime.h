@@ -27,10 +27,12 @@ struct DevBuf {
 
 struct Prof;
 
-// Small per-context device words (a status word read back by the tree build).
+// Small per-context words in device memory, and their page-locked copy on the
+// host: short results are read back through the latter.
 struct CtxCounters {
     uint32_t error;
     uint32_t pad[15];
+    DocStats doc;  // a parse's counters
 };
 
 }  // namespace ol
@@ -81,7 +83,6 @@ struct ol_doc {
     uint8_t *kinds = nullptr;
     uint8_t *depth8 = nullptr;
     ol::DocStats *stats = nullptr;
-    uint2 *fixup = nullptr;
     ol::DocStats host_stats{};
 };
 
