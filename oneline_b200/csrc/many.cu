@@ -4,22 +4,30 @@
 // (crates/oneline-simd/src/search.rs:259-282). Replaces the reference's
 // window-filter kernels and host sort (crates/oneline-gpu/src/many.rs:391-646).
 //
-// The compiled set (runtime_many.cu) deduplicates the patterns and builds a
-// trie over the unique ones; its depth-4 nodes are reached through a hash
-// table keyed by a position's first four bytes, and a two-hash filter of those
-// keys (16 KiB) sits in shared memory, copied there once per block with a bulk
-// TMA copy (cp.async.bulk, no multicast).
+// The compiled set (runtime_many.cu) deduplicates the patterns. In oneline text
+// most dictionary hits lie in and around runs of one byte (indent markers,
+// rules), so the patterns of up to four run bytes c that start with c^3 are
+// kept apart:
+//   * runs c^k: found with bit masks, without looking at any position alone;
+//   * c^r rest (r >= 3, rest starting with another byte): found from the end of
+//     a run, once for all r: a trie over the rests, whose nodes list (r, pattern).
+// All other patterns are in a trie whose depth-4 nodes are reached through a
+// hash table keyed by a position's first four bytes. Where a trie continues with
+// a run byte several times (a line break, then indent markers), the node where
+// that begins lists the nodes of the run, so that a walk takes it in one step,
+// by the run's length in the text. A filter of those keys, and of c c c
+// rest[0] for the run ends, sits in shared memory (16 KiB), copied there once
+// per block with a bulk TMA copy (cp.async.bulk, no multicast).
 //
-// dict_match_kernel: persistent blocks walk 16 KiB tiles staged in shared
-// memory. Each warp takes 32 consecutive positions at a time (lane = position):
-// filter, table probe, then all lanes walk the trie one depth per iteration.
-// A unique pattern u of length d is met at depth d by every lane where it
-// occurs, so `__match_any_sync` on u at that depth groups exactly those lanes:
-//   * heavy patterns (chosen per search from a sample of the text) get one
-//     bitmap word per 32 positions, the group's lane mask, written without
-//     atomics through a per-warp staging area, sector by sector;
-//   * light patterns append (u << 32 | offset) keys with one warp-aggregated
-//     atomic per depth, and their counts with one atomic per group.
+// dict_match_kernel: persistent warps take slices of the text in turn. Every
+// position is filtered (16 a lane, from registers), the candidates are queued
+// and walked 32 at a time, one per lane; nodes with patterns are queued in turn
+// and their hits written 32 nodes at a time. Every hit is found by the warp
+// whose slice holds its start.
+//   * heavy patterns (chosen per search from a sample of the text) set bits in
+//     a bitmap: the slice's words are gathered in shared memory and stored once;
+//   * light patterns append (u << 32 | offset) keys through a per-warp buffer,
+//     and count themselves.
 // Then: popcounts of the bitmaps and a column scan give every heavy hit its
 // rank; a stable radix sort orders the light keys; a single-block pass gives
 // every pattern id its first output slot; the emit kernels write each hit
@@ -33,23 +41,48 @@
 
 namespace ol {
 
-constexpr uint32_t DM_THREADS = 256;
-constexpr uint32_t DM_WARPS = DM_THREADS / 32;
+// Two blocks of 20 warps fit an SM (registers and shared memory, the filter in
+// each block): 597 us against 659 with four of 8 warps (64 MiB, 10,000
+// patterns). A text whose slices are all walked at once by blocks of four warps
+// is spread over the chip in those.
+constexpr uint32_t DM_THREADS = 640;
+constexpr uint32_t DM_SMALL_THREADS = 128, DM_SMALL_WARPS_PER_SM = 24;
 constexpr uint32_t DM_QCAP = 64;                          // per-warp candidate queue
 constexpr uint32_t DM_FILTER_WORDS = 1u << (kDictFilterBits - 5);
 constexpr uint32_t kMbarSpins = 1u << 24;
+constexpr uint32_t DM_LIGHT = 32;                         // per-warp buffer of light keys
+constexpr uint32_t DM_EVENTS = 64;                        // per-warp queue of nodes with hits
+constexpr uint32_t DM_POW = 7;                            // run masks of 1, 2, 4, .., 64 bytes
 // A warp's work item: SLICE text positions (staged with the longest pattern
 // after them) and their SLICE / 32 heavy-bitmap words per heavy pattern.
 template <uint32_t SLICE>
-struct DictSmem {
+struct DictWarp {
     static constexpr uint32_t kWords = SLICE / 32;
+    static constexpr uint32_t kRunWords = kWords + 2;  // the slice and the 64 positions after it
     static constexpr uint32_t kText = SLICE + kDictHalo;
     static_assert(kText % 16 == 0 && kDictWordsPerTile % kWords == 0 && kDictTile % SLICE == 0, "slice geometry");
+    alignas(16) uint8_t text[kText];
+    alignas(16) uint32_t bits[kDictMaxHeavy][kWords];  // heavy pattern h starts at the positions of the set bits
+    unsigned long long light[DM_LIGHT];
+    // bit p of words 2..: position p holds the run byte (two words of 0 before, two after)
+    uint32_t run[kDictMaxRuns][kRunWords + 4];
+    uint32_t pow[DM_POW][kRunWords + 1];        // one run byte's: 2^i of it start at the position (a word of 0 after)
+    unsigned long long ev_starts[DM_EVENTS];    // DictEvent
+    uint32_t ev_at[DM_EVENTS];
+    uint32_t n_light, n_events;
+    uint16_t queue[DM_QCAP];
+};
+template <uint32_t SLICE>
+struct DictSmem {
     uint32_t filter[DM_FILTER_WORDS];
-    alignas(16) uint8_t text[DM_WARPS][kText];
-    uint32_t hmask[DM_WARPS][SLICE];  // per slice position: bit h = heavy pattern h starts there
-    uint16_t queue[DM_WARPS][DM_QCAP];
+    uint32_t heavy_run[kDictMaxHeavy];  // the heavy run patterns: (j << 16) | (k << 8) | heavy index
+    uint32_t n_heavy_run;
     alignas(8) unsigned long long bar;
+    DictWarp<SLICE> w[DM_THREADS / 32];  // as many as the block has warps
+
+    static size_t bytes(uint32_t threads) {
+        return sizeof(DictSmem) - (DM_THREADS - threads) / 32 * sizeof(DictWarp<SLICE>);
+    }
 };
 
 // ---------------------------------------------------------------- TMA bulk --
@@ -90,7 +123,7 @@ __device__ __forceinline__ bool mbar_wait(unsigned long long *bar, uint32_t pari
 
 __device__ __forceinline__ uint32_t dict_child(const DictSet &s, const uint4 &nd, uint32_t b) {
     if (nd.y & kDictDenseFlag) return __ldg(s.dense + (size_t)nd.w * 256 + b);
-    const uint32_t n = nd.y;
+    const uint32_t n = nd.y & kDictEdgeMask;
     if (n == 0) return NONE;
     uint32_t e0 = nd.z & 0xFFu;
     if (e0 == b) return nd.z >> 8;
@@ -119,82 +152,191 @@ __device__ __forceinline__ uint32_t dict_probe(const DictSet &s, uint32_t key) {
 
 // ------------------------------------------------------------- matching ----
 
-// Emits unique pattern u at absolute offset pos: counts (count mode), a bit of
-// the walk's heavy mask, or a light key.
-__device__ __forceinline__ void dict_emit(const DictMatchArgs &a, uint32_t &hm, uint32_t u, uint64_t pos) {
+// The unique pattern of entry x, (heavy index + 1, or 0) << 16 | u, starts at
+// slice position p (absolute: pos): counts (count mode), a bit of the heavy
+// pattern's bitmap words, or a light key.
+template <uint32_t SLICE>
+__device__ __forceinline__ void dict_emit(const DictMatchArgs &a, DictWarp<SLICE> &w, uint32_t x, uint32_t p, uint64_t pos) {
+    const uint32_t u = x & 0xFFFFu, hv = (x >> 16) & 0xFFu;
     if (a.count_only) {
         const uint32_t peers = __match_any_sync(__activemask(), u);
         if ((peers & ((1u << (threadIdx.x & 31)) - 1u)) == 0) atomicAdd(a.counts + u, (uint32_t)__popc(peers));
         return;
     }
-    const uint32_t hv = __ldg(a.heavy_of_u + u);
-    if (hv != 0xFFu) {
-        hm |= 1u << hv;
-    } else {
-        atomicAdd(a.counts + u, 1u);
+    if (hv) {
+        atomicOr(&w.bits[hv - 1][p >> 5], 1u << (p & 31));
+        return;
+    }
+    atomicAdd(a.counts + u, 1u);
+    const unsigned long long key = ((unsigned long long)u << 32) | (uint32_t)pos;
+    const uint32_t at = atomicAdd(&w.n_light, 1u);
+    if (at < DM_LIGHT) {
+        w.light[at] = key;
+    } else {  // the buffer is full until the walk's lanes meet again
         const uint32_t slot = atomicAdd(a.light_n, 1u);
-        if (slot < a.light_cap) a.light_keys[slot] = ((unsigned long long)u << 32) | (uint32_t)pos;
+        if (slot < a.light_cap) a.light_keys[slot] = key;
     }
 }
 
-// Every unique pattern starting at slice position p: probe the table with the
-// position's first four bytes, then walk the trie byte by byte. Hits must end
-// by `lim` (the end of the text, or of the position's document in a batch).
-// Returns the heavy patterns found (bit h: heavy pattern h).
-__device__ __forceinline__ uint32_t dict_walk(const DictMatchArgs &a, const uint8_t *text, uint32_t p, uint64_t pos,
-                                              uint64_t lim, uint32_t &levels) {
-    const uint32_t key = (uint32_t)text[p] | ((uint32_t)text[p + 1] << 8) | ((uint32_t)text[p + 2] << 16) |
-                         ((uint32_t)text[p + 3] << 24);
-    uint32_t v = pos + kDictMinLen <= lim ? dict_probe(a.set, key) : NONE;
-    uint32_t d = kDictMinLen, hm = 0;
-    if (v != NONE && a.n_chains && key == (key & 0xFFu) * 0x01010101u) {
-        // The position starts a run of one byte c: if c has a chain, jump to
-        // the chain node of depth D = min(run, chain, max length, document
-        // end), taking every pattern c^4..c^D at once, then walk on from it.
-        const uint32_t c = key & 0xFFu;
-        uint32_t j = 0;
-        while (j < a.n_chains && ((a.chain_bytes >> (8 * j)) & 0xFFu) != c) j++;
-        if (j < a.n_chains) {
-            const DictChain *ch = a.chains + j;
-            uint32_t cap = min(__ldg(&ch->K), kDictMaxLen);
-            if (lim - pos < cap) cap = (uint32_t)(lim - pos);  // >= kDictMinLen: the probe ran
-            const uint32_t *tw = reinterpret_cast<const uint32_t *>(text);
-            const uint32_t C4 = c * 0x01010101u;
-            uint32_t run = kDictMinLen;
-            while (run < cap) {  // 4 bytes per step; the staged halo covers p + 67
-                const uint32_t q = p + run;
-                const uint32_t w = __funnelshift_r(tw[q >> 2], tw[(q >> 2) + 1], (q & 3) * 8);
-                const uint32_t z = zero_bytes(w ^ C4);
-                if (z == 0x80808080u) {
-                    run += 4;
-                    continue;
-                }
-                run += (__ffs(~z & 0x80808080u) - 8) >> 3;
-                break;
-            }
-            const uint32_t D = min(run, cap);
-            levels++;
-            hm = __ldg(&ch->cum[D]);
-            const uint32_t nl = __ldg(&ch->n_light);
-            for (uint32_t i = 0; i < nl; i++) {
-                const uint32_t e = __ldg(&ch->light[i]);
-                if ((e >> 24) > D) break;
-                dict_emit(a, hm, e & 0xFFFFFFu, pos);
-            }
-            if (D >= kDictMaxLen || pos + D >= lim) return hm;
-            v = dict_child(a.set, __ldg(a.set.nodes + __ldg(&ch->node[D])), text[p + D]);
-            d = D + 1;
-        }
+// The whole warp moves the buffered light keys to the search's list when at
+// least `least` are there.
+template <uint32_t SLICE>
+__device__ __forceinline__ void dict_flush(const DictMatchArgs &a, DictWarp<SLICE> &w, uint32_t least) {
+    const uint32_t lane = threadIdx.x & 31;
+    __syncwarp();
+    const uint32_t n = min(w.n_light, DM_LIGHT);
+    if (n < least) return;  // uniform
+    uint32_t base = 0;
+    if (lane == 0) base = atomicAdd(a.light_n, n);
+    base = __shfl_sync(0xFFFFFFFFu, base, 0);
+    for (uint32_t i = lane; i < n; i += 32)
+        if (base + i < a.light_cap) a.light_keys[base + i] = w.light[i];
+    __syncwarp();
+    if (lane == 0) w.n_light = 0;
+    __syncwarp();
+}
+
+// Hits of one node: patterns outs[o], outs[o + 1], ... start r before slice
+// position e for the set bits r of `starts` in turn; with `same`, all at e.
+// Packed: at = (same << 31) | (o << 11) | e.
+constexpr uint32_t kEventSame = 0x80000000u;
+
+template <uint32_t SLICE>
+__device__ __forceinline__ void dict_hits(const DictMatchArgs &a, DictWarp<SLICE> &w, unsigned long long starts, uint32_t at,
+                                          uint64_t s0) {
+    const uint32_t e = at & 0x7FFu;
+    const uint32_t *o = a.outs + ((at & ~kEventSame) >> 11);
+    uint32_t next = __ldg(o);  // a step ahead (the entry after the last is not used)
+    for (; starts; starts &= starts - 1) {
+        const uint32_t entry = next, p = (at & kEventSame) ? e : e + 1 - __ffsll(starts);
+        next = __ldg(++o);
+        dict_emit(a, w, entry, p, s0 + p);
     }
+}
+
+// A node's hits at once, when the queue is full until the walk's lanes meet
+// again. Out of line: the walk's code has to stay small (inlined with its
+// callers, the match kernel waited for instructions more than for anything
+// but memory).
+template <uint32_t SLICE>
+__device__ __noinline__ void dict_hits_now(const DictMatchArgs &a, DictWarp<SLICE> &w, unsigned long long starts, uint32_t at,
+                                           uint64_t s0) {
+    dict_hits(a, w, starts, at, s0);
+}
+
+template <uint32_t SLICE>
+__device__ __forceinline__ void dict_push(const DictMatchArgs &a, DictWarp<SLICE> &w, unsigned long long starts, uint32_t at,
+                                          uint64_t s0) {
+    const uint32_t i = atomicAdd(&w.n_events, 1u);
+    if (i < DM_EVENTS) {
+        w.ev_starts[i] = starts;
+        w.ev_at[i] = at;
+    } else {
+        dict_hits_now(a, w, starts, at, s0);
+    }
+}
+
+// The whole warp writes the hits of the queued nodes, one per lane, when at
+// least `least` are queued.
+template <uint32_t SLICE>
+__device__ __forceinline__ void dict_drain(const DictMatchArgs &a, DictWarp<SLICE> &w, uint32_t least, uint64_t s0) {
+    __syncwarp();
+    const uint32_t n = min(w.n_events, DM_EVENTS);
+    if (n < least) return;  // uniform
+    for (uint32_t i = threadIdx.x & 31; i < n; i += 32) dict_hits(a, w, w.ev_starts[i], w.ev_at[i], s0);
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) w.n_events = 0;
+    if (!a.count_only) dict_flush(a, w, DM_LIGHT / 2);
+    __syncwarp();
+}
+
+// Length of the run of run byte j that starts at slice position p (which holds
+// it), as far as the masks go.
+template <uint32_t SLICE>
+__device__ __forceinline__ uint32_t dict_run_from(const DictWarp<SLICE> &w, uint32_t j, uint32_t p) {
+    const uint32_t *rw = w.run[j] + 2 + (p >> 5);
+    const uint32_t lo = __funnelshift_r(rw[0], rw[1], p & 31);
+    if (lo != 0xFFFFFFFFu) return __ffs(~lo) - 1;
+    const uint32_t hi = __funnelshift_r(rw[1], rw[2], p & 31);
+    return 32 + (hi != 0xFFFFFFFFu ? __ffs(~hi) - 1 : 32);
+}
+
+// Every hit of the candidate at slice position p. Hits must end by `lim` (the
+// end of the text, or of the position's document in a batch).
+//   * c c c x of a run byte c, x another: the run's end e = p + 3 is walked, for
+//     the starts that lie in the slice, 3 to R (the run's length back to the
+//     slice's start) before e;
+//   * any other four bytes: the table gives the depth-4 node.
+template <uint32_t SLICE>
+__device__ __forceinline__ void dict_walk(const DictMatchArgs &a, DictWarp<SLICE> &w, uint32_t p, uint64_t s0, uint64_t lim,
+                                          uint32_t &levels) {
+    const uint32_t *tw = reinterpret_cast<const uint32_t *>(w.text);
+    const uint32_t key = __funnelshift_r(tw[p >> 2], tw[(p >> 2) + 1], (p & 3) * 8);
+    if (s0 + p + kDictMinLen > lim) return;
+    uint32_t j = a.set.n_runs;
+    if (((key ^ (key >> 8)) & 0xFFFFu) == 0)  // three equal bytes
+        for (j = 0; j < a.set.n_runs && ((a.set.run_bytes >> (8 * j)) & 0xFFu) != (key & 0xFFu);) j++;
+    // The text from slice position e on is matched against a trie from node v,
+    // t bytes so far; a node's patterns start r before e: r = 0, or the starts
+    // that lie in the slice, r0 to R.
+    uint32_t v, e = p, t = kDictMinLen, r0 = 0;
+    unsigned long long starts = 1;
+    if (j < a.set.n_runs) {
+        const uint32_t *rw = w.run[j] + (p >> 5);  // words p/32 - 2 .. p/32
+        const uint32_t hi = __funnelshift_r(rw[1], rw[2], p & 31), lo = __funnelshift_r(rw[0], rw[1], p & 31);
+        const uint32_t back = hi != 0xFFFFFFFFu ? __clz(~hi) : 32 + __clz(~lo);  // (__clz(0) = 32)
+        e = p + 3;
+        t = 1;
+        r0 = e > SLICE + 2 ? e - SLICE + 1 : 3u;
+        starts = (~0ull >> (kDictMaxLen - 1 - min(3 + back, kDictMaxLen - 1))) & (~0ull << r0);
+        v = __ldg(a.set.dense + (size_t)a.set.run_root[j] * 256 + (key >> 24));
+    } else {
+        v = dict_probe(a.set, key);
+    }
+    const uint32_t end = (uint32_t)min(lim - s0, (uint64_t)(SLICE + 2 * kDictMaxLen));  // lim, as a slice position
     while (v != NONE) {
         const uint4 nd = __ldg(a.set.nodes + v);
         levels++;
-        if (nd.x != NONE) dict_emit(a, hm, nd.x, pos);
-        if (d >= kDictMaxLen || pos + d >= lim) break;
-        v = dict_child(a.set, nd, text[p + d]);
-        d++;
+        if (nd.x != NONE) {
+            if (nd.x & kDictOneFlag) {
+                dict_push(a, w, 1ull, ((nd.x & ~kDictOneFlag) << 11) | e, s0);
+            } else {  // of the list's entries only those that count
+                const uint4 l = __ldg(a.set.lists + nd.x);
+                const unsigned long long all = ((unsigned long long)l.y << 32) | l.x, m = all & starts;
+                if (m) dict_push(a, w, m, ((l.z + __popcll(all & ((m & (0 - m)) - 1))) << 11) | e, s0);
+            }
+        }
+        if (t + r0 >= kDictMaxLen || e + t >= end) break;
+        const uint32_t b = w.text[e + t];
+        if ((nd.y & kDictPathFlag) && b == ((a.set.run_bytes >> (8 * ((nd.y >> 28) & 3u))) & 0xFFu)) {
+            // the node's run: K nodes, the patterns of those passed by, then on from the last one reached
+            const uint32_t *path = a.set.paths + ((nd.y >> 9) & 0x7FFFFu);
+            const uint32_t D = min(min(__ldg(path), min(kDictMaxLen - t, end - e - t)),
+                                   dict_run_from(w, (nd.y >> 28) & 3u, e + t));
+            const unsigned long long all = ((unsigned long long)__ldg(path + 2) << 32) | __ldg(path + 1);
+            const uint32_t n = __popcll(all & ((1ull << (D - 1)) - 1));  // D >= 1: b is the run byte
+            if (n) dict_push(a, w, (1ull << n) - 1, kEventSame | (__ldg(path + 3) << 11) | e, s0);
+            v = __ldg(path + 3 + D);
+            t += D;
+            continue;
+        }
+        v = dict_child(a.set, nd, b);
+        t++;
     }
-    return hm;
+}
+
+// 16-bit mask of the positions lo .. lo + 15 below n.
+__device__ __forceinline__ uint32_t below16(uint32_t n, uint32_t lo) {
+    return n <= lo ? 0u : n - lo >= 16 ? 0xFFFFu : (1u << (n - lo)) - 1u;
+}
+
+// The pattern run_byte(j)^k over the slice's word i: bit b is set where it
+// starts. pow[q] holds the starts of runs of 2^q: with 2^q <= k < 2^(q+1) a run
+// of k is one of 2^q here and one k - 2^q further on.
+template <uint32_t SLICE>
+__device__ __forceinline__ uint32_t dict_run_word(const DictWarp<SLICE> &w, uint32_t k, uint32_t i) {
+    const uint32_t q = 31 - __clz(k), s = k - (1u << q);  // k = 4..64: s <= 31
+    return w.pow[q][i] & __funnelshift_r(w.pow[q][i], w.pow[q][i + 1], s);
 }
 
 // End of the document holding pos (pos itself when pos lies between
@@ -211,18 +353,16 @@ __device__ __forceinline__ uint64_t dict_limit(const DictMatchArgs &a, uint64_t 
 // Each warp takes slices of SLICE positions in turn: it stages the slice (plus
 // the longest pattern) in its own shared memory, filters all positions 32 at a
 // time, queues the candidates and walks them 32 at a time (one per lane), so
-// walks run on full warps. A walk returns the heavy patterns of its position as
-// a 32-bit mask (no atomics); after the slice, ballots over each 32 positions'
-// masks transpose them into the heavy patterns' bitmap words, which lane h
-// stores for heavy pattern h. Warps never wait for one another.
+// walks run on full warps; then it finds the run patterns from the run bytes'
+// masks and stores the heavy patterns' words of the slice. Warps never wait for
+// one another.
 template <uint32_t SLICE>
-__global__ void __launch_bounds__(DM_THREADS) dict_match_kernel(DictMatchArgs a) {
-    using Smem = DictSmem<SLICE>;
-    constexpr uint32_t DM_SLICE = SLICE, DM_SLICE_WORDS = Smem::kWords, DM_TEXT_BYTES = Smem::kText;
+__global__ void __launch_bounds__(DM_THREADS, 2) dict_match_kernel(const __grid_constant__ DictMatchArgs a) {
+    using Warp = DictWarp<SLICE>;
     constexpr uint32_t DM_SLICES_PER_TILE = kDictTile / SLICE;
     extern __shared__ __align__(16) uint8_t dyn_smem[];
-    Smem &sm = *reinterpret_cast<Smem *>(dyn_smem);
-    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    DictSmem<SLICE> &sm = *reinterpret_cast<DictSmem<SLICE> *>(dyn_smem);
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n_warps = blockDim.x >> 5;
     const uint32_t lt = (1u << lane) - 1u;
 
     // The filter, once per block, by a bulk copy.
@@ -236,6 +376,12 @@ __global__ void __launch_bounds__(DM_THREADS) dict_match_kernel(DictMatchArgs a)
     // (A separate statement: folded into the wait's result, the test hook
     // made the whole match kernel 47% slower, 19.8 against 13.5 ms per GiB.)
     if (a.force_timeout) ok = false;
+    if (warp == 0) {
+        const uint32_t x = !a.count_only && lane < a.n_heavy ? a.heavy_run[lane] : 0u;
+        const uint32_t m = __ballot_sync(0xFFFFFFFFu, x != 0);
+        if (x) sm.heavy_run[__popc(m & lt)] = (x << 8) | lane;
+        if (lane == 0) sm.n_heavy_run = __popc(m);
+    }
     if (!__syncthreads_and(ok)) {
         if (tid == 0) atomicOr(a.error, OL_DEVERR_TIMEOUT);
         mbar_wait(&sm.bar, 0);  // let the copy land before the block exits
@@ -245,22 +391,38 @@ __global__ void __launch_bounds__(DM_THREADS) dict_match_kernel(DictMatchArgs a)
     const uint64_t N = a.text_len;
     const uint32_t n_words = a.n_tiles * kDictWordsPerTile;
     const uint32_t n_items = ((a.n_tiles + a.tile_stride - 1) / a.tile_stride) * DM_SLICES_PER_TILE;
-    const uint32_t H = a.count_only ? 0u : a.n_heavy;
-    uint8_t *text = sm.text[warp];
-    uint32_t *hmask = sm.hmask[warp];
+    const uint32_t H = a.count_only ? 0u : a.n_heavy, n_runs = a.set.n_runs, run_bytes = a.set.run_bytes;
     uint32_t cands = 0, levels = 0;  // per lane, for the search statistics
-    uint16_t *queue = sm.queue[warp];
+    Warp &w = sm.w[warp];
+    uint8_t *text = w.text;
+    uint16_t *queue = w.queue;
+    const uint32_t *tw = reinterpret_cast<const uint32_t *>(text);
+    if (lane == 0) w.n_light = w.n_events = 0;
+    if (lane < kDictMaxRuns) {
+        w.run[lane][0] = w.run[lane][1] = 0;
+        w.run[lane][Warp::kRunWords + 2] = w.run[lane][Warp::kRunWords + 3] = 0;
+    }
+    for (uint32_t i = lane; i < DM_POW; i += 32) w.pow[i][Warp::kRunWords] = 0;
+    if (lane < H && H)
+        for (uint32_t i = 0; i < Warp::kWords; i += 4) *reinterpret_cast<uint4 *>(&w.bits[lane][i]) = make_uint4(0, 0, 0, 0);
 
-    for (uint32_t item = blockIdx.x * DM_WARPS + warp; item < n_items; item += gridDim.x * DM_WARPS) {
+    for (uint32_t item = blockIdx.x * n_warps + warp; item < n_items; item += gridDim.x * n_warps) {
         const uint32_t slice = (item / DM_SLICES_PER_TILE) * a.tile_stride * DM_SLICES_PER_TILE + item % DM_SLICES_PER_TILE;
-        const uint64_t s0 = (uint64_t)slice * DM_SLICE;  // slices past the text only write zero words
+        const uint64_t s0 = (uint64_t)slice * SLICE;  // slices past the text only write zero words
+        constexpr uint32_t kPieces = SLICE / 16, kMine = (kPieces + 31) / 32;  // 16-byte pieces; a lane's
+        uint4 v[kMine];
         __syncwarp();
-        for (uint32_t o = lane * 16; o < DM_TEXT_BYTES; o += 32 * 16)
-            *reinterpret_cast<uint4 *>(&text[o]) = ld_stream16(a.text + s0 + o);
-        if (H)
-            for (uint32_t f = lane; f < DM_SLICE; f += 32) hmask[f] = 0;
+#pragma unroll
+        for (uint32_t i = 0; i < kMine; i++) {
+            const uint32_t piece = i * 32 + lane;
+            v[i] = ld_stream16(a.text + s0 + piece * 16);  // (SLICE = 256: up to 256 bytes past the slice)
+            if (piece < Warp::kText / 16) *reinterpret_cast<uint4 *>(&text[piece * 16]) = v[i];
+        }
+        if (kMine * 32 + lane < Warp::kText / 16)
+            *reinterpret_cast<uint4 *>(&text[(kMine * 32 + lane) * 16]) = ld_stream16(a.text + s0 + (kMine * 32 + lane) * 16);
+        // bytes of the text from the slice start on, as far as they matter here
+        const uint32_t have = N > s0 ? (uint32_t)min(N - s0, (uint64_t)(SLICE + 64)) : 0u;
         __syncwarp();
-        const uint32_t *tw = reinterpret_cast<const uint32_t *>(text);
         uint32_t hint = 0;
         if (a.seg_end) {  // first document ending after the slice start
             uint32_t lo = 0, hi = a.n_seg;
@@ -273,69 +435,152 @@ __global__ void __launch_bounds__(DM_THREADS) dict_match_kernel(DictMatchArgs a)
             }
             hint = lo;
         }
-        uint32_t qn = 0;
-        for (uint32_t step = 0; step < DM_SLICE / 32; step++) {
-            const uint32_t p = step * 32 + lane;
-            const uint64_t pos = s0 + p;
-            bool cand = false;
-            if (pos + kDictMinLen <= N) {
-                const uint32_t key = __funnelshift_r(tw[p >> 2], tw[(p >> 2) + 1], (p & 3) * 8);
-                const uint32_t h1 = dict_filter_h1(key), h2 = dict_filter_h2(key);
-                cand = ((sm.filter[h1 >> 5] >> (h1 & 31)) & (sm.filter[h2 >> 5] >> (h2 & 31)) & 1u) != 0;
+        // The run bytes' masks over the slice and the 64 positions after it.
+#pragma unroll 1
+        for (uint32_t j = 0; j < n_runs; j++) {
+            const uint32_t c = (run_bytes >> (8 * j)) & 0xFFu;
+#pragma unroll
+            for (uint32_t i = 0; i < kMine; i++) {
+                const uint32_t piece = i * 32 + lane;
+                uint32_t m = eq_mask16(v[i], c * 0x01010101u) & below16(have, piece * 16);
+                m |= __shfl_down_sync(0xFFFFFFFFu, m, 1) << 16;
+                if (!(lane & 1) && piece < kPieces) w.run[j][2 + piece / 2] = m;
             }
-            const uint32_t cm = __ballot_sync(0xFFFFFFFFu, cand);
-            if (cand) queue[qn + __popc(cm & lt)] = (uint16_t)p;
-            qn += __popc(cm);
-            __syncwarp();
-            if (qn >= 32) {  // walk 32 candidates, one per lane
-                const uint32_t q = queue[lane];
-                const uint32_t hm = dict_walk(a, text, q, s0 + q, dict_limit(a, s0 + q, hint), levels);
-                if (hm) hmask[q] = hm;
-                cands++;
-                __syncwarp();
-                const uint16_t keep = lane + 32 < qn ? queue[lane + 32] : (uint16_t)0;
-                __syncwarp();
-                if (lane + 32 < qn) queue[lane] = keep;
-                qn -= 32;
-                __syncwarp();
-            }
-        }
-        if (lane < qn) {
-            const uint32_t q = queue[lane];
-            const uint32_t hm = dict_walk(a, text, q, s0 + q, dict_limit(a, s0 + q, hint), levels);
-            if (hm) hmask[q] = hm;
-            cands++;
+            const uint32_t q = SLICE + lane;
+            const uint32_t m0 = __ballot_sync(0xFFFFFFFFu, text[q] == c && q < have);
+            const uint32_t m1 = __ballot_sync(0xFFFFFFFFu, text[q + 32] == c && q + 32 < have);
+            if (lane < 2) w.run[j][2 + Warp::kWords + lane] = lane ? m1 : m0;
         }
         __syncwarp();
-        if (H) {
-            // transpose: word w of heavy pattern h holds bit h of positions
-            // 32w..32w+31. Lane q has position 32w+q's mask (a row of a 32x32
-            // bit matrix); five butterfly rounds swap ever smaller off-diagonal
-            // blocks between lanes, after which lane h holds column h.
-            uint32_t words[DM_SLICE_WORDS];
+        // Candidates, lane by lane: bit q of cm is position piece * 16 + q.
+        uint32_t cm[kMine];
 #pragma unroll
-            for (uint32_t w = 0; w < DM_SLICE_WORDS; w++) {
-                uint32_t x = hmask[w * 32 + lane];
-                if (__any_sync(0xFFFFFFFFu, x != 0)) {
+        for (uint32_t i = 0; i < kMine; i++) {
+            const uint32_t piece = i * 32 + lane;
+            const uint32_t *pw = tw + (piece < kPieces ? piece * 4 : 0);
+            uint32_t m = 0, x = pw[0];
+#pragma unroll 1
+            for (uint32_t q = 0; q < 16; q += 4) {  // (rolled: the code has to stay small)
+                const uint32_t y = *++pw;
 #pragma unroll
-                    for (uint32_t j = 16; j > 0; j >>= 1) {
-                        const uint32_t left = j == 16 ? 0x0000FFFFu : j == 8 ? 0x00FF00FFu : j == 4 ? 0x0F0F0F0Fu
-                                              : j == 2 ? 0x33333333u : 0x55555555u;  // bits i with (i & j) == 0
-                        const uint32_t y = __shfl_xor_sync(0xFFFFFFFFu, x, j);
-                        x = (lane & j) ? (x & ~left) | ((y & ~left) >> j) : (x & left) | ((y & left) << j);
+                for (uint32_t b = 0; b < 4; b++) {
+                    const uint32_t key = b ? __funnelshift_r(x, y, 8 * b) : x;
+                    const uint32_t f = sm.filter[dict_filter_word(key)], g = dict_filter_bits(key);
+                    m |= ((f >> (g >> 27)) & (f >> ((g >> 22) & 31)) & (f >> ((g >> 17) & 31)) & 1u) << (q + b);
+                }
+                x = y;
+            }
+            m &= piece < kPieces ? below16(have > 3 ? have - 3 : 0u, piece * 16) : 0u;  // four bytes of text
+#pragma unroll 1
+            for (uint32_t j = 0; j < n_runs; j++) {  // c^4: inside a run, the masks find those
+                const uint32_t *rw = w.run[j] + 2 + (piece < kPieces ? piece / 2 : 0);
+                const uint32_t r = __funnelshift_r(rw[0], rw[1], (piece & 1) * 16);
+                m &= ~(r & (r >> 1) & (r >> 2) & (r >> 3));
+            }
+            cm[i] = m;
+        }
+        // The end of a run that covers the slice's last position and ends at
+        // least 3 further on is one more candidate, past the slice.
+        uint32_t tail = 0;
+#pragma unroll 1
+        for (uint32_t j = 0; j < n_runs; j++) {
+            if (!(w.run[j][Warp::kWords + 1] >> 31)) continue;  // uniform, and so is what follows
+            const uint32_t f = dict_run_from(w, j, SLICE);
+            if (f >= 3 && f < kDictMaxLen) tail = SLICE + f - 3;  // of one run byte at most
+        }
+        for (uint32_t qn = 0, at = 0, last = 0; !last;) {
+            while (qn < 32 && !last) {  // each lane's lowest candidate, until the queue holds a full round
+                uint32_t mine = cm[0];
+#pragma unroll
+                for (uint32_t i = 1; i < kMine; i++) mine = at == i ? cm[i] : mine;
+                const uint32_t any = __ballot_sync(0xFFFFFFFFu, mine != 0);
+                if (any) {
+                    if (mine) queue[qn + __popc(any & lt)] = (uint16_t)((at * 32 + lane) * 16 + __ffs(mine) - 1);
+                    qn += __popc(any);
+#pragma unroll
+                    for (uint32_t i = 0; i < kMine; i++)
+                        if (at == i) cm[i] = mine & (mine - 1);
+                } else if (++at == kMine) {
+                    if (tail && lane == 0) queue[qn] = (uint16_t)tail;
+                    qn += tail != 0;
+                    tail = 0;
+                    last = qn <= 32;
+                    if (!last) at = kMine - 1;
+                }
+            }
+            __syncwarp();
+            const uint32_t n = min(qn, 32u);
+            if (lane < n) {  // one candidate per lane
+                const uint32_t p = queue[lane];
+                dict_walk(a, w, p, s0, dict_limit(a, s0 + p, hint), levels);
+                cands++;
+            }
+            __syncwarp();
+            const uint16_t keep = lane + 32 < qn ? queue[lane + 32] : (uint16_t)0;
+            __syncwarp();
+            if (lane + 32 < qn) queue[lane] = keep;
+            qn -= n;
+            dict_drain(a, w, last ? 1 : DM_EVENTS / 2, s0);
+        }
+        // Run patterns, one run byte after the other.
+#pragma unroll 1
+        for (uint32_t j = 0; j < n_runs; j++) {
+            bool any = false;
+            for (uint32_t i = lane; i < Warp::kRunWords; i += 32) w.pow[0][i] = w.run[j][i + 2];
+#pragma unroll
+            for (uint32_t q = 1; q < DM_POW; q++) {
+                __syncwarp();
+                for (uint32_t i = lane; i < Warp::kRunWords; i += 32) {
+                    const uint32_t x = w.pow[q - 1][i], y = w.pow[q - 1][i + 1];
+                    const uint32_t z = x & (q == 6 ? y : __funnelshift_r(x, y, 1u << (q - 1)));
+                    w.pow[q][i] = z;
+                    if (q == 2) any |= i < Warp::kWords && z != 0;
+                }
+                if (q == 2 && !__any_sync(0xFFFFFFFFu, any)) break;  // no run of four
+            }
+            if (!__any_sync(0xFFFFFFFFu, any)) continue;
+            __syncwarp();
+            const uint32_t n_hr = sm.n_heavy_run;
+            for (uint32_t i = lane; i < n_hr * Warp::kWords; i += 32) {  // (pattern, word) pairs
+                const uint32_t x = sm.heavy_run[i / Warp::kWords];
+                if ((x >> 16) == j) w.bits[x & 0xFFu][i % Warp::kWords] = dict_run_word(w, (x >> 8) & 0xFFu, i % Warp::kWords);
+            }
+            // the light ones (all of them in count mode)
+            for (uint32_t n = 0; n < a.n_run_light; n++) {
+                const uint32_t x = __ldg(a.run_light + n);  // (j << 24) | (k << 16) | u
+                if ((x >> 24) != j) continue;
+                const uint32_t u = x & 0xFFFFu;
+                uint32_t sum = 0;
+                for (uint32_t i = lane; i < Warp::kWords; i += 32) {
+                    uint32_t m = dict_run_word(w, (x >> 16) & 0xFFu, i);
+                    sum += __popc(m);
+                    if (a.count_only) continue;
+                    for (; m; m &= m - 1) {
+                        const uint32_t p = i * 32 + __ffs(m) - 1;
+                        dict_emit(a, w, u, p, s0 + p);
                     }
                 }
-                words[w] = x;
+                if (a.count_only) {
+                    sum = __reduce_add_sync(0xFFFFFFFFu, sum);
+                    if (lane == 0 && sum) atomicAdd(a.counts + u, sum);
+                } else {
+                    dict_flush(a, w, DM_LIGHT / 2);
+                }
             }
-            // lane h stores heavy pattern h's words of the slice (contiguous, 16-byte stores)
-            if (lane < H) {
-                uint4 *dst = reinterpret_cast<uint4 *>(a.bitmap + (size_t)lane * n_words + (size_t)slice * DM_SLICE_WORDS);
+        }
+        __syncwarp();
+        // lane h stores heavy pattern h's words of the slice (contiguous, 16-byte stores) and clears them
+        if (lane < H) {
+            uint4 *dst = reinterpret_cast<uint4 *>(a.bitmap + (size_t)lane * n_words + (size_t)slice * Warp::kWords);
+            uint4 *src = reinterpret_cast<uint4 *>(w.bits[lane]);
 #pragma unroll
-                for (uint32_t w = 0; w < DM_SLICE_WORDS; w += 4)
-                    dst[w / 4] = make_uint4(words[w], words[w + 1], words[w + 2], words[w + 3]);
+            for (uint32_t i = 0; i < Warp::kWords / 4; i++) {
+                dst[i] = src[i];
+                src[i] = make_uint4(0, 0, 0, 0);
             }
         }
     }
+    if (!a.count_only) dict_flush(a, w, 1);
     if (a.stats) {  // candidates walked and trie nodes visited
         const uint32_t c = __reduce_add_sync(0xFFFFFFFFu, cands), l = __reduce_add_sync(0xFFFFFFFFu, levels);
         if (lane == 0) {
@@ -347,17 +592,22 @@ __global__ void __launch_bounds__(DM_THREADS) dict_match_kernel(DictMatchArgs a)
 
 template <uint32_t SLICE>
 static cudaError_t launch_match(const DictMatchArgs &a, int sm_count, uint32_t blocks_per_sm, cudaStream_t st) {
-    const size_t smem = sizeof(DictSmem<SLICE>);
-    cudaError_t e = cudaFuncSetAttribute(dict_match_kernel<SLICE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dict_match_kernel<SLICE>, DM_THREADS, smem);
-    if (e != cudaSuccess) return e;
-    if (blocks_per_sm) per_sm = std::min<int>(per_sm, (int)blocks_per_sm);
     const uint64_t n_items = (uint64_t)((a.n_tiles + a.tile_stride - 1) / a.tile_stride) * (kDictTile / SLICE);
-    const uint32_t grid = (uint32_t)std::min<uint64_t>((n_items + DM_WARPS - 1) / DM_WARPS,
-                                                       (uint64_t)std::max(per_sm, 1) * sm_count);
-    dict_match_kernel<SLICE><<<grid, DM_THREADS, smem, st>>>(a); OL_LAUNCHED();
+    const bool small = n_items <= (uint64_t)sm_count * DM_SMALL_WARPS_PER_SM;
+    const uint32_t threads = small ? DM_SMALL_THREADS : DM_THREADS, warps = threads / 32;
+    const size_t smem = DictSmem<SLICE>::bytes(threads);
+    cudaError_t e = cudaFuncSetAttribute(dict_match_kernel<SLICE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)sizeof(DictSmem<SLICE>));
+    if (e != cudaSuccess) return e;
+    uint64_t grid = (n_items + warps - 1) / warps;
+    if (!small || blocks_per_sm) {
+        int per_sm = 0;
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dict_match_kernel<SLICE>, threads, smem);
+        if (e != cudaSuccess) return e;
+        if (blocks_per_sm) per_sm = std::min<int>(per_sm, (int)blocks_per_sm);
+        grid = std::min<uint64_t>(grid, (uint64_t)std::max(per_sm, 1) * sm_count);
+    }
+    dict_match_kernel<SLICE><<<(uint32_t)grid, threads, smem, st>>>(a); OL_LAUNCHED();
     return cudaGetLastError();
 }
 
@@ -371,6 +621,19 @@ cudaError_t launch_dict_match(const DictMatchArgs &a, int sm_count, cudaStream_t
         case 1024: return launch_match<1024>(a, sm_count, blocks_per_sm, st);
         default: return launch_match<512>(a, sm_count, blocks_per_sm, st);
     }
+}
+
+// The lists' entries of one search: each with its pattern's heavy index.
+__global__ void dict_outs_kernel(const uint32_t *__restrict__ outs, const uint8_t *__restrict__ heavy_of_u, uint32_t n,
+                                 uint32_t *__restrict__ to) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) to[i] = (((heavy_of_u[outs[i]] + 1u) & 0xFFu) << 16) | outs[i];
+}
+
+cudaError_t launch_dict_outs(const uint32_t *outs, const uint8_t *heavy_of_u, uint32_t n, uint32_t *to, cudaStream_t st) {
+    if (n == 0) return cudaSuccess;
+    dict_outs_kernel<<<(n + 255) / 256, 256, 0, st>>>(outs, heavy_of_u, n, to); OL_LAUNCHED();
+    return cudaGetLastError();
 }
 
 // ------------------------------------------------------------ heavy ranks --

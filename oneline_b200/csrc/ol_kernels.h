@@ -175,14 +175,18 @@ constexpr uint32_t kDictHalo = 80;            // staged past the tile: > longest
 constexpr uint32_t kDictMinLen = 4;           // the filter keys on a pattern's first 4 bytes
 constexpr uint32_t kDictMaxLen = 64;
 constexpr uint32_t kDictMaxHeavy = 32;        // patterns whose hits go to bitmaps in one search
-constexpr uint32_t kDictFilterBits = 17;      // 2^17-bit two-hash filter (16 KiB of shared memory)
+constexpr uint32_t kDictFilterBits = 17;      // 2^17-bit filter (16 KiB of shared memory)
 constexpr uint32_t kDictWordsPerTile = kDictTile / 32;
 constexpr uint32_t kDictSortChunk = 512;      // keys per warp in the light-hit radix sort
+constexpr uint32_t kDictMaxRuns = 4;          // run bytes of a set
 
 // Filter and table hashes of a pattern's first four bytes (little-endian u32);
-// the host compiler uses the same functions.
-__host__ __device__ inline uint32_t dict_filter_h1(uint32_t w) { return (w * 0x85EBCA77u) >> (32 - kDictFilterBits); }
-__host__ __device__ inline uint32_t dict_filter_h2(uint32_t w) { return (w * 0xC2B2AE3Du) >> (32 - kDictFilterBits); }
+// the host compiler uses the same functions. The filter's word holds three bits
+// of a key (bits 27.., 22.., 17.. of dict_filter_bits), so that a test is one
+// shared-memory load; with 10,000 keys it lets 1.5% of other positions through
+// (two bits in two words: 2.2%).
+__host__ __device__ inline uint32_t dict_filter_word(uint32_t w) { return (w * 0x85EBCA77u) >> (32 - kDictFilterBits + 5); }
+__host__ __device__ inline uint32_t dict_filter_bits(uint32_t w) { return w * 0xC2B2AE3Du; }
 __host__ __device__ inline uint32_t dict_table_h(uint32_t w, uint32_t bits) { return (w * 0x9E3779B1u) >> (32 - bits); }
 
 // Device view of a compiled pattern set. Patterns are deduplicated ("unique
@@ -193,28 +197,36 @@ struct DictSet {
     const uint2 *table;      // open addressing: {first 4 bytes, trie node at depth 4}; empty: .y == NONE
     uint32_t table_bits;
     uint32_t max_probe;      // longest probe distance of any key
-    const uint4 *nodes;      // {unique pattern ending here or NONE, edge count (| kDictDenseFlag),
-                             //  edge 0, edge 1 | extra start | dense table}
+    const uint4 *nodes;      // {patterns: kDictOneFlag | an index in outs, an index in lists, or NONE; edge count (| kDictDenseFlag)
+                             //  (| kDictPathFlag, run byte << 28, start in paths << 9); edge 0;
+                             //  edge 1 | extra start | dense table}
     const uint32_t *extra;   // edges 1.. of nodes with 3..kDictDenseMin children; edge = (child << 8) | byte,
                              // sorted by byte
     const uint32_t *dense;   // 256 children (NONE: no edge) per node with more than kDictDenseMin children
     uint32_t n_u;
+    // The patterns that end at a node of a run byte's trie: bit r of the 64-bit
+    // mask {x, y} for a pattern c^r rest, their u from outs[z] on, r ascending
+    // (outs ends with an unused entry).
+    const uint4 *lists;
+    const uint32_t *outs;
+    uint32_t n_outs;
+    // Run bytes c (byte j of run_bytes): their patterns c^r rest, r >= 3, hang in
+    // a trie over the rests whose root is dense table run_root[j]. A node of the
+    // other trie with kDictPathFlag has a child for c, which has one, and so on:
+    // paths holds the length K of that run, the 64-bit mask of its nodes that
+    // have a pattern (bit 0: the first), where their patterns begin in outs (one
+    // each), and the K nodes.
+    uint32_t n_runs, run_bytes;
+    uint32_t run_root[kDictMaxRuns];
+    const uint32_t *paths;
 };
 constexpr uint32_t kDictDenseMin = 8;
 constexpr uint32_t kDictDenseFlag = 0x80000000u;
-
-// A byte run in the trie: the path c^4, c^5, ..., c^K (K <= kDictMaxLen) of
-// one byte c, built per search. A walk that starts inside a run of c jumps to
-// the deepest chain node its run reaches: the heavy patterns on the way are
-// one mask, the light ones a short list.
-constexpr uint32_t kDictMaxChains = 4;
-constexpr uint32_t kDictChainMin = 8;  // shorter chains are walked node by node
-struct DictChain {
-    uint32_t byte, K, n_light, pad;
-    uint32_t node[kDictMaxLen + 1];   // trie node of c^d, d = 4..K
-    uint32_t cum[kDictMaxLen + 1];    // heavy bits of the patterns c^4 .. c^d
-    uint32_t light[kDictMaxLen + 1];  // (d << 24) | u of the light patterns on the chain, d ascending
-};
+constexpr uint32_t kDictPathFlag = 0x40000000u;
+constexpr uint32_t kDictOneFlag = 0x40000000u;  // in a node's patterns
+constexpr uint32_t kDictEdgeMask = 0x1FFu;
+constexpr uint32_t kDictPathMin = 3;          // shorter runs are walked node by node
+constexpr uint32_t kDictPathWords = 1u << 19;  // addressable words of paths (nodes past them go without)
 
 struct DictMatchArgs {
     DictSet set;
@@ -237,16 +249,17 @@ struct DictMatchArgs {
     const unsigned long long *seg_end;
     uint32_t n_seg;
     unsigned long long *stats;  // optional: += candidates walked, trie nodes visited
-    // Byte-run chains (not in count mode): n_chains of them, their bytes
-    // packed in chain_bytes (byte j = chain j's byte).
-    const DictChain *chains;
-    uint32_t n_chains;
-    uint32_t chain_bytes;
+    const uint32_t *outs;       // set.outs, with (heavy index + 1) << 16 of the heavy patterns (launch_dict_outs)
+    const uint32_t *heavy_run;  // [kDictMaxHeavy]: (j << 8) | k of a heavy run pattern run_byte(j)^k, else 0
+    const uint32_t *run_light;  // (j << 24) | (k << 16) | u of the run patterns that are not heavy (count mode: all)
+    uint32_t n_run_light;
     // Test hook (ol_ctx_inject): each block takes its wait-timeout branch
     // after its filter copy has landed, as if the bounded wait had run out.
     uint32_t force_timeout;
 };
 
+// to[i] = outs[i], with the heavy index of pattern outs[i].
+cudaError_t launch_dict_outs(const uint32_t *outs, const uint8_t *heavy_of_u, uint32_t n, uint32_t *to, cudaStream_t st);
 cudaError_t launch_dict_match(const DictMatchArgs &a, int sm_count, cudaStream_t st, uint32_t slice = 512,
                               uint32_t blocks_per_sm = 0);
 // Per (4096-word block, heavy pattern) popcounts, [n_heavy][ld] column-major.

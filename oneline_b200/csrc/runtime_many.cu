@@ -16,28 +16,24 @@
 
 using namespace ol;
 
-// The trie path of a run of one byte, as compiled: node and unique pattern
-// (or NONE) at each depth 4..K.
-struct DictRunPath {
-    uint32_t byte = 0, K = 0;
-    uint32_t node[ol::kDictMaxLen + 1] = {};
-    uint32_t u[ol::kDictMaxLen + 1] = {};
-};
-
 struct ol_patset {
     ol_ctx *ctx = nullptr;
     uint32_t n_ids = 0, n_u = 0, n_nodes = 0;
     DevBuf blob;
     DictSet dev{};
     const uint32_t *u_of_id = nullptr, *dup_start = nullptr, *dup_ids = nullptr;
-    std::vector<DictRunPath> runs;  // the longest byte runs (at most kDictMaxChains)
+    const uint32_t *d_runs = nullptr;  // device: the run patterns, as DictMatchArgs::run_light has them
+    std::vector<uint32_t> runs;        // the same on the host
 };
 
 namespace {
 
 struct TrieNode {
     std::vector<std::pair<uint8_t, uint32_t>> kids;
-    uint32_t out = NONE;
+    std::vector<uint32_t> outs;  // patterns that end here: (r << 24) | u
+    int in = -1;                 // byte of the edge from the parent (-1: an entry)
+    bool rest = false;           // in a run byte's trie
+    bool walked = false;         // walks reach it: at depth 4 or more of the other trie
 };
 
 size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
@@ -54,7 +50,7 @@ struct ManyScratch {
     uint32_t *light_n, *error, *id_counts, *sort_hist, *sort_totals;
     uint8_t *heavy_of_u;
     unsigned long long *id_base, *total, *stats;
-    DictChain *chains;
+    uint32_t *outs, *heavy_run, *run_light;
 };
 
 }  // namespace
@@ -85,13 +81,48 @@ extern "C" ol_status ol_patset_compile(ol_ctx *ctx, const ol_doc *doc, const uin
     }
     const uint32_t U = (uint32_t)u_str.size();
 
-    // Trie over the unique patterns; the node after the first four bytes of each.
-    std::vector<TrieNode> trie(1);
+    // Run bytes: the (at most four) bytes c with the most unique patterns that
+    // start with c^4. '\n' is left to the trie: a run of any other byte lies
+    // inside one document of a batch.
+    std::vector<uint32_t> starts(256, 0);
+    auto leading = [](const std::string &p) {  // length of the run that p starts with
+        size_t r = 1;
+        while (r < p.size() && p[r] == p[0]) r++;
+        return (uint32_t)r;
+    };
+    for (const std::string *p : u_str)
+        if ((*p)[0] != '\n' && leading(*p) >= 4) starts[(uint8_t)(*p)[0]]++;
+    std::vector<uint32_t> run_bytes;
+    for (uint32_t c = 0; c < 256; c++)
+        if (starts[c]) run_bytes.push_back(c);
+    std::sort(run_bytes.begin(), run_bytes.end(), [&](uint32_t x, uint32_t y) { return starts[x] > starts[y]; });
+    if (run_bytes.size() > kDictMaxRuns) run_bytes.resize(kDictMaxRuns);
+    const uint32_t n_runs = (uint32_t)run_bytes.size();
+
+    // The run bytes' tries (roots: nodes 1 .. n_runs) over what follows c^r in
+    // the patterns that start with c^3, and the trie over all other patterns
+    // (root: node 0) with the node after the first four bytes of each.
+    std::vector<TrieNode> trie(1 + n_runs);
     std::unordered_map<uint32_t, uint32_t> key_node;
+    std::vector<uint32_t> filter_keys, runs;
     for (uint32_t u = 0; u < U; u++) {
         const std::string &p = *u_str[u];
         uint32_t v = 0;
-        for (size_t j = 0; j < p.size(); j++) {
+        size_t first = 0;
+        const uint32_t r = leading(p);
+        for (uint32_t j = 0; r >= 3 && j < n_runs; j++) {
+            if (run_bytes[j] != (uint8_t)p[0]) continue;
+            v = 1 + j;
+            first = r;
+        }
+        if (v && first == p.size()) {  // c^k (k >= 4)
+            runs.push_back(((v - 1) << 24) | (r << 16) | u);
+            continue;
+        }
+        uint32_t key;
+        memcpy(&key, p.data() + (v ? first - 3 : 0), 4);  // c c c rest[0], or the first four bytes
+        filter_keys.push_back(key);
+        for (size_t j = first; j < p.size(); j++) {
             uint8_t b = (uint8_t)p[j];
             uint32_t next = NONE;
             for (auto &k : trie[v].kids)
@@ -100,26 +131,74 @@ extern "C" ol_status ol_patset_compile(ol_ctx *ctx, const ol_doc *doc, const uin
                 next = (uint32_t)trie.size();
                 trie[v].kids.emplace_back(b, next);
                 trie.emplace_back();
+                trie[next].rest = first != 0;
+                trie[next].walked = !first && j >= kDictMinLen - 1;
+                trie[next].in = j == (first ? first : kDictMinLen - 1) ? -1 : b;
             }
             v = next;
-            if (j == kDictMinLen - 1) {
-                uint32_t key;
-                memcpy(&key, p.data(), 4);
-                key_node[key] = v;
-            }
+            if (!first && j == kDictMinLen - 1) key_node[key] = v;
         }
-        trie[v].out = u;
+        trie[v].outs.push_back(((first ? r : 0u) << 24) | u);
     }
     const uint32_t n_nodes = (uint32_t)trie.size();
     if (n_nodes >= (1u << 24)) return ctx_fail(ctx, OL_ERR_BAD_PATTERN, "pattern set too large for the trie");
     std::vector<uint4> nodes(n_nodes);
-    std::vector<uint32_t> extra, dense;
+    std::vector<uint32_t> extra, dense, outs, paths, path_of(n_nodes, NONE);
+    std::vector<uint4> lists;
+    // The runs of run bytes in the trie (kDictPathFlag), and their nodes' patterns.
+    for (uint32_t v = n_runs + 1; v < n_nodes; v++) nodes[v].x = NONE;
+    for (uint32_t v = n_runs + 1; v < n_nodes; v++) {
+        for (uint32_t j = 0; j < n_runs && path_of[v] == NONE && trie[v].walked; j++) {
+            if (trie[v].in == (int)run_bytes[j]) continue;  // the run begins before v
+            std::vector<uint32_t> run;
+            for (uint32_t x = v; x != NONE;) {
+                uint32_t next = NONE;
+                for (auto &e : trie[x].kids)
+                    if (e.first == run_bytes[j]) next = e.second;
+                if (next != NONE) run.push_back(next);
+                x = next;
+            }
+            if (run.size() < kDictPathMin || paths.size() + 4 + run.size() > kDictPathWords) continue;
+            path_of[v] = (j << 28) | ((uint32_t)paths.size() << 9);
+            uint64_t mask = 0;
+            const uint32_t first = (uint32_t)outs.size();
+            for (uint32_t i = 0; i < run.size(); i++) {  // at most 60
+                const TrieNode &x = trie[run[i]];
+                if (x.outs.empty()) continue;
+                mask |= 1ull << i;
+                nodes[run[i]].x = kDictOneFlag | (uint32_t)outs.size();
+                outs.push_back(x.outs[0]);
+            }
+            paths.insert(paths.end(), {(uint32_t)run.size(), (uint32_t)mask, (uint32_t)(mask >> 32), first});
+            paths.insert(paths.end(), run.begin(), run.end());
+        }
+    }
+    for (uint32_t v = 0; v < n_nodes; v++) {
+        auto &o = trie[v].outs;
+        if (v <= n_runs) nodes[v].x = NONE;
+        if (o.empty() || nodes[v].x != NONE) continue;
+        if (!trie[v].rest) {  // one pattern: they are unique
+            nodes[v].x = kDictOneFlag | (uint32_t)outs.size();
+            outs.push_back(o[0]);
+            continue;
+        }
+        std::sort(o.begin(), o.end());  // r ascending, 3..63
+        nodes[v].x = (uint32_t)lists.size();
+        uint4 l{0, 0, (uint32_t)outs.size(), 0};
+        for (uint32_t x : o) {
+            (x >> 24 < 32 ? l.x : l.y) |= 1u << ((x >> 24) & 31);
+            outs.push_back(x & 0xFFFFFFu);
+        }
+        lists.push_back(l);
+    }
+    outs.push_back(0);
     for (uint32_t v = 0; v < n_nodes; v++) {
         auto &k = trie[v].kids;
         std::sort(k.begin(), k.end());
-        uint4 r{trie[v].out, (uint32_t)k.size(), 0, 0};
+        uint4 r{nodes[v].x, (uint32_t)k.size(), 0, 0};
+        if (path_of[v] != NONE) r.y |= kDictPathFlag | path_of[v];
         auto pack = [](const std::pair<uint8_t, uint32_t> &e) { return (e.second << 8) | e.first; };
-        if (k.size() > kDictDenseMin) {
+        if (k.size() > kDictDenseMin || (v >= 1 && v <= n_runs)) {
             // many children: a 256-entry table, one load per step
             r.y |= kDictDenseFlag;
             r.w = (uint32_t)(dense.size() / 256);
@@ -137,46 +216,20 @@ extern "C" ol_status ol_patset_compile(ol_ctx *ctx, const ol_doc *doc, const uin
     }
     if (extra.empty()) extra.push_back(0);
     if (dense.empty()) dense.push_back(NONE);
+    if (paths.empty()) paths.push_back(0);
 
-    // Byte runs: the trie path c^4, c^5, ... of each byte c that starts a
-    // pattern with c^4; the longest ones (at least kDictChainMin deep) let
-    // walks inside long runs of c skip down the path (dict_walk).
-    std::vector<DictRunPath> runs;
-    for (uint32_t c = 0; c < 256; c++) {
-        auto it = key_node.find(c * 0x01010101u);
-        if (it == key_node.end()) continue;
-        DictRunPath r;
-        r.byte = c;
-        uint32_t v = it->second, d = kDictMinLen;
-        r.node[d] = v;
-        r.u[d] = trie[v].out;
-        while (d < kDictMaxLen) {
-            uint32_t next = NONE;
-            for (auto &k : trie[v].kids)
-                if (k.first == c) next = k.second;
-            if (next == NONE) break;
-            v = next;
-            d++;
-            r.node[d] = v;
-            r.u[d] = trie[v].out;
-        }
-        r.K = d;
-        if (r.K >= kDictChainMin) runs.push_back(r);
-    }
-    std::sort(runs.begin(), runs.end(), [](const DictRunPath &x, const DictRunPath &y) { return x.K > y.K; });
-    if (runs.size() > kDictMaxChains) runs.resize(kDictMaxChains);
-
-    // Filter and hash table over the distinct first-four-byte keys.
+    // The filter, and the hash table over the distinct first-four-byte keys.
     std::vector<uint32_t> filter(1u << (kDictFilterBits - 5), 0);
     uint32_t table_bits = 10;
     while ((1u << table_bits) < 2 * key_node.size()) table_bits++;
     std::vector<uint2> table(1u << table_bits, make_uint2(0, NONE));
     uint32_t max_probe = 0;
+    for (uint32_t key : filter_keys) {
+        const uint32_t g = dict_filter_bits(key);
+        filter[dict_filter_word(key)] |= (1u << (g >> 27)) | (1u << ((g >> 22) & 31)) | (1u << ((g >> 17) & 31));
+    }
     for (auto &kv : key_node) {
         uint32_t key = kv.first;
-        uint32_t h1 = dict_filter_h1(key), h2 = dict_filter_h2(key);
-        filter[h1 >> 5] |= 1u << (h1 & 31);
-        filter[h2 >> 5] |= 1u << (h2 & 31);
         uint32_t slot = dict_table_h(key, table_bits), dist = 0;
         while (table[slot].y != NONE) {
             slot = (slot + 1) & ((1u << table_bits) - 1);
@@ -204,7 +257,11 @@ extern "C" ol_status ol_patset_compile(ol_ctx *ctx, const ol_doc *doc, const uin
     size_t off_uid = align256(off_dense + sz_dense), sz_uid = (size_t)n * 4;
     size_t off_ds = align256(off_uid + sz_uid), sz_ds = dup_start.size() * 4;
     size_t off_di = align256(off_ds + sz_ds), sz_di = dup_ids.size() * 4;
-    size_t total = align256(off_di + sz_di);
+    size_t off_outs = align256(off_di + sz_di), sz_outs = outs.size() * 4;
+    size_t off_runs = align256(off_outs + sz_outs), sz_runs = runs.size() * 4;
+    size_t off_paths = align256(off_runs + std::max<size_t>(sz_runs, 4)), sz_paths = paths.size() * 4;
+    size_t off_lists = align256(off_paths + sz_paths), sz_lists = lists.size() * sizeof(uint4);
+    size_t total = align256(off_lists + sz_lists);
     std::vector<uint8_t> host(total, 0);
     memcpy(host.data() + off_filter, filter.data(), sz_filter);
     memcpy(host.data() + off_table, table.data(), sz_table);
@@ -214,6 +271,10 @@ extern "C" ol_status ol_patset_compile(ol_ctx *ctx, const ol_doc *doc, const uin
     memcpy(host.data() + off_uid, u_of_id.data(), sz_uid);
     memcpy(host.data() + off_ds, dup_start.data(), sz_ds);
     memcpy(host.data() + off_di, dup_ids.data(), sz_di);
+    memcpy(host.data() + off_outs, outs.data(), sz_outs);
+    if (sz_runs) memcpy(host.data() + off_runs, runs.data(), sz_runs);
+    memcpy(host.data() + off_paths, paths.data(), sz_paths);
+    if (sz_lists) memcpy(host.data() + off_lists, lists.data(), sz_lists);
 
     std::lock_guard<std::recursive_mutex> g(ctx->mu);
     cudaSetDevice(ctx->device);
@@ -242,6 +303,16 @@ extern "C" ol_status ol_patset_compile(ol_ctx *ctx, const ol_doc *doc, const uin
     s->u_of_id = (const uint32_t *)(b + off_uid);
     s->dup_start = (const uint32_t *)(b + off_ds);
     s->dup_ids = (const uint32_t *)(b + off_di);
+    s->dev.lists = (const uint4 *)(b + off_lists);
+    s->dev.outs = (const uint32_t *)(b + off_outs);
+    s->dev.n_outs = (uint32_t)outs.size();
+    s->dev.paths = (const uint32_t *)(b + off_paths);
+    s->dev.n_runs = n_runs;
+    for (uint32_t j = 0; j < n_runs; j++) {
+        s->dev.run_bytes |= run_bytes[j] << (8 * j);
+        s->dev.run_root[j] = nodes[1 + j].w;
+    }
+    s->d_runs = (const uint32_t *)(b + off_runs);
     s->runs = std::move(runs);
     *out = s;
     return OL_OK;
@@ -289,7 +360,8 @@ ol_status ol::many_run(ol_ctx *ctx, const ol_doc *d, const ol_patset *set, uint6
     size_t o_hcounts = carve(at, (size_t)kDictMaxHeavy * hld * 4), o_hbases = carve(at, (size_t)kDictMaxHeavy * hld * 4);
     size_t o_ln = carve(at, 16), o_idc = carve(at, (size_t)n * 4), o_idb = carve(at, (size_t)n * 8), o_tot = carve(at, 16);
     size_t o_stot = carve(at, 256 * 4), o_stats = carve(at, 16);
-    size_t o_chains = carve(at, kDictMaxChains * sizeof(DictChain));
+    size_t o_outs = carve(at, (size_t)set->dev.n_outs * 4);
+    size_t o_hrun = carve(at, kDictMaxHeavy * 4), o_rlight = carve(at, std::max<size_t>(set->runs.size(), 1) * 4);
     const size_t fixed = at;
     cudaError_t e = ctx->dict_small.reserve(fixed, st);
     if (e != cudaSuccess) return ctx_cuda(ctx, e, "search_many");
@@ -310,7 +382,9 @@ ol_status ol::many_run(ol_ctx *ctx, const ol_doc *d, const ol_patset *set, uint6
         m.total = (unsigned long long *)(b + o_tot);
         m.sort_totals = (uint32_t *)(b + o_stot);
         m.stats = (unsigned long long *)(b + o_stats);
-        m.chains = (DictChain *)(b + o_chains);
+        m.outs = (uint32_t *)(b + o_outs);
+        m.heavy_run = (uint32_t *)(b + o_hrun);
+        m.run_light = (uint32_t *)(b + o_rlight);
         m.sort_hist = (uint32_t *)(b + fixed);
         return m;
     };
@@ -329,6 +403,9 @@ ol_status ol::many_run(ol_ctx *ctx, const ol_doc *d, const ol_patset *set, uint6
     ma.count_only = 1;
     ma.counts = m.sample_counts;
     ma.error = m.error;
+    ma.outs = set->dev.outs;
+    ma.run_light = set->d_runs;
+    ma.n_run_light = (uint32_t)set->runs.size();
     ma.seg_start = seg_start;
     ma.seg_end = seg_end;
     ma.n_seg = n_seg;
@@ -372,34 +449,21 @@ ol_status ol::many_run(ol_ctx *ctx, const ol_doc *d, const ol_patset *set, uint6
         heavy_u[h] = cand[h].second;
         heavy_of[cand[h].second] = (uint8_t)h;
     }
-    // The byte-run chains of this search: heavy bits accumulated down each run,
-    // and its light patterns.
-    std::vector<DictChain> chains(set->runs.size());
-    uint32_t chain_bytes = 0;
-    for (size_t j = 0; j < set->runs.size(); j++) {
-        const DictRunPath &r = set->runs[j];
-        DictChain &c = chains[j];
-        memset(&c, 0, sizeof c);
-        c.byte = r.byte;
-        c.K = r.K;
-        chain_bytes |= r.byte << (8 * j);
-        uint32_t acc = 0;
-        for (uint32_t dd = kDictMinLen; dd <= r.K; dd++) {
-            c.node[dd] = r.node[dd];
-            const uint32_t u = r.u[dd];
-            if (u != NONE) {
-                if (heavy_of[u] != 0xFF)
-                    acc |= 1u << heavy_of[u];
-                else
-                    c.light[c.n_light++] = (dd << 24) | u;
-            }
-            c.cum[dd] = acc;
-        }
+    // The run patterns: heavy ones by heavy index, the others listed.
+    std::vector<uint32_t> heavy_run(kDictMaxHeavy, 0), run_light;
+    for (uint32_t x : set->runs) {
+        const uint8_t h = heavy_of[x & 0xFFFFu];
+        if (h != 0xFF)
+            heavy_run[h] = x >> 16;
+        else
+            run_light.push_back(x);
     }
     e = cudaMemcpyAsync(m.heavy_of_u, heavy_of.data(), U, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess && !chains.empty())
-        e = cudaMemcpyAsync(m.chains, chains.data(), chains.size() * sizeof(DictChain), cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(m.heavy_run, heavy_run.data(), kDictMaxHeavy * 4, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess && !run_light.empty())
+        e = cudaMemcpyAsync(m.run_light, run_light.data(), run_light.size() * 4, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(m.heavy_u, heavy_u.data(), kDictMaxHeavy * 4, cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = launch_dict_outs(set->dev.outs, m.heavy_of_u, set->dev.n_outs, m.outs, st);
     if (e == cudaSuccess && H) e = ctx->dict_bitmap.reserve((size_t)H * n_words * 4, st);
     if (e != cudaSuccess) return ctx_cuda(ctx, e, "search_many");
 
@@ -422,9 +486,10 @@ ol_status ol::many_run(ol_ctx *ctx, const ol_doc *d, const ol_patset *set, uint6
         ma.light_keys = (unsigned long long *)ctx->dict_keys.ptr;
         ma.light_cap = (uint32_t)cap;
         ma.light_n = m.light_n;
-        ma.chains = m.chains;
-        ma.n_chains = (uint32_t)chains.size();
-        ma.chain_bytes = chain_bytes;
+        ma.outs = m.outs;
+        ma.heavy_run = m.heavy_run;
+        ma.run_light = m.run_light;
+        ma.n_run_light = (uint32_t)run_light.size();
         if (e == cudaSuccess) {
             GpuPass pass(ctx, "dictionary: match");
             e = launch_dict_match(ma, ctx->sm_count, st, ctx->tune.dict_slice, ctx->tune.dict_blocks_per_sm);
