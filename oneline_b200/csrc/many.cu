@@ -390,7 +390,8 @@ __global__ void __launch_bounds__(DM_THREADS, 2) dict_match_kernel(const __grid_
 
     const uint64_t N = a.text_len;
     const uint32_t n_words = a.n_tiles * kDictWordsPerTile;
-    const uint32_t n_items = ((a.n_tiles + a.tile_stride - 1) / a.tile_stride) * DM_SLICES_PER_TILE;
+    const uint32_t per_tile = DM_SLICES_PER_TILE / a.slices;  // items of a tile, of a.slices slices each
+    const uint32_t n_items = ((a.n_tiles + a.tile_stride - 1) / a.tile_stride) * per_tile;
     const uint32_t H = a.count_only ? 0u : a.n_heavy, n_runs = a.set.n_runs, run_bytes = a.set.run_bytes;
     uint32_t cands = 0, levels = 0;  // per lane, for the search statistics
     Warp &w = sm.w[warp];
@@ -406,8 +407,10 @@ __global__ void __launch_bounds__(DM_THREADS, 2) dict_match_kernel(const __grid_
     if (lane < H && H)
         for (uint32_t i = 0; i < Warp::kWords; i += 4) *reinterpret_cast<uint4 *>(&w.bits[lane][i]) = make_uint4(0, 0, 0, 0);
 
-    for (uint32_t item = blockIdx.x * n_warps + warp; item < n_items; item += gridDim.x * n_warps) {
-        const uint32_t slice = (item / DM_SLICES_PER_TILE) * a.tile_stride * DM_SLICES_PER_TILE + item % DM_SLICES_PER_TILE;
+    // item by item, slice by slice; `found`: the item's hits of heavy pattern `lane`
+    for (uint32_t item = blockIdx.x * n_warps + warp, nth = 0, found = 0; item < n_items;) {
+        const uint32_t tile = (item / per_tile) * a.tile_stride;
+        const uint32_t slice = tile * DM_SLICES_PER_TILE + (item % per_tile) * a.slices + nth;
         const uint64_t s0 = (uint64_t)slice * SLICE;  // slices past the text only write zero words
         constexpr uint32_t kPieces = SLICE / 16, kMine = (kPieces + 31) / 32;  // 16-byte pieces; a lane's
         uint4 v[kMine];
@@ -575,9 +578,16 @@ __global__ void __launch_bounds__(DM_THREADS, 2) dict_match_kernel(const __grid_
             uint4 *src = reinterpret_cast<uint4 *>(w.bits[lane]);
 #pragma unroll
             for (uint32_t i = 0; i < Warp::kWords / 4; i++) {
-                dst[i] = src[i];
+                const uint4 x = src[i];
+                found += __popc(x.x) + __popc(x.y) + __popc(x.z) + __popc(x.w);
+                dst[i] = x;
                 src[i] = make_uint4(0, 0, 0, 0);
             }
+        }
+        if (++nth == a.slices) {
+            if (found) atomicAdd(a.heavy_counts + (size_t)lane * a.heavy_ld + tile, found);  // (lane < H)
+            nth = found = 0;
+            item += gridDim.x * n_warps;
         }
     }
     if (!a.count_only) dict_flush(a, w, 1);
@@ -591,8 +601,9 @@ __global__ void __launch_bounds__(DM_THREADS, 2) dict_match_kernel(const __grid_
 }
 
 template <uint32_t SLICE>
-static cudaError_t launch_match(const DictMatchArgs &a, int sm_count, uint32_t blocks_per_sm, cudaStream_t st) {
-    const uint64_t n_items = (uint64_t)((a.n_tiles + a.tile_stride - 1) / a.tile_stride) * (kDictTile / SLICE);
+static cudaError_t launch_match(const DictMatchArgs &args, int sm_count, uint32_t blocks_per_sm, cudaStream_t st) {
+    DictMatchArgs a = args;
+    uint64_t n_items = (uint64_t)((a.n_tiles + a.tile_stride - 1) / a.tile_stride) * (kDictTile / SLICE);
     const bool small = n_items <= (uint64_t)sm_count * DM_SMALL_WARPS_PER_SM;
     const uint32_t threads = small ? DM_SMALL_THREADS : DM_THREADS, warps = threads / 32;
     const size_t smem = DictSmem<SLICE>::bytes(threads);
@@ -606,6 +617,13 @@ static cudaError_t launch_match(const DictMatchArgs &a, int sm_count, uint32_t b
         if (e != cudaSuccess) return e;
         if (blocks_per_sm) per_sm = std::min<int>(per_sm, (int)blocks_per_sm);
         grid = std::min<uint64_t>(grid, (uint64_t)std::max(per_sm, 1) * sm_count);
+    }
+    // items of several slices, as long as every warp gets a few dozen of them:
+    // the heavy hits of an item are counted in registers
+    a.slices = 1;
+    while (a.slices < 8 && a.slices * 2 * SLICE <= kDictTile && n_items >= grid * warps * 32) {
+        a.slices *= 2;
+        n_items /= 2;
     }
     dict_match_kernel<SLICE><<<(uint32_t)grid, threads, smem, st>>>(a); OL_LAUNCHED();
     return cudaGetLastError();
@@ -636,13 +654,7 @@ cudaError_t launch_dict_outs(const uint32_t *outs, const uint8_t *heavy_of_u, ui
     return cudaGetLastError();
 }
 
-// ------------------------------------------------------------ heavy ranks --
-
 constexpr uint32_t DH_THREADS = 256;
-constexpr uint32_t DH_WORDS_PER_THREAD = 16;
-constexpr uint32_t DH_WORDS = DH_THREADS * DH_WORDS_PER_THREAD;  // 4096 words per block
-
-uint32_t dict_heavy_blocks(uint32_t n_words) { return (n_words + DH_WORDS - 1) / DH_WORDS; }
 
 // Block sum / exclusive scan helpers for 256 threads.
 __device__ __forceinline__ uint32_t block_exclusive_256(uint32_t x, uint32_t *warp_sum, uint32_t *total) {
@@ -665,34 +677,6 @@ __device__ __forceinline__ uint32_t block_exclusive_256(uint32_t x, uint32_t *wa
     __syncthreads();
     if (total) *total = all;
     return before + inc - x;
-}
-
-__global__ void __launch_bounds__(DH_THREADS) dict_heavy_count_kernel(const uint32_t *__restrict__ bitmap,
-                                                                       uint32_t n_words, uint32_t *counts,
-                                                                       uint32_t ld) {
-    __shared__ uint32_t warp_sum[DH_THREADS / 32];
-    const uint32_t h = blockIdx.y, b = blockIdx.x;
-    const uint32_t w0 = b * DH_WORDS + threadIdx.x * DH_WORDS_PER_THREAD;
-    const uint32_t *col = bitmap + (size_t)h * n_words;
-    uint32_t c = 0;
-    if (w0 < n_words) {  // n_words is a multiple of 512: a thread's 16 words are all in range
-#pragma unroll
-        for (uint32_t i = 0; i < DH_WORDS_PER_THREAD; i += 4) {
-            uint4 q = __ldg(reinterpret_cast<const uint4 *>(col + w0 + i));
-            c += __popc(q.x) + __popc(q.y) + __popc(q.z) + __popc(q.w);
-        }
-    }
-    uint32_t total;
-    block_exclusive_256(c, warp_sum, &total);
-    if (threadIdx.x == 0) counts[(size_t)h * ld + b] = total;
-}
-
-cudaError_t launch_dict_heavy_count(const uint32_t *bitmap, uint32_t n_words, uint32_t n_heavy, uint32_t *counts,
-                                    uint32_t ld, cudaStream_t st) {
-    if (n_heavy == 0 || n_words == 0) return cudaSuccess;
-    dim3 grid(dict_heavy_blocks(n_words), n_heavy);
-    dict_heavy_count_kernel<<<grid, DH_THREADS, 0, st>>>(bitmap, n_words, counts, ld); OL_LAUNCHED();
-    return cudaGetLastError();
 }
 
 // ---------------------------------------------------- light-key radix sort --
@@ -865,7 +849,6 @@ cudaError_t launch_dict_ids(const DictEmitArgs &a, cudaStream_t st) {
 // (pattern u32, offset u64) pair of arrays. Streaming stores: the emission
 // never reads them back.
 __device__ __forceinline__ void put_hit(const DictEmitArgs &a, unsigned long long slot, uint32_t id, uint32_t off) {
-    if (slot >= a.max_hits) return;
     if (a.hit_off) {
         __stcs(a.hit_pat + slot, id);
         __stcs(a.hit_off + slot, (unsigned long long)off);
@@ -874,91 +857,111 @@ __device__ __forceinline__ void put_hit(const DictEmitArgs &a, unsigned long lon
     }
 }
 
-// Heavy hits: block (b, h) expands words [4096b, 4096b + 4096) of bitmap h,
-// warp w the 512 words [4096b + 512w, ...), 32 words per round. Each lane
-// lists its word's hits, at their ranks from a warp scan of the popcounts, in
-// the warp's shared buffer; the warp then writes the round's hits to
-// consecutive slots, so every store instruction covers 32 consecutive hits.
+// Heavy hits: a warp expands the 512 bitmap words of one tile of one heavy
+// pattern (a tile without hits, known from the match pass's counts, is left at
+// once), 128 words a round, four a lane: one scan of the lanes' popcounts gives
+// every hit its rank, each lane lists its words' hits in the warp's buffer, and
+// the warp writes them to consecutive slots, for one id after the other. Four
+// words a lane instead of one make a round's scan, and its longest lane, count
+// for four times the hits.
+// What bounds it is the writing of 8 bytes a hit: a plain fill runs at 7.1 TB/s
+// in one region, but the ids of one unique pattern are as many regions written
+// at a time, and a kernel that only stores reaches 4.9 TB/s into 12 of them
+// this way. 256 MiB, 10,000 patterns, 7.7 GB of hits: 2.28 ms with one word a
+// lane and the block's words read twice, 1.79 ms (4.3 TB/s) now. Blocks of one,
+// two or four tiles that list first and write one stretch per id then took 1.81
+// to 2.0 ms; listing again for every one to four ids, 1.8 to 3.3 ms.
 // The ids of a unique pattern and their first output slots are read once per
-// block into shared memory (up to DH_MAX_DUPS of them), not once per 32 hits.
+// block into shared memory (up to DH_MAX_DUPS of them).
 constexpr uint32_t DH_MAX_DUPS = 64;
+constexpr uint32_t DH_BUF = 1024;  // hits listed at a time
 
-__global__ void __launch_bounds__(DH_THREADS) dict_emit_heavy_kernel(DictEmitArgs a) {
-    __shared__ uint32_t warp_tot[DH_THREADS / 32];
+// A run of n listed hits of one id into consecutive slots, by one warp; four
+// stores in flight per lane.
+template <bool PAIR>
+__device__ __forceinline__ void put_run(const DictEmitArgs &a, unsigned long long slot, uint32_t id, uint32_t text0,
+                                        const uint16_t *buf, uint32_t n) {
+    uint2 *hits = a.hits + slot;
+    uint32_t *pat = a.hit_pat + slot;
+    unsigned long long *off = a.hit_off + slot;
+    auto put = [&](uint32_t j, uint32_t x) {
+        if (PAIR) {
+            __stcs(pat + j, id);
+            __stcs(off + j, (unsigned long long)x);
+        } else {
+            __stcs(hits + j, make_uint2(id, x));
+        }
+    };
+    uint32_t j = threadIdx.x & 31;
+    for (; j + 96 < n; j += 128) {
+        uint32_t x[4];
+#pragma unroll
+        for (uint32_t i = 0; i < 4; i++) x[i] = text0 + buf[j + 32 * i];
+#pragma unroll
+        for (uint32_t i = 0; i < 4; i++) put(j + 32 * i, x[i]);
+    }
+    for (; j < n; j += 32) put(j, text0 + buf[j]);
+}
+
+template <bool PAIR>
+__global__ void __launch_bounds__(DH_THREADS, 6) dict_emit_heavy_kernel(DictEmitArgs a) {
     __shared__ uint32_t dup_id[DH_MAX_DUPS];
     __shared__ unsigned long long dup_base[DH_MAX_DUPS];
-    __shared__ uint32_t hit_buf[DH_THREADS / 32][32 * 32];  // per warp: one round's hit offsets, in order
-    const uint32_t h = blockIdx.y, b = blockIdx.x;
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t *buf = hit_buf[warp];
-    const uint32_t *col = a.bitmap + (size_t)h * a.n_words;
+    __shared__ uint16_t hit_buf[DH_THREADS / 32][DH_BUF];  // per warp: hit offsets in the tile, in order
+    const uint32_t h = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t tile = blockIdx.x * (DH_THREADS / 32) + warp;
     const uint32_t u = a.heavy_u[h];
-    const uint32_t d0 = a.dup_start[u], d1 = a.dup_start[u + 1];
-    const uint32_t n_dup = d1 - d0;
+    const uint32_t d0 = a.dup_start[u], n_dup = a.dup_start[u + 1] - d0;
     const bool cached = n_dup <= DH_MAX_DUPS;
     if (cached && threadIdx.x < n_dup) {
         const uint32_t id = __ldg(a.dup_ids + d0 + threadIdx.x);
         dup_id[threadIdx.x] = id;
         dup_base[threadIdx.x] = a.id_base[id];
     }
-    const uint32_t w0 = b * DH_WORDS + warp * (DH_WORDS / (DH_THREADS / 32));
-    constexpr uint32_t kRounds = DH_WORDS / (DH_THREADS / 32) / 32;  // 16
-    uint32_t c = 0;
-    for (uint32_t r = 0; r < kRounds; r++) {
-        const uint32_t idx = w0 + r * 32 + lane;
-        c += idx < a.n_words ? __popc(__ldg(col + idx)) : 0u;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xFFFFFFFFu, c, o);
-    if (lane == 0) warp_tot[warp] = c;
     __syncthreads();
-    uint32_t rank = a.heavy_bases[(size_t)h * a.ld + b];
-    for (uint32_t w = 0; w < warp; w++) rank += warp_tot[w];
-    if (c == 0) return;  // uniform over the warp
-    // each round's bitmap word is loaded a round ahead, so its latency hides
-    // behind the previous round's listing and stores
-    uint32_t nxt = w0 + lane < a.n_words ? __ldg(col + w0 + lane) : 0u;
+    if (tile >= a.n_tiles || a.heavy_counts[(size_t)h * a.ld + tile] == 0) return;  // uniform over the warp
+    uint16_t *buf = hit_buf[warp];
+    unsigned long long rank = a.heavy_bases[(size_t)h * a.ld + tile];
+    constexpr uint32_t kRounds = kDictWordsPerTile / 128;
+    const uint4 *col = reinterpret_cast<const uint4 *>(a.bitmap + ((size_t)h * a.n_tiles + tile) * kDictWordsPerTile);
+    uint4 words[kRounds];
+#pragma unroll
+    for (uint32_t r = 0; r < kRounds; r++) words[r] = __ldcs(col + r * 32 + lane);
+#pragma unroll
     for (uint32_t r = 0; r < kRounds; r++) {
-        const uint32_t idx = w0 + r * 32 + lane;
-        const uint32_t word = nxt;
-        if (r + 1 < kRounds) nxt = idx + 32 < a.n_words ? __ldg(col + idx + 32) : 0u;
-        const uint32_t cnt = __popc(word);
+        const uint32_t x[4] = {words[r].x, words[r].y, words[r].z, words[r].w};
+        const uint32_t cnt = __popc(x[0]) + __popc(x[1]) + __popc(x[2]) + __popc(x[3]);
         uint32_t inc = cnt;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            uint32_t t = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+            const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, inc, o);
             if ((int)lane >= o) inc += t;
         }
-        const uint32_t excl = inc - cnt;
-        const uint32_t T = __shfl_sync(0xFFFFFFFFu, inc, 31);  // <= 1024
-        // each lane lists its word's hit offsets at their ranks in the warp's
-        // buffer; then the warp writes them, 32 consecutive hits per store
-        {
-            uint32_t bits = word, r2 = excl;
-            const uint32_t wbase = idx * 32;
-            while (bits) {
-                const uint32_t bb = __ffs(bits) - 1;
-                bits &= bits - 1;
-                buf[r2++] = wbase + bb;
-            }
-        }
-        __syncwarp();
-        for (uint32_t base = 0; base < T; base += 32) {
-            const uint32_t j = base + lane;
-            if (j < T) {
-                const uint32_t off = buf[j];
-                if (cached) {
-                    for (uint32_t d = 0; d < n_dup; d++) put_hit(a, dup_base[d] + rank + j, dup_id[d], off);
-                } else {
-                    for (uint32_t d = d0; d < d1; d++) {
-                        const uint32_t id = __ldg(a.dup_ids + d);
-                        put_hit(a, a.id_base[id] + rank + j, id, off);
-                    }
+        const uint32_t all = __shfl_sync(0xFFFFFFFFu, inc, 31);
+        // all lanes at once when the buffer holds their hits, else eight lanes
+        // (at most 1024 hits) after the other
+        const uint32_t step = all <= DH_BUF ? 32 : 8;
+        for (uint32_t g = 0; g < 32 && all; g += step) {
+            const uint32_t before = g ? __shfl_sync(0xFFFFFFFFu, inc, g - 1) : 0u;
+            const uint32_t T = __shfl_sync(0xFFFFFFFFu, inc, g + step - 1) - before;
+            if (lane >= g && lane < g + step) {
+                uint32_t at = inc - cnt - before;
+#pragma unroll
+                for (uint32_t i = 0; i < 4; i++) {
+                    const uint32_t base = (r * 128 + lane * 4 + i) * 32;
+                    for (uint32_t bits = x[i]; bits; bits &= bits - 1) buf[at++] = (uint16_t)(base + __ffs(bits) - 1);
                 }
             }
+            __syncwarp();
+            for (uint32_t d = 0; d < n_dup; d++) {
+                const uint32_t id = cached ? dup_id[d] : __ldg(a.dup_ids + d0 + d);
+                const unsigned long long slot = (cached ? dup_base[d] : a.id_base[id]) + rank;
+                const uint32_t n = slot >= a.max_hits ? 0u : (uint32_t)min((unsigned long long)T, a.max_hits - slot);
+                put_run<PAIR>(a, slot, id, tile * kDictTile, buf, n);
+            }
+            __syncwarp();  // the buffer is filled again
+            rank += T;
         }
-        __syncwarp();  // the buffer is refilled by the next round
-        rank += T;
     }
 }
 
@@ -971,15 +974,20 @@ __global__ void dict_emit_light_kernel(DictEmitArgs a) {
     const uint32_t d0 = a.dup_start[u], d1 = a.dup_start[u + 1];
     for (uint32_t d = d0; d < d1; d++) {
         const uint32_t id = a.dup_ids[d];
-        put_hit(a, a.id_base[id] + rank, id, off);
+        const unsigned long long slot = a.id_base[id] + rank;
+        if (slot < a.max_hits) put_hit(a, slot, id, off);
     }
 }
 
 cudaError_t launch_dict_emit(const DictEmitArgs &a, cudaStream_t st) {
     if (a.max_hits == 0) return cudaSuccess;
-    if (a.n_heavy && a.n_words) {
-        dim3 grid(dict_heavy_blocks(a.n_words), a.n_heavy);
-        dict_emit_heavy_kernel<<<grid, DH_THREADS, 0, st>>>(a); OL_LAUNCHED();
+    if (a.n_heavy && a.n_tiles) {
+        dim3 grid((a.n_tiles + DH_THREADS / 32 - 1) / (DH_THREADS / 32), a.n_heavy);
+        if (a.hit_off) {
+            dict_emit_heavy_kernel<true><<<grid, DH_THREADS, 0, st>>>(a); OL_LAUNCHED();
+        } else {
+            dict_emit_heavy_kernel<false><<<grid, DH_THREADS, 0, st>>>(a); OL_LAUNCHED();
+        }
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }

@@ -239,6 +239,9 @@ struct DictMatchArgs {
     const uint8_t *heavy_of_u;  // heavy index or 0xFF
     uint32_t n_heavy;
     uint32_t *bitmap;        // [n_heavy][n_tiles * kDictWordsPerTile]
+    uint32_t *heavy_counts;  // [n_heavy][heavy_ld]: += hits per tile
+    uint32_t heavy_ld;
+    uint32_t slices;         // consecutive slices per item (set by the launch)
     unsigned long long *light_keys;  // (u << 32) | offset, unordered
     uint32_t light_cap;
     uint32_t *light_n;
@@ -262,10 +265,6 @@ struct DictMatchArgs {
 cudaError_t launch_dict_outs(const uint32_t *outs, const uint8_t *heavy_of_u, uint32_t n, uint32_t *to, cudaStream_t st);
 cudaError_t launch_dict_match(const DictMatchArgs &a, int sm_count, cudaStream_t st, uint32_t slice = 512,
                               uint32_t blocks_per_sm = 0);
-// Per (4096-word block, heavy pattern) popcounts, [n_heavy][ld] column-major.
-cudaError_t launch_dict_heavy_count(const uint32_t *bitmap, uint32_t n_words, uint32_t n_heavy, uint32_t *counts,
-                                    uint32_t ld, cudaStream_t st);
-uint32_t dict_heavy_blocks(uint32_t n_words);
 // Stable LSD radix sort of n 64-bit keys on bits [0, key_bits), 8 per pass;
 // the result ends in keys (tmp is the other buffer); hist needs
 // 2 * 256 * scan_ld(chunks) words and digit totals 256 words.
@@ -274,14 +273,14 @@ cudaError_t launch_dict_sort(unsigned long long *keys, unsigned long long *tmp, 
 uint32_t dict_sort_chunks(uint32_t n);
 
 struct DictEmitArgs {
-    uint32_t n_ids, n_u, n_heavy, n_words;
+    uint32_t n_ids, n_u, n_heavy, n_tiles;
     const uint32_t *u_of_id;
     const uint32_t *dup_start;   // [n_u + 1]
     const uint32_t *dup_ids;     // ids grouped by unique pattern, ascending
     const uint8_t *heavy_of_u;
     const uint32_t *heavy_u;     // [n_heavy]
     const uint32_t *heavy_totals;
-    const uint32_t *heavy_bases; // [n_heavy][ld]
+    const uint32_t *heavy_counts, *heavy_bases;  // [n_heavy][ld], per tile
     uint32_t ld;
     const uint32_t *bitmap;
     const uint32_t *light_count; // [n_u]

@@ -346,7 +346,7 @@ ol_status ol::many_run(ol_ctx *ctx, const ol_doc *d, const ol_patset *set, uint6
     if (N < kDictMinLen) return OL_OK;
     const uint32_t n_tiles = (uint32_t)((N + kDictTile - 1) / kDictTile);
     const uint32_t n_words = n_tiles * kDictWordsPerTile;
-    const uint32_t hblocks = dict_heavy_blocks(n_words), hld = scan_ld(hblocks);
+    const uint32_t hld = scan_ld(n_tiles);
 
     // Small scratch (sort histograms sized for the worst light count: grown below if needed).
     auto carve = [](size_t &at, size_t bytes) {
@@ -475,6 +475,9 @@ ol_status ol::many_run(ol_ctx *ctx, const ol_doc *d, const ol_patset *set, uint6
         if (e == cudaSuccess) e = cudaMemsetAsync(m.light_count, 0, (size_t)U * 4, st);
         if (e == cudaSuccess) e = cudaMemsetAsync(m.light_n, 0, 16, st);
         if (e == cudaSuccess) e = cudaMemsetAsync(m.stats, 0, 16, st);
+        if (e == cudaSuccess && H) e = cudaMemsetAsync(m.heavy_counts, 0, (size_t)H * hld * 4, st);
+        ma.heavy_counts = m.heavy_counts;
+        ma.heavy_ld = hld;
         ma.stats = m.stats;
         ma.force_timeout = 0;
         ma.tile_stride = 1;
@@ -508,8 +511,7 @@ ol_status ol::many_run(ol_ctx *ctx, const ol_doc *d, const ol_patset *set, uint6
     // 3. Heavy ranks, light order, per-id slots.
     GpuPass order_pass(ctx, "dictionary: rank and sort");
     if (H) {
-        e = launch_dict_heavy_count((const uint32_t *)ctx->dict_bitmap.ptr, n_words, H, m.heavy_counts, hld, st);
-        if (e == cudaSuccess) e = launch_scan_columns(m.heavy_counts, m.heavy_bases, m.heavy_totals, hblocks, H, hld, st);
+        e = launch_scan_columns(m.heavy_counts, m.heavy_bases, m.heavy_totals, n_tiles, H, hld, st);
         if (e != cudaSuccess) return ctx_cuda(ctx, e, "search_many heavy");
     }
     unsigned long long *keys = (unsigned long long *)ctx->dict_keys.ptr;
@@ -535,13 +537,14 @@ ol_status ol::many_run(ol_ctx *ctx, const ol_doc *d, const ol_patset *set, uint6
     ea.n_ids = n;
     ea.n_u = U;
     ea.n_heavy = H;
-    ea.n_words = n_words;
+    ea.n_tiles = n_tiles;
     ea.u_of_id = set->u_of_id;
     ea.dup_start = set->dup_start;
     ea.dup_ids = set->dup_ids;
     ea.heavy_of_u = m.heavy_of_u;
     ea.heavy_u = m.heavy_u;
     ea.heavy_totals = m.heavy_totals;
+    ea.heavy_counts = m.heavy_counts;
     ea.heavy_bases = m.heavy_bases;
     ea.ld = hld;
     ea.bitmap = H ? (const uint32_t *)ctx->dict_bitmap.ptr : nullptr;
