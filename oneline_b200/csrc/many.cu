@@ -26,12 +26,14 @@
 // whose slice holds its start.
 //   * heavy patterns (chosen per search from a sample of the text) set bits in
 //     a bitmap: the slice's words are gathered in shared memory and stored once;
-//   * light patterns append (u << 32 | offset) keys through a per-warp buffer,
-//     and count themselves.
-// Then: popcounts of the bitmaps and a column scan give every heavy hit its
-// rank; a stable radix sort orders the light keys; a single-block pass gives
-// every pattern id its first output slot; the emit kernels write each hit
-// once per id that holds the same bytes (duplicates are reported once per id).
+//   * light patterns append (u, offset) keys through a per-warp buffer, and
+//     count themselves.
+// Before it, the same kernel counts hits on a sample of the text, and
+// dict_plan_kernel picks the heavy patterns from the counts, on the device.
+// After it, a column scan of the heavy hits per tile gives every heavy hit its
+// rank; a radix sort orders the light keys; a single-block pass gives every
+// pattern id its first output slot; the emit kernels write each hit once per id
+// that holds the same bytes (duplicates are reported once per id).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -168,7 +170,7 @@ __device__ __forceinline__ void dict_emit(const DictMatchArgs &a, DictWarp<SLICE
         return;
     }
     atomicAdd(a.counts + u, 1u);
-    const unsigned long long key = ((unsigned long long)u << 32) | (uint32_t)pos;
+    const unsigned long long key = ((unsigned long long)u << a.off_bits) | pos;
     const uint32_t at = atomicAdd(&w.n_light, 1u);
     if (at < DM_LIGHT) {
         w.light[at] = key;
@@ -377,7 +379,7 @@ __global__ void __launch_bounds__(DM_THREADS, 2) dict_match_kernel(const __grid_
     // made the whole match kernel 47% slower, 19.8 against 13.5 ms per GiB.)
     if (a.force_timeout) ok = false;
     if (warp == 0) {
-        const uint32_t x = !a.count_only && lane < a.n_heavy ? a.heavy_run[lane] : 0u;
+        const uint32_t x = !a.count_only && lane < a.plan->n_heavy ? a.heavy_run[lane] : 0u;
         const uint32_t m = __ballot_sync(0xFFFFFFFFu, x != 0);
         if (x) sm.heavy_run[__popc(m & lt)] = (x << 8) | lane;
         if (lane == 0) sm.n_heavy_run = __popc(m);
@@ -392,7 +394,8 @@ __global__ void __launch_bounds__(DM_THREADS, 2) dict_match_kernel(const __grid_
     const uint32_t n_words = a.n_tiles * kDictWordsPerTile;
     const uint32_t per_tile = DM_SLICES_PER_TILE / a.slices;  // items of a tile, of a.slices slices each
     const uint32_t n_items = ((a.n_tiles + a.tile_stride - 1) / a.tile_stride) * per_tile;
-    const uint32_t H = a.count_only ? 0u : a.n_heavy, n_runs = a.set.n_runs, run_bytes = a.set.run_bytes;
+    const uint32_t H = a.count_only ? 0u : a.plan->n_heavy, n_runs = a.set.n_runs, run_bytes = a.set.run_bytes;
+    const uint32_t n_run_light = a.count_only ? a.n_run_light : a.plan->n_run_light;
     uint32_t cands = 0, levels = 0;  // per lane, for the search statistics
     Warp &w = sm.w[warp];
     uint8_t *text = w.text;
@@ -549,7 +552,7 @@ __global__ void __launch_bounds__(DM_THREADS, 2) dict_match_kernel(const __grid_
                 if ((x >> 16) == j) w.bits[x & 0xFFu][i % Warp::kWords] = dict_run_word(w, (x >> 8) & 0xFFu, i % Warp::kWords);
             }
             // the light ones (all of them in count mode)
-            for (uint32_t n = 0; n < a.n_run_light; n++) {
+            for (uint32_t n = 0; n < n_run_light; n++) {
                 const uint32_t x = __ldg(a.run_light + n);  // (j << 24) | (k << 16) | u
                 if ((x >> 24) != j) continue;
                 const uint32_t u = x & 0xFFFFu;
@@ -634,6 +637,10 @@ static cudaError_t launch_match(const DictMatchArgs &args, int sm_count, uint32_
 cudaError_t launch_dict_match(const DictMatchArgs &a, int sm_count, cudaStream_t st, uint32_t slice,
                               uint32_t blocks_per_sm) {
     if (a.n_tiles == 0) return cudaSuccess;
+    // half the serial work per warp where the text leaves most of the chip idle
+    if (slice == 512 && (uint64_t)((a.n_tiles + a.tile_stride - 1) / a.tile_stride) * (kDictTile / 256) <=
+                            (uint64_t)sm_count * DM_SMALL_WARPS_PER_SM)
+        slice = 256;
     switch (slice) {
         case 256: return launch_match<256>(a, sm_count, blocks_per_sm, st);
         case 1024: return launch_match<1024>(a, sm_count, blocks_per_sm, st);
@@ -641,18 +648,78 @@ cudaError_t launch_dict_match(const DictMatchArgs &a, int sm_count, cudaStream_t
     }
 }
 
-// The lists' entries of one search: each with its pattern's heavy index.
-__global__ void dict_outs_kernel(const uint32_t *__restrict__ outs, const uint8_t *__restrict__ heavy_of_u, uint32_t n,
-                                 uint32_t *__restrict__ to) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) to[i] = (((heavy_of_u[outs[i]] + 1u) & 0xFFu) << 16) | outs[i];
+// ------------------------------------------------------------------ plan ----
+
+constexpr uint32_t DP_THREADS = 1024;
+
+// One block picks the heavy patterns from the sample counts: the (at most 32)
+// most frequent of those at or above `least`, lower u first among equals. (Of
+// more than 1024 such patterns any 1024 are looked at: which patterns are heavy
+// changes nothing but the time.) Then the lists that the match pass reads.
+__global__ void __launch_bounds__(DP_THREADS) dict_plan_kernel(DictPlanArgs a) {
+    __shared__ uint32_t cand_u[DP_THREADS], cand_n[DP_THREADS], n_cand, n_light_runs;
+    __shared__ unsigned long long light;
+    const uint32_t tid = threadIdx.x;
+    if (tid == 0) {
+        n_cand = n_light_runs = 0;
+        light = 0;
+    }
+    if (tid < kDictMaxHeavy) a.heavy_run[tid] = a.heavy_u[tid] = 0;
+    __syncthreads();
+    unsigned long long below = 0;
+    for (uint32_t u = tid; u < a.set.n_u; u += DP_THREADS) {
+        const uint32_t n = a.sample_counts[u];
+        a.heavy_of_u[u] = 0xFF;
+        uint32_t at = DP_THREADS;
+        if (n >= a.least) at = atomicAdd(&n_cand, 1u);
+        if (at < DP_THREADS) {
+            cand_u[at] = u;
+            cand_n[at] = n;
+        } else {
+            below += n;
+        }
+    }
+    if (below) atomicAdd(&light, below);
+    __syncthreads();
+    const uint32_t c = min(n_cand, DP_THREADS);
+    if (tid < c) {
+        uint32_t rank = 0;
+        for (uint32_t i = 0; i < c; i++)
+            rank += cand_n[i] > cand_n[tid] || (cand_n[i] == cand_n[tid] && cand_u[i] < cand_u[tid]);
+        if (rank < kDictMaxHeavy) {
+            a.heavy_u[rank] = cand_u[tid];
+            a.heavy_of_u[cand_u[tid]] = (uint8_t)rank;
+        } else {
+            atomicAdd(&light, (unsigned long long)cand_n[tid]);
+        }
+    }
+    __syncthreads();  // heavy_of_u is complete (one block: its own global writes)
+    for (uint32_t i = tid; i < a.n_runs; i += DP_THREADS) {
+        const uint32_t x = a.runs[i];
+        const uint32_t h = a.heavy_of_u[x & 0xFFFFu];
+        if (h != 0xFFu)
+            a.heavy_run[h] = x >> 16;
+        else
+            a.run_light[atomicAdd(&n_light_runs, 1u)] = x;
+    }
+    for (uint32_t i = tid; i < a.set.n_outs; i += DP_THREADS) {
+        const uint32_t u = a.set.outs[i];
+        a.outs[i] = (((a.heavy_of_u[u] + 1u) & 0xFFu) << 16) | u;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        a.plan->n_heavy = min(c, kDictMaxHeavy);
+        a.plan->n_run_light = n_light_runs;
+        a.plan->light_sample = light;
+    }
 }
 
-cudaError_t launch_dict_outs(const uint32_t *outs, const uint8_t *heavy_of_u, uint32_t n, uint32_t *to, cudaStream_t st) {
-    if (n == 0) return cudaSuccess;
-    dict_outs_kernel<<<(n + 255) / 256, 256, 0, st>>>(outs, heavy_of_u, n, to); OL_LAUNCHED();
+cudaError_t launch_dict_plan(const DictPlanArgs &a, cudaStream_t st) {
+    dict_plan_kernel<<<1, DP_THREADS, 0, st>>>(a); OL_LAUNCHED();
     return cudaGetLastError();
 }
+
+// ------------------------------------------------------- block-wide sums ----
 
 constexpr uint32_t DH_THREADS = 256;
 
@@ -680,94 +747,136 @@ __device__ __forceinline__ uint32_t block_exclusive_256(uint32_t x, uint32_t *wa
 }
 
 // ---------------------------------------------------- light-key radix sort --
+//
+// LSD radix sort of the keys, 8 bits a pass, over as many bits as a key has
+// (offset bits and pattern bits next to each other). Keys differ, so the order
+// is one. A block ranks 4096 keys in shared memory, a warp 512 of them in order
+// (lanes with the same digit by __match_any_sync), and writes them digit by
+// digit: runs of 16 keys on average, where single keys were scattered before
+// (4.3 M keys: a pass takes
+// 12 + 4 + 50 us, 21 + 9 + 60 before).
 
 constexpr uint32_t DS_THREADS = 256;
 constexpr uint32_t DS_WARPS = DS_THREADS / 32;
-constexpr uint32_t DS_PER_LANE = kDictSortChunk / 32;
+constexpr uint32_t DS_STEPS = kDictSortBlock / DS_THREADS;  // keys per lane
 
-uint32_t dict_sort_chunks(uint32_t n) { return (n + kDictSortChunk - 1) / kDictSortChunk; }
+uint32_t dict_sort_blocks(uint32_t n) { return (n + kDictSortBlock - 1) / kDictSortBlock; }
 
-// Per-warp digit histograms: chunk c (one warp) holds keys [512c, 512c + 512).
 __global__ void __launch_bounds__(DS_THREADS) dict_sort_hist_kernel(const unsigned long long *__restrict__ keys,
                                                                      uint32_t n, uint32_t shift, uint32_t *hist,
-                                                                     uint32_t ld, uint32_t chunks) {
-    __shared__ uint32_t sh[DS_WARPS][256];
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t c = blockIdx.x * DS_WARPS + warp;
-    for (uint32_t d = lane; d < 256; d += 32) sh[warp][d] = 0;
+                                                                     uint32_t ld) {
+    __shared__ uint32_t sh[256];
+    sh[threadIdx.x] = 0;
+    __syncthreads();
+#pragma unroll
+    for (uint32_t i = 0; i < DS_STEPS; i++) {
+        const uint32_t idx = blockIdx.x * kDictSortBlock + i * DS_THREADS + threadIdx.x;
+        if (idx < n) atomicAdd(&sh[(uint32_t)(keys[idx] >> shift) & 255u], 1u);
+    }
+    __syncthreads();
+    hist[(size_t)threadIdx.x * ld + blockIdx.x] = sh[threadIdx.x];
+}
+
+// Ranks of `n` keys (at most 512 per warp) by digit: on return rank[i] is key
+// i's place in the block's order, and start[d] the first place of digit d.
+// cursor: 256 words per warp. The whole block calls (NT threads).
+template <uint32_t NT, uint32_t STEPS>
+__device__ __forceinline__ void sort_ranks(const unsigned long long (&key)[STEPS], uint32_t first, uint32_t n, uint32_t shift,
+                                           uint16_t (*cursor)[256], uint32_t *start, uint32_t *warp_sum,
+                                           uint32_t (&rank)[STEPS]) {
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, lt = (1u << lane) - 1u;
+    for (uint32_t d = lane; d < 256; d += 32) cursor[warp][d] = 0;
     __syncwarp();
-    if (c < chunks) {
-#pragma unroll 4
-        for (uint32_t i = 0; i < DS_PER_LANE; i++) {
-            uint32_t idx = c * kDictSortChunk + i * 32 + lane;
-            if (idx < n) atomicAdd(&sh[warp][(uint32_t)(keys[idx] >> shift) & 255u], 1u);
+#pragma unroll
+    for (uint32_t i = 0; i < STEPS; i++) {
+        const bool valid = first + i * 32 + lane < n;
+        const uint32_t vm = __ballot_sync(0xFFFFFFFFu, valid);
+        uint32_t d = 0, peers = 0;
+        if (valid) {
+            d = (uint32_t)(key[i] >> shift) & 255u;
+            peers = __match_any_sync(vm, d);
+            rank[i] = cursor[warp][d] + __popc(peers & lt);  // in the warp, among the digit's keys
         }
         __syncwarp();
-        for (uint32_t d = lane; d < 256; d += 32) hist[(size_t)d * ld + c] = sh[warp][d];
+        if (valid && (peers & lt) == 0) cursor[warp][d] += (uint16_t)__popc(peers);
+        __syncwarp();
+    }
+    __syncthreads();
+    // digit d (thread d): the warps' counts become their first places among the digit's keys
+    uint32_t total = 0;
+    if (tid < 256) {
+#pragma unroll 8
+        for (uint32_t w = 0; w < NT / 32; w++) {
+            const uint32_t c = cursor[w][tid];
+            cursor[w][tid] = (uint16_t)total;
+            total += c;
+        }
+        uint32_t inc = total;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, inc, o);
+            if ((int)lane >= o) inc += t;
+        }
+        if (lane == 31) warp_sum[warp] = inc;
+        start[tid] = inc - total;
+    }
+    __syncthreads();
+    if (tid < 256)
+        for (uint32_t w = 0; w < warp; w++) start[tid] += warp_sum[w];
+    __syncthreads();
+#pragma unroll
+    for (uint32_t i = 0; i < STEPS; i++) {
+        const uint32_t d = (uint32_t)(key[i] >> shift) & 255u;
+        if (first + i * 32 + lane < n) rank[i] += start[d] + cursor[warp][d];
     }
 }
 
-// Stable scatter: each warp walks its chunk in order, 32 keys at a time; lanes
-// with the same digit take consecutive slots in lane order.
 __global__ void __launch_bounds__(DS_THREADS) dict_sort_scatter_kernel(const unsigned long long *__restrict__ in,
                                                                         unsigned long long *__restrict__ out,
                                                                         uint32_t n, uint32_t shift,
                                                                         const uint32_t *__restrict__ base,
                                                                         const uint32_t *__restrict__ totals,
-                                                                        uint32_t ld, uint32_t chunks) {
-    __shared__ uint32_t start[256];
-    __shared__ uint32_t warp_sum[DS_WARPS];
-    __shared__ uint32_t cursor[DS_WARPS][256];
+                                                                        uint32_t ld) {
+    __shared__ unsigned long long sorted[kDictSortBlock];
+    __shared__ uint16_t cursor[DS_WARPS][256];
+    __shared__ uint32_t start[256], to[256], warp_sum[DS_WARPS];
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    // digit starts: exclusive scan of the 256 digit totals
-    start[tid] = block_exclusive_256(totals[tid], warp_sum, nullptr);
+    const uint32_t b0 = blockIdx.x * kDictSortBlock, m = min(n - b0, kDictSortBlock), first = warp * (DS_STEPS * 32);
+    unsigned long long key[DS_STEPS];
+#pragma unroll
+    for (uint32_t i = 0; i < DS_STEPS; i++) {
+        const uint32_t j = first + i * 32 + lane;
+        key[i] = j < m ? in[b0 + j] : 0ull;
+    }
+    // the digits' first places in the output: totals before the digit, and the blocks before this one
+    to[tid] = block_exclusive_256(totals[tid], warp_sum, nullptr) + base[(size_t)tid * ld + blockIdx.x];
+    uint32_t rank[DS_STEPS];
+    sort_ranks<DS_THREADS, DS_STEPS>(key, first, m, shift, cursor, start, warp_sum, rank);
+#pragma unroll
+    for (uint32_t i = 0; i < DS_STEPS; i++)
+        if (first + i * 32 + lane < m) sorted[rank[i]] = key[i];
     __syncthreads();
-    const uint32_t c = blockIdx.x * DS_WARPS + warp;
-    if (c >= chunks) return;
-    for (uint32_t d = lane; d < 256; d += 32) cursor[warp][d] = start[d] + base[(size_t)d * ld + c];
-    __syncwarp();
-    const uint32_t lt = (1u << lane) - 1u;
-    unsigned long long nkey = c * kDictSortChunk + lane < n ? in[c * kDictSortChunk + lane] : 0ull;  // a step ahead
-    for (uint32_t i = 0; i < DS_PER_LANE; i++) {
-        const uint32_t idx = c * kDictSortChunk + i * 32 + lane;
-        const bool valid = idx < n;
-        const uint32_t vm = __ballot_sync(0xFFFFFFFFu, valid);
-        if (!vm) break;
-        const unsigned long long key = nkey;
-        if (i + 1 < DS_PER_LANE) nkey = idx + 32 < n ? in[idx + 32] : 0ull;
-        uint32_t d = 0, peers = 0;
-        if (valid) {
-            d = (uint32_t)(key >> shift) & 255u;
-            peers = __match_any_sync(vm, d);
-            out[cursor[warp][d] + __popc(peers & lt)] = key;
-        }
-        __syncwarp();
-        if (valid && (peers & lt) == 0) cursor[warp][d] += __popc(peers);
-        __syncwarp();
+    for (uint32_t j = tid; j < m; j += DS_THREADS) {
+        const unsigned long long k = sorted[j];
+        const uint32_t d = (uint32_t)(k >> shift) & 255u;
+        out[to[d] + j - start[d]] = k;
     }
 }
 
 cudaError_t launch_dict_sort(unsigned long long *keys, unsigned long long *tmp, uint32_t n, uint32_t key_bits,
-                             uint32_t *hist, uint32_t *totals, cudaStream_t st) {
-    if (n < 2) return cudaSuccess;
-    const uint32_t chunks = dict_sort_chunks(n);
-    const uint32_t ld = scan_ld(chunks);
+                             uint32_t *hist, uint32_t *totals, unsigned long long **sorted, cudaStream_t st) {
+    const uint32_t blocks = dict_sort_blocks(n), ld = scan_ld(blocks);
     uint32_t *counts = hist, *bases = hist + (size_t)256 * ld;
-    const uint32_t blocks = (chunks + DS_WARPS - 1) / DS_WARPS;
     unsigned long long *src = keys, *dst = tmp;
-    uint32_t passes = (key_bits + 7) / 8;
-    passes += passes & 1;  // an even number of passes leaves the result in keys
-    for (uint32_t p = 0; p < passes; p++) {
-        const uint32_t shift = 8 * p;
-        dict_sort_hist_kernel<<<blocks, DS_THREADS, 0, st>>>(src, n, shift, counts, ld, chunks); OL_LAUNCHED();
-        cudaError_t e = launch_scan_columns(counts, bases, totals, chunks, 256, ld, st);
+    for (uint32_t shift = 0; shift < key_bits && n > 1; shift += 8) {
+        dict_sort_hist_kernel<<<blocks, DS_THREADS, 0, st>>>(src, n, shift, counts, ld); OL_LAUNCHED();
+        cudaError_t e = launch_scan_columns(counts, bases, totals, blocks, 256, ld, st);
         if (e != cudaSuccess) return e;
-        dict_sort_scatter_kernel<<<blocks, DS_THREADS, 0, st>>>(src, dst, n, shift, bases, totals, ld, chunks); OL_LAUNCHED();
+        dict_sort_scatter_kernel<<<blocks, DS_THREADS, 0, st>>>(src, dst, n, shift, bases, totals, ld); OL_LAUNCHED();
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        unsigned long long *t = src;
-        src = dst;
-        dst = t;
+        std::swap(src, dst);
     }
+    *sorted = src;
     return cudaSuccess;
 }
 
@@ -777,7 +886,7 @@ constexpr uint32_t DI_THREADS = 1024;
 
 // One block: per id its count and first output slot (u64 exclusive scan in id
 // order), the total, and per unique pattern the start of its light keys.
-__global__ void __launch_bounds__(DI_THREADS) dict_ids_kernel(DictEmitArgs a) {
+__device__ __forceinline__ void dict_ids(const DictEmitArgs &a) {
     __shared__ unsigned long long wsum64[DI_THREADS / 32];
     __shared__ uint32_t wsum32[DI_THREADS / 32];
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -836,6 +945,54 @@ __global__ void __launch_bounds__(DI_THREADS) dict_ids_kernel(DictEmitArgs a) {
             run += a.heavy_of_u[u] == 0xFFu ? a.light_count[u] : 0u;
         }
     }
+}
+
+__global__ void __launch_bounds__(DI_THREADS) dict_ids_kernel(DictEmitArgs a) { dict_ids(a); }
+
+// A search with few light keys: one block sorts them (all passes in shared
+// memory) and places the ids; with more keys than it takes it leaves them and
+// the caller sorts. A 256 KiB text and 40 patterns took 19 launches for this.
+__global__ void __launch_bounds__(DI_THREADS) dict_sort_ids_kernel(DictEmitArgs a, unsigned long long *keys, uint32_t key_bits) {
+    extern __shared__ __align__(16) uint8_t dyn_smem[];
+    constexpr uint32_t STEPS = kDictSortBlock / DI_THREADS;
+    unsigned long long *sorted = reinterpret_cast<unsigned long long *>(dyn_smem);
+    uint16_t(*cursor)[256] = reinterpret_cast<uint16_t(*)[256]>(sorted + kDictSortBlock);
+    __shared__ uint32_t start[256], warp_sum[8];
+    const uint32_t lane = threadIdx.x & 31, first = (threadIdx.x >> 5) * (STEPS * 32);
+    const uint32_t n = *a.light_n_dev;
+    if (n > 1 && n <= kDictSortBlock) {
+        unsigned long long key[STEPS];
+#pragma unroll
+        for (uint32_t i = 0; i < STEPS; i++) {
+            const uint32_t j = first + i * 32 + lane;
+            key[i] = j < n ? keys[j] : 0ull;
+        }
+        for (uint32_t shift = 0; shift < key_bits; shift += 8) {
+            uint32_t rank[STEPS];
+            sort_ranks<DI_THREADS, STEPS>(key, first, n, shift, cursor, start, warp_sum, rank);
+#pragma unroll
+            for (uint32_t i = 0; i < STEPS; i++)
+                if (first + i * 32 + lane < n) sorted[rank[i]] = key[i];
+            __syncthreads();
+#pragma unroll
+            for (uint32_t i = 0; i < STEPS; i++) {
+                const uint32_t j = first + i * 32 + lane;
+                key[i] = j < n ? sorted[j] : 0ull;
+            }
+        }
+#pragma unroll
+        for (uint32_t i = 0; i < STEPS; i++)
+            if (first + i * 32 + lane < n) keys[first + i * 32 + lane] = key[i];
+    }
+    dict_ids(a);
+}
+
+cudaError_t launch_dict_sort_ids(const DictEmitArgs &a, unsigned long long *keys, uint32_t key_bits, cudaStream_t st) {
+    const size_t smem = kDictSortBlock * 8 + (DI_THREADS / 32) * 256 * 2;
+    cudaError_t e = cudaFuncSetAttribute(dict_sort_ids_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    dict_sort_ids_kernel<<<1, DI_THREADS, smem, st>>>(a, keys, key_bits); OL_LAUNCHED();
+    return cudaGetLastError();
 }
 
 cudaError_t launch_dict_ids(const DictEmitArgs &a, cudaStream_t st) {
@@ -910,6 +1067,7 @@ __global__ void __launch_bounds__(DH_THREADS, 6) dict_emit_heavy_kernel(DictEmit
     __shared__ uint16_t hit_buf[DH_THREADS / 32][DH_BUF];  // per warp: hit offsets in the tile, in order
     const uint32_t h = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t tile = blockIdx.x * (DH_THREADS / 32) + warp;
+    if (h >= a.plan->n_heavy) return;
     const uint32_t u = a.heavy_u[h];
     const uint32_t d0 = a.dup_start[u], n_dup = a.dup_start[u + 1] - d0;
     const bool cached = n_dup <= DH_MAX_DUPS;
@@ -966,16 +1124,18 @@ __global__ void __launch_bounds__(DH_THREADS, 6) dict_emit_heavy_kernel(DictEmit
 }
 
 __global__ void dict_emit_light_kernel(DictEmitArgs a) {
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= a.light_n) return;
-    const unsigned long long key = a.light_keys[k];
-    const uint32_t u = (uint32_t)(key >> 32), off = (uint32_t)key;
-    const uint32_t rank = k - a.light_base[u];
-    const uint32_t d0 = a.dup_start[u], d1 = a.dup_start[u + 1];
-    for (uint32_t d = d0; d < d1; d++) {
-        const uint32_t id = a.dup_ids[d];
-        const unsigned long long slot = a.id_base[id] + rank;
-        if (slot < a.max_hits) put_hit(a, slot, id, off);
+    const uint32_t n = *a.light_n_dev;
+    if (n > a.light_max) return;  // unsorted (dict_sort_ids_kernel): the caller emits once more
+    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+        const unsigned long long key = a.light_keys[k];
+        const uint32_t u = (uint32_t)(key >> a.off_bits), off = (uint32_t)(key & ((1ull << a.off_bits) - 1));
+        const uint32_t rank = k - a.light_base[u];
+        const uint32_t d0 = a.dup_start[u], d1 = a.dup_start[u + 1];
+        for (uint32_t d = d0; d < d1; d++) {
+            const uint32_t id = a.dup_ids[d];
+            const unsigned long long slot = a.id_base[id] + rank;
+            if (slot < a.max_hits) put_hit(a, slot, id, off);
+        }
     }
 }
 
@@ -991,8 +1151,8 @@ cudaError_t launch_dict_emit(const DictEmitArgs &a, cudaStream_t st) {
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
-    if (a.light_n) {
-        dict_emit_light_kernel<<<(a.light_n + 255) / 256, 256, 0, st>>>(a); OL_LAUNCHED();
+    if (a.light_max) {
+        dict_emit_light_kernel<<<(a.light_max + 255) / 256, 256, 0, st>>>(a); OL_LAUNCHED();
         return cudaGetLastError();
     }
     return cudaSuccess;

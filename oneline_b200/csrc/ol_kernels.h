@@ -177,7 +177,7 @@ constexpr uint32_t kDictMaxLen = 64;
 constexpr uint32_t kDictMaxHeavy = 32;        // patterns whose hits go to bitmaps in one search
 constexpr uint32_t kDictFilterBits = 17;      // 2^17-bit filter (16 KiB of shared memory)
 constexpr uint32_t kDictWordsPerTile = kDictTile / 32;
-constexpr uint32_t kDictSortChunk = 512;      // keys per warp in the light-hit radix sort
+constexpr uint32_t kDictSortBlock = 4096;     // keys per block in the light-hit radix sort
 constexpr uint32_t kDictMaxRuns = 4;          // run bytes of a set
 
 // Filter and table hashes of a pattern's first four bytes (little-endian u32);
@@ -228,6 +228,24 @@ constexpr uint32_t kDictEdgeMask = 0x1FFu;
 constexpr uint32_t kDictPathMin = 3;          // shorter runs are walked node by node
 constexpr uint32_t kDictPathWords = 1u << 19;  // addressable words of paths (nodes past them go without)
 
+// What a search decides from its sample counts, on the device.
+struct DictPlan {
+    uint32_t n_heavy;      // patterns whose hits go to bitmaps
+    uint32_t n_run_light;  // run patterns that are not among them
+    unsigned long long light_sample;  // hits of the others in the sample
+};
+struct DictPlanArgs {
+    DictSet set;
+    const uint32_t *sample_counts;  // [n_u]
+    uint32_t least;                 // sample count of a heavy pattern
+    const uint32_t *runs;           // the set's run patterns, as DictMatchArgs::run_light has them
+    uint32_t n_runs;
+    uint8_t *heavy_of_u;            // the rest: written
+    uint32_t *heavy_u, *heavy_run, *run_light, *outs;
+    DictPlan *plan;
+};
+cudaError_t launch_dict_plan(const DictPlanArgs &a, cudaStream_t st);
+
 struct DictMatchArgs {
     DictSet set;
     const uint8_t *text;     // padded like every resident text
@@ -237,12 +255,13 @@ struct DictMatchArgs {
     uint32_t count_only;     // 1: counts[u] += every hit; 0: heavy bitmaps + light keys
     uint32_t *counts;        // per unique pattern (count mode: all hits; else light hits)
     const uint8_t *heavy_of_u;  // heavy index or 0xFF
-    uint32_t n_heavy;
+    const DictPlan *plan;    // (not in count mode)
     uint32_t *bitmap;        // [n_heavy][n_tiles * kDictWordsPerTile]
     uint32_t *heavy_counts;  // [n_heavy][heavy_ld]: += hits per tile
     uint32_t heavy_ld;
     uint32_t slices;         // consecutive slices per item (set by the launch)
-    unsigned long long *light_keys;  // (u << 32) | offset, unordered
+    unsigned long long *light_keys;  // (u << off_bits) | offset, unordered
+    uint32_t off_bits;
     uint32_t light_cap;
     uint32_t *light_n;
     uint32_t *error;
@@ -252,28 +271,27 @@ struct DictMatchArgs {
     const unsigned long long *seg_end;
     uint32_t n_seg;
     unsigned long long *stats;  // optional: += candidates walked, trie nodes visited
-    const uint32_t *outs;       // set.outs, with (heavy index + 1) << 16 of the heavy patterns (launch_dict_outs)
+    const uint32_t *outs;       // set.outs, with (heavy index + 1) << 16 of the heavy patterns (launch_dict_plan)
     const uint32_t *heavy_run;  // [kDictMaxHeavy]: (j << 8) | k of a heavy run pattern run_byte(j)^k, else 0
     const uint32_t *run_light;  // (j << 24) | (k << 16) | u of the run patterns that are not heavy (count mode: all)
-    uint32_t n_run_light;
+    uint32_t n_run_light;       // (count mode; else the plan's)
     // Test hook (ol_ctx_inject): each block takes its wait-timeout branch
     // after its filter copy has landed, as if the bounded wait had run out.
     uint32_t force_timeout;
 };
 
-// to[i] = outs[i], with the heavy index of pattern outs[i].
-cudaError_t launch_dict_outs(const uint32_t *outs, const uint8_t *heavy_of_u, uint32_t n, uint32_t *to, cudaStream_t st);
 cudaError_t launch_dict_match(const DictMatchArgs &a, int sm_count, cudaStream_t st, uint32_t slice = 512,
                               uint32_t blocks_per_sm = 0);
-// Stable LSD radix sort of n 64-bit keys on bits [0, key_bits), 8 per pass;
-// the result ends in keys (tmp is the other buffer); hist needs
-// 2 * 256 * scan_ld(chunks) words and digit totals 256 words.
+// Radix sort of n different 64-bit keys on bits [0, key_bits), 8 per pass;
+// *sorted is where the result is, keys or tmp; hist needs
+// 2 * 256 * scan_ld(dict_sort_blocks(n)) words, totals 256 words.
 cudaError_t launch_dict_sort(unsigned long long *keys, unsigned long long *tmp, uint32_t n, uint32_t key_bits,
-                             uint32_t *hist, uint32_t *totals, cudaStream_t st);
-uint32_t dict_sort_chunks(uint32_t n);
+                             uint32_t *hist, uint32_t *totals, unsigned long long **sorted, cudaStream_t st);
+uint32_t dict_sort_blocks(uint32_t n);
 
 struct DictEmitArgs {
-    uint32_t n_ids, n_u, n_heavy, n_tiles;
+    uint32_t n_ids, n_u, n_heavy, n_tiles;  // n_heavy: at least the plan's
+    const DictPlan *plan;
     const uint32_t *u_of_id;
     const uint32_t *dup_start;   // [n_u + 1]
     const uint32_t *dup_ids;     // ids grouped by unique pattern, ascending
@@ -286,7 +304,9 @@ struct DictEmitArgs {
     const uint32_t *light_count; // [n_u]
     uint32_t *light_base;        // [n_u] (written by the id pass)
     const unsigned long long *light_keys;  // sorted
-    uint32_t light_n;
+    const uint32_t *light_n_dev;
+    uint32_t light_max;          // more light keys than this are not emitted
+    uint32_t off_bits;
     uint32_t *id_counts;         // [n_ids]
     unsigned long long *id_base; // [n_ids]
     unsigned long long *total;
@@ -298,6 +318,9 @@ struct DictEmitArgs {
     unsigned long long *hit_off;
 };
 cudaError_t launch_dict_ids(const DictEmitArgs &a, cudaStream_t st);
+// The same after a sort of the light keys (in place) in one launch, when there
+// are at most kDictSortBlock of them; more are left unsorted.
+cudaError_t launch_dict_sort_ids(const DictEmitArgs &a, unsigned long long *keys, uint32_t key_bits, cudaStream_t st);
 
 // Digests (digest.cu): *out += sum of per-element hashes of a[0..n).
 cudaError_t launch_digest_u32(const uint32_t *a, uint64_t n, uint32_t seed, unsigned long long *out, cudaStream_t st);

@@ -60,6 +60,25 @@ void DevBuf::release(cudaStream_t st) {
     bytes = 0;
 }
 
+cudaError_t HostBuf::reserve(size_t need) {
+    if (need <= bytes) return cudaSuccess;
+    release();
+    need = std::max<size_t>(need, 4096);
+    cudaError_t e = cudaMallocHost((void **)&ptr, need);
+    if (e != cudaSuccess) {
+        ptr = nullptr;
+        return e;
+    }
+    bytes = need;
+    return cudaSuccess;
+}
+
+void HostBuf::release() {
+    if (ptr) cudaFreeHost(ptr);
+    ptr = nullptr;
+    bytes = 0;
+}
+
 uint32_t parse_tiles(uint64_t len) { return (uint32_t)((len + kParseTile - 1) / kParseTile); }
 uint64_t text_alloc_bytes(uint64_t len) { return (uint64_t)parse_tiles(len) * kParseTile + kTextPad; }
 uint32_t round_lines(uint64_t n) { return (uint32_t)std::min<uint64_t>(((n + kTreeTile - 1) / kTreeTile) * kTreeTile, 0xFFFFF000ull); }
@@ -151,6 +170,8 @@ extern "C" void ol_ctx_destroy(ol_ctx *ctx) {
     ctx->dict_bitmap.release(ctx->stream);
     ctx->dict_keys.release(ctx->stream);
     ctx->dict_hits.release(ctx->stream);
+    ctx->dict_sort.release(ctx->stream);
+    ctx->host_words.release();
     if (ctx->counters) cudaFreeAsync(ctx->counters, ctx->stream);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     if (ctx->host_counters) cudaFreeHost(ctx->host_counters);

@@ -25,6 +25,15 @@ struct DevBuf {
     void release(cudaStream_t st);
 };
 
+// Page-locked host memory, grown on demand (no copy of it may be in flight
+// when it grows).
+struct HostBuf {
+    uint8_t *ptr = nullptr;
+    size_t bytes = 0;
+    cudaError_t reserve(size_t need);
+    void release();
+};
+
 struct Prof;
 
 // Small per-context words in device memory, and their page-locked copy on the
@@ -61,6 +70,8 @@ struct ol_ctx {
     ol::DevBuf dict_small;   // dictionary search: per-pattern counts, ranks, slots
     ol::DevBuf dict_bitmap;  // heavy-pattern bitmaps
     ol::DevBuf dict_keys;    // light-hit keys and the sort's second buffer
+    ol::DevBuf dict_sort;    // the light-hit sort's histograms
+    ol::HostBuf host_words;  // short results read back (page-locked)
     ol::DevBuf dict_hits;    // hits of the blocking search before the download
     ol::CtxCounters *counters = nullptr;
     ol::CtxCounters *host_counters = nullptr;  // pinned

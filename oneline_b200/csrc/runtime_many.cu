@@ -6,6 +6,8 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
+#include <cstddef>
 #include <cstring>
 #include <mutex>
 #include <string>
@@ -44,13 +46,11 @@ uint32_t bits_for(uint32_t v) {  // bits needed to hold values 0..v
     return b;
 }
 
-// Scratch of one dictionary search, carved from ctx->dict_small.
-struct ManyScratch {
-    uint32_t *sample_counts, *light_count, *light_base, *heavy_u, *heavy_totals, *heavy_counts, *heavy_bases;
-    uint32_t *light_n, *error, *id_counts, *sort_hist, *sort_totals;
-    uint8_t *heavy_of_u;
-    unsigned long long *id_base, *total, *stats;
-    uint32_t *outs, *heavy_run, *run_light;
+// Words a search reads back: one copy, together with the id counts.
+struct ManyMeta {
+    DictPlan plan;
+    uint32_t light_n, error;
+    unsigned long long total, walked, nodes;
 };
 
 }  // namespace
@@ -335,6 +335,15 @@ extern "C" uint32_t ol_patset_unique(const ol_patset *s) { return s ? s->n_u : 0
 // The whole search; hits go to d_hits (capacity max_hits) when given, else to
 // host_hits through ctx->dict_hits. counts (n_ids) and *total are host outputs.
 // seg_start/seg_end (device, n_seg): batches, whose hits stay inside a document.
+//
+// The host waits as seldom as the sizes allow. Texts of up to kPlanTiles tiles
+// go from the sample to the match pass on the device's own plan, with scratch
+// for as many heavy patterns as there can be; larger ones read the plan first.
+// With up to kFewTiles tiles the light keys are taken to be few enough for one
+// block to sort; if they were not, the host learns it with the counts, sorts
+// them and places the ids (and writes device hits) once more.
+constexpr uint32_t kPlanTiles = 4096, kFewTiles = 256, kSampleTiles = 160;
+
 ol_status ol::many_run(ol_ctx *ctx, const ol_doc *d, const ol_patset *set, uint64_t max_hits, uint32_t heavy_min_hits,
                        uint32_t *counts, uint64_t *total, const HitDest &dest,
                        const unsigned long long *seg_start, const unsigned long long *seg_end, uint32_t n_seg) {
@@ -345,55 +354,47 @@ ol_status ol::many_run(ol_ctx *ctx, const ol_doc *d, const ol_patset *set, uint6
     memset(counts, 0, (size_t)n * 4);
     if (N < kDictMinLen) return OL_OK;
     const uint32_t n_tiles = (uint32_t)((N + kDictTile - 1) / kDictTile);
-    const uint32_t n_words = n_tiles * kDictWordsPerTile;
-    const uint32_t hld = scan_ld(n_tiles);
+    const uint32_t n_words = n_tiles * kDictWordsPerTile, hld = scan_ld(n_tiles);
+    const uint32_t off_bits = std::max<uint32_t>(bits_for((uint32_t)(N - 1)), 1), key_bits = off_bits + bits_for(U - 1);
 
-    // Small scratch (sort histograms sized for the worst light count: grown below if needed).
-    auto carve = [](size_t &at, size_t bytes) {
-        size_t o = at;
-        at = align256(at + bytes);
+    // Scratch, carved from ctx->dict_small. Id counts and meta are read back
+    // together; meta's counters up to the sample counts start from zero.
+    size_t at = 0;
+    auto carve = [&](size_t bytes, size_t align = 16) {
+        at = (at + align - 1) & ~(align - 1);
+        const size_t o = at;
+        at += bytes;
         return o;
     };
-    size_t at = 0;
-    size_t o_sample = carve(at, (size_t)U * 4), o_lcount = carve(at, (size_t)U * 4), o_lbase = carve(at, (size_t)U * 4);
-    size_t o_heavy_of = carve(at, U), o_heavy_u = carve(at, kDictMaxHeavy * 4), o_htot = carve(at, kDictMaxHeavy * 4);
-    size_t o_hcounts = carve(at, (size_t)kDictMaxHeavy * hld * 4), o_hbases = carve(at, (size_t)kDictMaxHeavy * hld * 4);
-    size_t o_ln = carve(at, 16), o_idc = carve(at, (size_t)n * 4), o_idb = carve(at, (size_t)n * 8), o_tot = carve(at, 16);
-    size_t o_stot = carve(at, 256 * 4), o_stats = carve(at, 16);
-    size_t o_outs = carve(at, (size_t)set->dev.n_outs * 4);
-    size_t o_hrun = carve(at, kDictMaxHeavy * 4), o_rlight = carve(at, std::max<size_t>(set->runs.size(), 1) * 4);
-    const size_t fixed = at;
-    cudaError_t e = ctx->dict_small.reserve(fixed, st);
+    const size_t o_idc = carve((size_t)n * 4), o_meta = carve(sizeof(ManyMeta));
+    const size_t o_lcount = carve((size_t)U * 4), o_hcounts = carve((size_t)kDictMaxHeavy * hld * 4), rezero_end = at;
+    const size_t o_sample = carve((size_t)U * 4), zero_end = at;
+    const size_t o_lbase = carve((size_t)U * 4), o_heavy_of = carve(U), o_heavy_u = carve(kDictMaxHeavy * 4);
+    const size_t o_htot = carve(kDictMaxHeavy * 4), o_hbases = carve((size_t)kDictMaxHeavy * hld * 4);
+    const size_t o_hrun = carve(kDictMaxHeavy * 4), o_rlight = carve(std::max<size_t>(set->runs.size(), 1) * 4);
+    const size_t o_outs = carve((size_t)set->dev.n_outs * 4), o_idb = carve((size_t)n * 8), o_stot = carve(256 * 4);
+    cudaError_t e = ctx->dict_small.reserve(at, st);
+    const size_t back = o_meta + sizeof(ManyMeta);  // bytes read back
+    if (e == cudaSuccess) e = ctx->host_words.reserve(back);
     if (e != cudaSuccess) return ctx_cuda(ctx, e, "search_many");
-    auto scratch_at = [&](uint8_t *b) {
-        ManyScratch m;
-        m.sample_counts = (uint32_t *)(b + o_sample);
-        m.light_count = (uint32_t *)(b + o_lcount);
-        m.light_base = (uint32_t *)(b + o_lbase);
-        m.heavy_of_u = b + o_heavy_of;
-        m.heavy_u = (uint32_t *)(b + o_heavy_u);
-        m.heavy_totals = (uint32_t *)(b + o_htot);
-        m.heavy_counts = (uint32_t *)(b + o_hcounts);
-        m.heavy_bases = (uint32_t *)(b + o_hbases);
-        m.light_n = (uint32_t *)(b + o_ln);
-        m.error = m.light_n + 1;
-        m.id_counts = (uint32_t *)(b + o_idc);
-        m.id_base = (unsigned long long *)(b + o_idb);
-        m.total = (unsigned long long *)(b + o_tot);
-        m.sort_totals = (uint32_t *)(b + o_stot);
-        m.stats = (unsigned long long *)(b + o_stats);
-        m.outs = (uint32_t *)(b + o_outs);
-        m.heavy_run = (uint32_t *)(b + o_hrun);
-        m.run_light = (uint32_t *)(b + o_rlight);
-        m.sort_hist = (uint32_t *)(b + fixed);
-        return m;
+    uint8_t *b = (uint8_t *)ctx->dict_small.ptr;
+    ManyMeta *meta = (ManyMeta *)(b + o_meta);
+    const ManyMeta *hm = (const ManyMeta *)(ctx->host_words.ptr + o_meta);
+    uint32_t *light_count = (uint32_t *)(b + o_lcount), *heavy_counts = (uint32_t *)(b + o_hcounts);
+    uint32_t *heavy_bases = (uint32_t *)(b + o_hbases), *heavy_totals = (uint32_t *)(b + o_htot);
+    const size_t o_zero = o_meta + offsetof(ManyMeta, light_n);
+    auto read_meta = [&]() -> cudaError_t {  // id counts and meta, as the stream has them now
+        cudaError_t r = cudaMemcpyAsync(ctx->host_words.ptr, b, back, cudaMemcpyDeviceToHost, st);
+        return r == cudaSuccess ? cudaStreamSynchronize(st) : r;
     };
-    ManyScratch m = scratch_at((uint8_t *)ctx->dict_small.ptr);
 
     // 1. Counts on a sample of tiles (every tile when the text is small) pick
     //    the heavy patterns: those expected to have at least `threshold` hits.
-    const uint32_t stride = std::max<uint32_t>(1, n_tiles / 256);
+    const uint32_t sample = std::min(std::max(n_tiles / 8, 4u), kSampleTiles), stride = std::max<uint32_t>(1, n_tiles / sample);
     const uint32_t n_work = (n_tiles + stride - 1) / stride;
+    const double scale = (double)n_tiles / (double)n_work;
+    const double threshold = heavy_min_hits ? (double)heavy_min_hits
+                                            : std::max(4096.0, (double)N / (double)std::max<uint32_t>(ctx->tune.dict_heavy_divisor, 1));
     DictMatchArgs ma{};
     ma.set = set->dev;
     ma.text = d->text;
@@ -401,8 +402,8 @@ ol_status ol::many_run(ol_ctx *ctx, const ol_doc *d, const ol_patset *set, uint6
     ma.n_tiles = n_tiles;
     ma.tile_stride = stride;
     ma.count_only = 1;
-    ma.counts = m.sample_counts;
-    ma.error = m.error;
+    ma.counts = (uint32_t *)(b + o_sample);
+    ma.error = &meta->error;
     ma.outs = set->dev.outs;
     ma.run_light = set->d_runs;
     ma.n_run_light = (uint32_t)set->runs.size();
@@ -412,188 +413,187 @@ ol_status ol::many_run(ol_ctx *ctx, const ol_doc *d, const ol_patset *set, uint6
     // an armed injected timeout is taken by this search's first match pass
     ma.force_timeout = (ctx->inject & OL_INJECT_DICT_WAIT_TIMEOUT) ? 1u : 0u;
     ctx->inject &= ~OL_INJECT_DICT_WAIT_TIMEOUT;
-    e = cudaMemsetAsync(m.sample_counts, 0, (size_t)U * 4, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(m.light_n, 0, 16, st);
+    e = cudaMemsetAsync(b + o_zero, 0, zero_end - o_zero, st);
     if (e == cudaSuccess) {
         GpuPass pass(ctx, "dictionary: sample counts");
         e = launch_dict_match(ma, ctx->sm_count, st, ctx->tune.dict_slice, ctx->tune.dict_blocks_per_sm);
     }
-    std::vector<uint32_t> sample(U);
-    uint32_t flags[2] = {0, 0};
-    if (e == cudaSuccess) e = cudaMemcpyAsync(sample.data(), m.sample_counts, (size_t)U * 4, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(flags, m.light_n, 8, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    prof_mark(ctx, "dictionary: wait for the sample");
-    if (e != cudaSuccess) return ctx_cuda(ctx, e, "search_many sample");
-    if (flags[1] & OL_DEVERR_TIMEOUT) return ctx_fail(ctx, OL_ERR_TIMEOUT, "search_many: a bounded wait ran out");
-    const double scale = (double)n_tiles / (double)n_work;
-    const double threshold = heavy_min_hits ? (double)heavy_min_hits : std::max(4096.0, (double)N / (double)std::max<uint32_t>(ctx->tune.dict_heavy_divisor, 1));
-    std::vector<std::pair<double, uint32_t>> cand;
-    double light_est = 0;
-    for (uint32_t u = 0; u < U; u++) {
-        double ex = sample[u] * scale;
-        if (sample[u] && ex >= threshold)
-            cand.emplace_back(-ex, u);
-        else
-            light_est += ex;
+    DictPlanArgs pa{};
+    pa.set = set->dev;
+    pa.sample_counts = ma.counts;
+    pa.least = (uint32_t)std::min(std::max(std::ceil(threshold / scale), 1.0), 4294967295.0);
+    pa.runs = set->d_runs;
+    pa.n_runs = (uint32_t)set->runs.size();
+    pa.heavy_of_u = b + o_heavy_of;
+    pa.heavy_u = (uint32_t *)(b + o_heavy_u);
+    pa.heavy_run = (uint32_t *)(b + o_hrun);
+    pa.run_light = (uint32_t *)(b + o_rlight);
+    pa.outs = (uint32_t *)(b + o_outs);
+    pa.plan = &meta->plan;
+    if (e == cudaSuccess) e = launch_dict_plan(pa, st);
+    uint32_t H = kDictMaxHeavy;
+    uint64_t cap = std::max<uint64_t>(N / 16, 65536);
+    if (e == cudaSuccess && n_tiles > kPlanTiles) {
+        e = read_meta();
+        prof_mark(ctx, "dictionary: wait for the sample");
+        if (e != cudaSuccess) return ctx_cuda(ctx, e, "search_many sample");
+        if (hm->error & OL_DEVERR_TIMEOUT) return ctx_fail(ctx, OL_ERR_TIMEOUT, "search_many: a bounded wait ran out");
+        H = hm->plan.n_heavy;
+        cap = std::min<uint64_t>(0xFFFFFFF0ull, (uint64_t)((double)hm->plan.light_sample * scale * 1.25) + 65536);
     }
-    std::sort(cand.begin(), cand.end());
-    if (cand.size() > kDictMaxHeavy) {
-        for (size_t i = kDictMaxHeavy; i < cand.size(); i++) light_est += -cand[i].first;
-        cand.resize(kDictMaxHeavy);
-    }
-    const uint32_t H = (uint32_t)cand.size();
-    std::vector<uint8_t> heavy_of(U, 0xFF);
-    std::vector<uint32_t> heavy_u(kDictMaxHeavy, 0);
-    for (uint32_t h = 0; h < H; h++) {
-        heavy_u[h] = cand[h].second;
-        heavy_of[cand[h].second] = (uint8_t)h;
-    }
-    // The run patterns: heavy ones by heavy index, the others listed.
-    std::vector<uint32_t> heavy_run(kDictMaxHeavy, 0), run_light;
-    for (uint32_t x : set->runs) {
-        const uint8_t h = heavy_of[x & 0xFFFFu];
-        if (h != 0xFF)
-            heavy_run[h] = x >> 16;
-        else
-            run_light.push_back(x);
-    }
-    e = cudaMemcpyAsync(m.heavy_of_u, heavy_of.data(), U, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(m.heavy_run, heavy_run.data(), kDictMaxHeavy * 4, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess && !run_light.empty())
-        e = cudaMemcpyAsync(m.run_light, run_light.data(), run_light.size() * 4, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(m.heavy_u, heavy_u.data(), kDictMaxHeavy * 4, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = launch_dict_outs(set->dev.outs, m.heavy_of_u, set->dev.n_outs, m.outs, st);
     if (e == cudaSuccess && H) e = ctx->dict_bitmap.reserve((size_t)H * n_words * 4, st);
     if (e != cudaSuccess) return ctx_cuda(ctx, e, "search_many");
 
-    // 2. The match pass; grown and re-run if the light keys overflow.
-    uint64_t cap = std::min<uint64_t>(0xFFFFFFF0ull, (uint64_t)(light_est * 1.25) + 65536);
-    uint32_t light_n = 0;
-    for (int attempt = 0; attempt < 3; attempt++) {
+    // 2. The match pass; 3. heavy ranks, light order, per-id slots; 4. hits.
+    //    The light keys' buffer is grown and the match pass run again if they
+    //    overflow it.
+    DictEmitArgs ea{};
+    auto timed_out = [&]() { return (hm->error & OL_DEVERR_TIMEOUT) != 0; };
+    auto hits_dest = [&](uint64_t k) -> cudaError_t {  // where hits go on the device: k of them
+        if (dest.off && !dest.pair_on_host) {
+            ea.hit_pat = dest.pat;
+            ea.hit_off = reinterpret_cast<unsigned long long *>(dest.off);
+        } else if (dest.dev) {
+            ea.hits = reinterpret_cast<uint2 *>(dest.dev);
+        } else {
+            const size_t off_at = (k * 4 + 255) & ~(size_t)255;  // pair form in scratch: patterns, then offsets
+            cudaError_t r = ctx->dict_hits.reserve(dest.off ? off_at + k * 8 : k * 8, st);
+            if (r != cudaSuccess) return r;
+            if (dest.off) {
+                ea.hit_pat = (uint32_t *)ctx->dict_hits.ptr;
+                ea.hit_off = (unsigned long long *)((uint8_t *)ctx->dict_hits.ptr + off_at);
+            } else {
+                ea.hits = (uint2 *)ctx->dict_hits.ptr;
+            }
+        }
+        ea.max_hits = k;
+        return cudaSuccess;
+    };
+    const bool on_device = max_hits && (dest.dev || (dest.off && !dest.pair_on_host));
+    bool emitted = false;
+    for (int attempt = 0;; attempt++) {
         e = ctx->dict_keys.reserve((size_t)cap * 16, st);
-        if (e == cudaSuccess) e = cudaMemsetAsync(m.light_count, 0, (size_t)U * 4, st);
-        if (e == cudaSuccess) e = cudaMemsetAsync(m.light_n, 0, 16, st);
-        if (e == cudaSuccess) e = cudaMemsetAsync(m.stats, 0, 16, st);
-        if (e == cudaSuccess && H) e = cudaMemsetAsync(m.heavy_counts, 0, (size_t)H * hld * 4, st);
-        ma.heavy_counts = m.heavy_counts;
-        ma.heavy_ld = hld;
-        ma.stats = m.stats;
+        cap = std::min<uint64_t>(ctx->dict_keys.bytes / 16, 0xFFFFFFF0ull);
+        if (e == cudaSuccess && attempt) e = cudaMemsetAsync(b + o_zero, 0, rezero_end - o_zero, st);
+        unsigned long long *keys = (unsigned long long *)ctx->dict_keys.ptr;
+        ma.stats = &meta->walked;
         ma.force_timeout = 0;
         ma.tile_stride = 1;
         ma.count_only = 0;
-        ma.counts = m.light_count;
-        ma.heavy_of_u = m.heavy_of_u;
-        ma.n_heavy = H;
-        ma.bitmap = H ? (uint32_t *)ctx->dict_bitmap.ptr : nullptr;
-        ma.light_keys = (unsigned long long *)ctx->dict_keys.ptr;
+        ma.counts = light_count;
+        ma.heavy_of_u = pa.heavy_of_u;
+        ma.plan = pa.plan;
+        ma.bitmap = (uint32_t *)ctx->dict_bitmap.ptr;
+        ma.heavy_counts = heavy_counts;
+        ma.heavy_ld = hld;
+        ma.light_keys = keys;
+        ma.off_bits = off_bits;
         ma.light_cap = (uint32_t)cap;
-        ma.light_n = m.light_n;
-        ma.outs = m.outs;
-        ma.heavy_run = m.heavy_run;
-        ma.run_light = m.run_light;
-        ma.n_run_light = (uint32_t)run_light.size();
+        ma.light_n = &meta->light_n;
+        ma.outs = pa.outs;
+        ma.heavy_run = pa.heavy_run;
+        ma.run_light = pa.run_light;
         if (e == cudaSuccess) {
             GpuPass pass(ctx, "dictionary: match");
             e = launch_dict_match(ma, ctx->sm_count, st, ctx->tune.dict_slice, ctx->tune.dict_blocks_per_sm);
         }
-        if (e == cudaSuccess) e = cudaMemcpyAsync(flags, m.light_n, 8, cudaMemcpyDeviceToHost, st);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-        prof_mark(ctx, "dictionary: wait for the match pass");
+        bool known = n_tiles > kFewTiles;  // the light key count, on the host
+        if (e == cudaSuccess && known) e = read_meta();
+        if (known) prof_mark(ctx, "dictionary: wait for the match pass");
         if (e != cudaSuccess) return ctx_cuda(ctx, e, "search_many match");
-        if (flags[1] & OL_DEVERR_TIMEOUT) return ctx_fail(ctx, OL_ERR_TIMEOUT, "search_many: a bounded wait ran out");
-        light_n = flags[0];
-        if (light_n <= cap) break;
-        cap = (uint64_t)light_n + 1024;
-        if (attempt == 2) return ctx_fail(ctx, OL_ERR_CUDA, "search_many: light hit count kept growing");
-    }
-
-    // 3. Heavy ranks, light order, per-id slots.
-    GpuPass order_pass(ctx, "dictionary: rank and sort");
-    if (H) {
-        e = launch_scan_columns(m.heavy_counts, m.heavy_bases, m.heavy_totals, n_tiles, H, hld, st);
-        if (e != cudaSuccess) return ctx_cuda(ctx, e, "search_many heavy");
-    }
-    unsigned long long *keys = (unsigned long long *)ctx->dict_keys.ptr;
-    if (light_n > 1) {
-        const size_t hist_bytes = (size_t)2 * 256 * scan_ld(dict_sort_chunks(light_n)) * 4;
-        if (ctx->dict_small.bytes < fixed + hist_bytes) {
-            // keep the scratch written so far: grow into a fresh buffer and copy it over
-            DevBuf grown;
-            e = grown.reserve(fixed + hist_bytes, st);
-            if (e == cudaSuccess) e = cudaMemcpyAsync(grown.ptr, ctx->dict_small.ptr, fixed, cudaMemcpyDeviceToDevice, st);
-            if (e != cudaSuccess) {
-                grown.release(st);
-                return ctx_cuda(ctx, e, "search_many sort");
+        if (known && timed_out()) return ctx_fail(ctx, OL_ERR_TIMEOUT, "search_many: a bounded wait ran out");
+        if (known && hm->light_n > cap) {
+            if (attempt == 2) return ctx_fail(ctx, OL_ERR_CUDA, "search_many: light hit count kept growing");
+            cap = (uint64_t)hm->light_n + 1024;
+            continue;
+        }
+        ea.n_ids = n;
+        ea.n_u = U;
+        ea.n_heavy = H;
+        ea.n_tiles = n_tiles;
+        ea.plan = pa.plan;
+        ea.u_of_id = set->u_of_id;
+        ea.dup_start = set->dup_start;
+        ea.dup_ids = set->dup_ids;
+        ea.heavy_of_u = pa.heavy_of_u;
+        ea.heavy_u = pa.heavy_u;
+        ea.heavy_totals = heavy_totals;
+        ea.heavy_counts = heavy_counts;
+        ea.heavy_bases = heavy_bases;
+        ea.ld = hld;
+        ea.bitmap = (const uint32_t *)ctx->dict_bitmap.ptr;
+        ea.light_count = light_count;
+        ea.light_base = (uint32_t *)(b + o_lbase);
+        ea.light_keys = keys;
+        ea.light_n_dev = &meta->light_n;
+        ea.light_max = known ? hm->light_n : kDictSortBlock;
+        ea.off_bits = off_bits;
+        ea.id_counts = (uint32_t *)(b + o_idc);
+        ea.id_base = (unsigned long long *)(b + o_idb);
+        ea.total = &meta->total;
+        auto order = [&]() -> cudaError_t {  // light order and per-id slots
+            cudaError_t r;
+            if (!known || hm->light_n <= kDictSortBlock) return launch_dict_sort_ids(ea, keys, key_bits, st);
+            const uint32_t light_n = hm->light_n;
+            r = ctx->dict_sort.reserve((size_t)2 * 256 * scan_ld(dict_sort_blocks(light_n)) * 4, st);
+            unsigned long long *sorted = keys;
+            if (r == cudaSuccess)
+                r = launch_dict_sort(keys, keys + cap, light_n, key_bits, (uint32_t *)ctx->dict_sort.ptr, (uint32_t *)(b + o_stot),
+                                     &sorted, st);
+            ea.light_keys = sorted;
+            ea.light_max = light_n;
+            return r == cudaSuccess ? launch_dict_ids(ea, st) : r;
+        };
+        auto emit = [&]() {
+            GpuPass pass(ctx, "dictionary: emit");
+            return launch_dict_emit(ea, st);
+        };
+        {
+            GpuPass order_pass(ctx, "dictionary: rank and sort");
+            if (H) e = launch_scan_columns(heavy_counts, heavy_bases, heavy_totals, n_tiles, H, hld, st);
+            if (e == cudaSuccess) e = order();
+        }
+        if (e == cudaSuccess && on_device) {
+            e = hits_dest(max_hits);
+            if (e == cudaSuccess) e = emit();
+            emitted = true;
+        }
+        if (e == cudaSuccess) e = read_meta();
+        prof_mark(ctx, "dictionary: wait for the slots");
+        if (e != cudaSuccess) return ctx_cuda(ctx, e, "search_many");
+        if (timed_out()) return ctx_fail(ctx, OL_ERR_TIMEOUT, "search_many: a bounded wait ran out");
+        if (!known && hm->light_n > kDictSortBlock) {  // more light keys than one block sorts
+            if (hm->light_n > cap) {
+                if (attempt == 2) return ctx_fail(ctx, OL_ERR_CUDA, "search_many: light hit count kept growing");
+                cap = (uint64_t)hm->light_n + 1024;
+                continue;
             }
-            ctx->dict_small.release(st);
-            ctx->dict_small = grown;
-            m = scratch_at((uint8_t *)ctx->dict_small.ptr);
+            known = true;
+            GpuPass order_pass(ctx, "dictionary: rank and sort");
+            e = order();
+            order_pass.done();
+            if (e == cudaSuccess && emitted) e = emit();
+            if (e == cudaSuccess) e = read_meta();
+            if (e != cudaSuccess) return ctx_cuda(ctx, e, "search_many");
         }
-        e = launch_dict_sort(keys, keys + cap, light_n, 32 + bits_for(U - 1), m.sort_hist, m.sort_totals, st);
-        if (e != cudaSuccess) return ctx_cuda(ctx, e, "search_many sort");
+        break;
     }
-    DictEmitArgs ea{};
-    ea.n_ids = n;
-    ea.n_u = U;
-    ea.n_heavy = H;
-    ea.n_tiles = n_tiles;
-    ea.u_of_id = set->u_of_id;
-    ea.dup_start = set->dup_start;
-    ea.dup_ids = set->dup_ids;
-    ea.heavy_of_u = m.heavy_of_u;
-    ea.heavy_u = m.heavy_u;
-    ea.heavy_totals = m.heavy_totals;
-    ea.heavy_counts = m.heavy_counts;
-    ea.heavy_bases = m.heavy_bases;
-    ea.ld = hld;
-    ea.bitmap = H ? (const uint32_t *)ctx->dict_bitmap.ptr : nullptr;
-    ea.light_count = m.light_count;
-    ea.light_base = m.light_base;
-    ea.light_keys = keys;
-    ea.light_n = light_n;
-    ea.id_counts = m.id_counts;
-    ea.id_base = m.id_base;
-    ea.total = m.total;
-    e = launch_dict_ids(ea, st);
-    order_pass.done();
-    unsigned long long tot = 0;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&tot, m.total, 8, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(counts, m.id_counts, (size_t)n * 4, cudaMemcpyDeviceToHost, st);
-    unsigned long long walk[2] = {0, 0};
-    if (e == cudaSuccess) e = cudaMemcpyAsync(walk, m.stats, 16, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    prof_mark(ctx, "dictionary: wait for the slots");
-    if (e != cudaSuccess) return ctx_cuda(ctx, e, "search_many ids");
-    *total = tot;
+    memcpy(counts, ctx->host_words.ptr + o_idc, (size_t)n * 4);
+    *total = hm->total;
     ctx->dict_stats[0] = N;
-    ctx->dict_stats[1] = walk[0];
-    ctx->dict_stats[2] = walk[1];
-    ctx->dict_stats[3] = H;
-    ctx->dict_stats[4] = light_n;
-    ctx->dict_stats[5] = tot;
+    ctx->dict_stats[1] = hm->walked;
+    ctx->dict_stats[2] = hm->nodes;
+    ctx->dict_stats[3] = hm->plan.n_heavy;
+    ctx->dict_stats[4] = hm->light_n;
+    ctx->dict_stats[5] = hm->total;
+    const uint64_t k = std::min<uint64_t>(hm->total, max_hits);
+    if (k == 0 || emitted) return OL_OK;
 
-    // 4. Hits.
-    const uint64_t k = std::min<uint64_t>(tot, max_hits);
-    if (k == 0) return OL_OK;
-    ea.max_hits = k;
-    const size_t off_at = (k * 4 + 255) & ~(size_t)255;  // pair form in scratch: patterns, then offsets
-    if (dest.off && !dest.pair_on_host) {
-        ea.hit_pat = dest.pat;
-        ea.hit_off = reinterpret_cast<unsigned long long *>(dest.off);
-    } else if (dest.dev) {
-        ea.hits = reinterpret_cast<uint2 *>(dest.dev);
-    } else {
-        const size_t need = dest.off ? off_at + k * 8 : k * 8;
-        if ((e = ctx->dict_hits.reserve(need, st)) != cudaSuccess) return ctx_cuda(ctx, e, "search_many hits");
-        if (dest.off) {
-            ea.hit_pat = (uint32_t *)ctx->dict_hits.ptr;
-            ea.hit_off = (unsigned long long *)((uint8_t *)ctx->dict_hits.ptr + off_at);
-        } else {
-            ea.hits = (uint2 *)ctx->dict_hits.ptr;
-        }
-    }
-    {
+    // Hits for the host: through scratch of their number.
+    ea.n_heavy = hm->plan.n_heavy;
+    ea.light_max = hm->light_n;
+    e = hits_dest(k);
+    if (e == cudaSuccess) {
         GpuPass pass(ctx, "dictionary: emit");
         e = launch_dict_emit(ea, st);
     }
