@@ -105,11 +105,14 @@ constexpr uint32_t kSearchMaxPatterns = 8;  // patterns per launch
 // pattern bytes (search_add_pattern) and read by every block as kernel
 // parameters.
 struct SearchPatMeta {
-    uint32_t pre[4];  // bytes 0..3, each replicated into a word (0 past the end)
-    uint32_t anc[4];  // anchor words (len >= 8): bytes [r, r + 4) little-endian, r = 1..4
+    uint32_t pre[4];  // bytes 0..3 (found by its rarest four bytes: r0..r0 + 3), each replicated into a word (0 past the end)
+    uint32_t anc[4];  // anchor words: bytes [r, r + 4) little-endian, r = r0 + 1 .. r0 + 4
     uint32_t len;
-    uint32_t f4;      // byte 0 replicated
+    uint32_t r0;
+    uint32_t last4;   // the last four bytes (len >= 4)
 };
+constexpr uint32_t kSearchPatBytes = 512;       // pattern bytes passed as kernel parameters
+constexpr uint32_t kSearchFinishTiles = 256;    // texts up to this size are finished in one launch
 
 struct SearchArgs {
     const uint8_t *text;     // padded: n_tiles * kSearchTile + kSearchMaxStagedPattern + 16 readable bytes
@@ -117,7 +120,7 @@ struct SearchArgs {
     uint32_t n_tiles;
     uint32_t np;                                // patterns in this launch (1..8)
     uint32_t halo;                              // round_up(longest - 1, 16); > 4096 only when np == 1
-    const uint8_t *pat[kSearchMaxPatterns];     // device copies
+    const uint8_t *pat[kSearchMaxPatterns];     // device copies (16-byte aligned), or nullptr: in pat_bytes
     uint32_t pat_len[kSearchMaxPatterns];
     uint32_t *out[kSearchMaxPatterns];          // ascending offsets, first max_out[p] of them
     uint32_t max_out[kSearchMaxPatterns];
@@ -136,12 +139,21 @@ struct SearchArgs {
     SearchPatMeta meta[kSearchMaxPatterns];
     uint32_t anchor_hash[kSearchMaxPatterns * 4];  // anchor-map bits of the patterns of >= 8 bytes
     uint32_t n_anchor;
-    uint32_t len_class[3];  // bit p: pattern p has <= 4 bytes; 5..7 bytes; 8 or more (search_add_pattern)
+    uint32_t anchor_words;  // aligned text words past a tile that may be anchors of starts in it
+    // bit p: pattern p is decided whole (up to 7 bytes); found by its anchors, by
+    // its rarest four bytes, or as a run of one byte (search_add_pattern)
+    uint32_t len_class[4];
+    // The bytes of patterns without a device copy, each from a 16-byte boundary.
+    uint32_t n_pat_bytes;
+    uint32_t pat_at[kSearchMaxPatterns];
+    alignas(16) uint8_t pat_bytes[kSearchPatBytes];
 };
 constexpr uint32_t kSearchStageCap = 8192;  // staged hits per tile (all patterns of a launch)
 
-// Appends a pattern to a launch (slot a.np): its device copy, and the
-// constants the kernels take from its host bytes.
+// Appends a pattern to a launch (slot a.np): its device copy (nullptr: its
+// bytes go into the launch's parameters, which search_takes_pattern_bytes tells
+// have room), and the constants the kernels take from its host bytes.
+bool search_takes_pattern_bytes(const SearchArgs &a, uint32_t len);
 void search_add_pattern(SearchArgs &a, const uint8_t *host, const uint8_t *dev, uint32_t len, uint32_t *out,
                         uint32_t max_out);
 cudaError_t launch_search(const SearchArgs &a, cudaStream_t st);

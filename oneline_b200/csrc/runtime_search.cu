@@ -17,17 +17,24 @@ static uint32_t halo_for(uint32_t m) { return ((m > 0 ? m - 1 : 0) + 15u) & ~15u
 
 namespace {
 
+// Patterns of up to this length travel in the launch's parameters (eight of
+// them fit), longer ones through device memory.
+constexpr uint32_t kInlinePattern = kSearchPatBytes / kSearchMaxPatterns;
+
 // Enqueues searches of n patterns over doc, at most 8 per launch (longer than
 // the staged limit: one per launch). Results stay on the device: d_totals[i]
-// and d_outs[i]. Pattern bytes are copied to device memory first.
+// and d_outs[i]. The bytes of long patterns are copied to device memory first.
 cudaError_t enqueue_multi(ol_ctx *ctx, const ol_doc *d, const uint8_t *const *pats, const uint32_t *lens, uint32_t n,
                           const uint32_t *max_out, uint32_t *d_totals, uint32_t *const *d_outs) {
     cudaStream_t st = ctx->stream;
     uint32_t n_tiles = (uint32_t)((d->text_len + kSearchTile - 1) / kSearchTile);
     size_t total_bytes = 0;
-    for (uint32_t i = 0; i < n; i++) total_bytes += (lens[i] + 15) & ~15u;
-    cudaError_t e = ctx->pattern_dev.reserve(std::max<size_t>(total_bytes, 16), st);
-    if (e == cudaSuccess) e = ctx->scratch_a.reserve((size_t)scan_ld(n_tiles) * kSearchMaxPatterns * 4 * 2, st);
+    for (uint32_t i = 0; i < n; i++)
+        if (lens[i] > kInlinePattern) total_bytes += (lens[i] + 15) & ~15u;
+    cudaError_t e = ctx->scratch_a.reserve((size_t)scan_ld(n_tiles) * kSearchMaxPatterns * 4 * 2, st);
+    std::vector<const uint8_t *> dp(n, nullptr);
+    if (e == cudaSuccess && total_bytes == 0) return ol::launch_multi(ctx, d, pats, dp.data(), lens, n, max_out, d_totals, d_outs);
+    if (e == cudaSuccess) e = ctx->pattern_dev.reserve(total_bytes, st);
     if (e != cudaSuccess) return e;
     // Patterns travel through pinned host staging so the copy is truly async
     // and the caller's buffers may be reused once this call returns.
@@ -47,23 +54,24 @@ cudaError_t enqueue_multi(ol_ctx *ctx, const ol_doc *d, const uint8_t *const *pa
     std::vector<size_t> at(n);
     size_t w = 0;
     for (uint32_t i = 0; i < n; i++) {
+        if (lens[i] <= kInlinePattern) continue;
         at[i] = w;
         memcpy(ctx->pat_host + w, pats[i], lens[i]);
         w += (lens[i] + 15) & ~15u;
     }
     uint8_t *dpat = (uint8_t *)ctx->pattern_dev.ptr;
-    if ((e = cudaMemcpyAsync(dpat, ctx->pat_host, std::max<size_t>(w, 1), cudaMemcpyHostToDevice, st)) != cudaSuccess) return e;
+    if ((e = cudaMemcpyAsync(dpat, ctx->pat_host, w, cudaMemcpyHostToDevice, st)) != cudaSuccess) return e;
     if ((e = cudaEventRecord(ctx->pat_done, st)) != cudaSuccess) return e;
-    std::vector<const uint8_t *> dp(n);
-    for (uint32_t i = 0; i < n; i++) dp[i] = dpat + at[i];
+    for (uint32_t i = 0; i < n; i++)
+        if (lens[i] > kInlinePattern) dp[i] = dpat + at[i];
     return ol::launch_multi(ctx, d, pats, dp.data(), lens, n, max_out, d_totals, d_outs);
 }
 
 }  // namespace
 
-// Launches the searches of n patterns already in device memory (dpats[i]; the
-// same bytes on the host: hpats[i]) over doc, at most 8 per launch (longer
-// than the staged limit: one per launch). Only stream operations: a CUDA
+// Launches the searches of n patterns (hpats[i]; those longer than
+// kInlinePattern also in device memory, dpats[i]) over doc, at most 8 per launch
+// (longer than the staged limit: one per launch). Only stream operations: a CUDA
 // graph can capture it once the context's scratch is large enough.
 cudaError_t ol::launch_multi(ol_ctx *ctx, const ol_doc *d, const uint8_t *const *hpats, const uint8_t *const *dpats,
                              const uint32_t *lens, uint32_t n, const uint32_t *max_out, uint32_t *d_totals,
@@ -100,7 +108,7 @@ cudaError_t ol::launch_multi(ol_ctx *ctx, const ol_doc *d, const uint8_t *const 
         while (i < n && a.np < kSearchMaxPatterns) {
             bool long_pat = halo_for(lens[i]) > kSearchMaxStagedPattern;
             if (a.np > 0 && (alone || long_pat)) break;
-            search_add_pattern(a, hpats[i], dpats[i], lens[i], d_outs[i], max_out[i]);
+            search_add_pattern(a, hpats[i], lens[i] <= kInlinePattern ? nullptr : dpats[i], lens[i], d_outs[i], max_out[i]);
             halo = std::max(halo, halo_for(lens[i]));
             i++;
             if (alone) break;
@@ -113,6 +121,9 @@ cudaError_t ol::launch_multi(ol_ctx *ctx, const ol_doc *d, const uint8_t *const 
 }
 
 namespace {
+
+// Results (room for every match asked for) up to this size come back in one copy.
+constexpr size_t kWholeResult = 64 << 10;
 
 // Blocking multi-pattern search into host buffers.
 ol_status search_multi_host(ol_ctx *ctx, const ol_doc *d, const uint8_t *const *pats, const uint32_t *lens, uint32_t n,
@@ -130,7 +141,12 @@ ol_status search_multi_host(ol_ctx *ctx, const ol_doc *d, const uint8_t *const *
         }
     if (idx.empty()) return OL_OK;
     cudaError_t e = ctx->search_out.reserve(out_words * 4 + 64 * 4, st);
+    // a small result comes back whole in one copy, totals and room for matches;
+    // else the totals first, then the matches there are
+    const bool whole = idx.size() <= 64 && out_words * 4 <= kWholeResult;
+    if (e == cudaSuccess) e = ctx->host_words.reserve(64 * 4 + (whole ? out_words * 4 : 0));
     if (e != cudaSuccess) return ctx_cuda(ctx, e, "search");
+    const uint32_t *back = (const uint32_t *)ctx->host_words.ptr;
     uint32_t *dev = (uint32_t *)ctx->search_out.ptr;
     uint32_t *d_totals = dev;  // 64 slots
     std::vector<const uint8_t *> p2;
@@ -147,11 +163,21 @@ ol_status search_multi_host(ol_ctx *ctx, const ol_doc *d, const uint8_t *const *
     for (size_t c = 0; c < idx.size(); c += 64) {
         uint32_t cn = (uint32_t)std::min<size_t>(64, idx.size() - c);
         e = enqueue_multi(ctx, d, p2.data() + c, l2.data() + c, cn, m2.data() + c, d_totals, o2.data() + c);
-        uint32_t tot_h[64];
-        if (e == cudaSuccess) e = cudaMemcpyAsync(tot_h, d_totals, cn * 4, cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(ctx->host_words.ptr, d_totals, whole ? (64 + out_words) * 4 : cn * 4, cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         prof_mark(ctx, "search: wait for totals");
         if (e != cudaSuccess) return ctx_cuda(ctx, e, "search");
+        uint32_t tot_h[64];
+        memcpy(tot_h, back, cn * 4);
+        if (whole) {
+            for (uint32_t j = 0; j < cn; j++) {
+                totals[idx[j]] = tot_h[j];
+                const uint32_t k = std::min(tot_h[j], m2[j]);
+                if (k) memcpy(outs[idx[j]], back + (o2[j] - dev), (size_t)k * 4);
+            }
+            return OL_OK;
+        }
         {
             GpuPass pass(ctx, "download");
             for (uint32_t j = 0; j < cn; j++) {
