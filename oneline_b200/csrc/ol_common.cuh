@@ -30,7 +30,6 @@ struct FlatNode {
 // Device status bits (DocStats::error and friends).
 constexpr uint32_t OL_DEVERR_TIMEOUT = 1u << 0;   // a bounded wait ran out
 constexpr uint32_t OL_DEVERR_CAPACITY = 1u << 1;  // an output buffer was too small
-constexpr uint32_t OL_DEVERR_DEEP = 1u << 3;      // a content line deeper than the fast tree path handles
 
 // Per-launch counters that live in device memory next to a document.
 struct DocStats {

@@ -17,7 +17,9 @@ struct DocStats;
 
 constexpr uint32_t kParseTile = 16384;  // text bytes per parse tile
 constexpr uint32_t kParseHalo = 256;    // bytes staged past a tile
-constexpr uint32_t kTreeTile = 4096;    // lines per tree tile (256 threads x 16)
+constexpr uint32_t kTreeTile = 4096;      // lines per tree tile (256 threads x 16)
+constexpr uint32_t kTreeSmallTile = 1024;  // of a document of at most kTreeFewTiles such tiles
+constexpr uint32_t kTreeFewTiles = 64;     // tiles whose summaries every block scans itself
 constexpr uint32_t kTreeLevels = 32;    // depth levels of the fast tree path
 
 constexpr uint32_t kParseSlotCap = 1024;      // staged lines per tile
@@ -67,7 +69,7 @@ struct TreeArgs {
     const uint8_t *kinds;
     const uint8_t *depth8;
     uint32_t L;
-    uint32_t n_tiles;        // ceil(L / kTreeTile)
+    uint32_t n_tiles;        // ceil(L / tree_tile_lines(L))
     uint32_t levels;         // max content depth + 1 (<= kTreeLevels)
     uint32_t *tile_last;     // n_tiles * kTreeLevels: last content line + 1 of each depth in the tile (0: none)
     uint32_t *tile_first;    // n_tiles * kTreeLevels: first content line of each depth in the tile (NONE: none)
@@ -80,6 +82,7 @@ struct TreeArgs {
     uint32_t *next_sibling;
 };
 
+uint32_t tree_tile_lines(uint32_t L);  // lines per tile of a document of L lines
 cudaError_t launch_tree_fast(const TreeArgs &a, cudaStream_t st);
 
 // Any-depth path (content lines deeper than kTreeLevels-1).

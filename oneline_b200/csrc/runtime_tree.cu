@@ -33,7 +33,7 @@ namespace {
 cudaError_t enqueue_tree_fast(ol_ctx *ctx, const ol_doc *d, ol_tree *t) {
     cudaStream_t st = ctx->stream;
     uint32_t L = d->line_count;
-    uint32_t n_tiles = (L + kTreeTile - 1) / kTreeTile;
+    const uint32_t lines = tree_tile_lines(L), n_tiles = (L + lines - 1) / lines;
     size_t words = (size_t)n_tiles * kTreeLevels;
     cudaError_t e = ctx->scratch_a.reserve(words * 4 * 4, st);
     if (e != cudaSuccess) return e;
@@ -109,14 +109,9 @@ ol_status build(ol_ctx *ctx, const ol_doc *d, ol_tree *t, uint32_t flags, bool w
     }
     if (e != cudaSuccess) return ctx_cuda(ctx, e, "tree");
     if (!wait) return OL_OK;
-    uint32_t err = 0;
-    e = cudaMemcpyAsync(&ctx->host_counters->error, &d->stats->error, 4, cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    e = cudaStreamSynchronize(ctx->stream);
     prof_mark(ctx, "tree: wait for links");
-    if (e != cudaSuccess) return ctx_cuda(ctx, e, "tree");
-    err = ctx->host_counters->error;
-    if (err & OL_DEVERR_DEEP) return ctx_fail(ctx, OL_ERR_CUDA, "tree: depth above the fast path reached the kernels");
-    return OL_OK;
+    return ctx_cuda(ctx, e, "tree");
 }
 
 }  // namespace

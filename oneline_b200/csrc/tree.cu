@@ -10,7 +10,11 @@
 // derived from those links.
 //
 // Fast path (every content line has depth < 32; D = max depth + 1 levels),
-// three kernels over tiles of 4096 lines (256 threads x 16 consecutive lines):
+// three kernels over tiles of 4096 lines (256 threads x 16 consecutive lines;
+// of 1024 lines, 4 a thread, where that leaves at most kTreeFewTiles tiles: a
+// thread's lines are a serial chain). With at most kTreeFewTiles tiles the
+// second kernel is left out and every block of the third one scans the tiles'
+// summaries itself; a single tile needs the third one alone:
 //   summary : per tile and level k, the last and the first line of depth k;
 //   scan    : per level, the exclusive prefix max (last line before the tile)
 //             and suffix min (first line after it) over the tiles;
@@ -35,48 +39,54 @@
 namespace ol {
 
 constexpr uint32_t TR_THREADS = 256;
-constexpr uint32_t TR_RUN = 16;
-static_assert(TR_THREADS * TR_RUN == kTreeTile, "tree tile");
+static_assert(TR_THREADS * 16 == kTreeTile && TR_THREADS * 4 == kTreeSmallTile, "tree tiles");
 
 __device__ __forceinline__ uint32_t mask_below(uint32_t d) { return d >= 32 ? 0xFFFFFFFFu : ((1u << d) - 1u); }
 __device__ __forceinline__ uint32_t mask_le(uint32_t d) { return d >= 31 ? 0xFFFFFFFFu : ((2u << d) - 1u); }
 
-// The 16 lines of thread `tid` of tile `tile`: kinds and depths packed four per word.
+// The RUN lines (4 or 16) of thread `tid` of tile `tile`: the level of each, or
+// 0xFF for a blank line, four per word. Depths >= levels cannot reach this path
+// (the host picks the any-depth path for them).
+template <uint32_t RUN>
 struct Run {
-    uint4 kd, dp;
+    uint32_t lv[RUN / 4];
     uint64_t first;
 };
 
-__device__ __forceinline__ Run load_run(const TreeArgs &a, uint32_t tile, uint32_t tid) {
-    Run r;
-    r.first = (uint64_t)tile * kTreeTile + tid * TR_RUN;
-    if (r.first + 16 <= a.L) {
-        r.kd = *reinterpret_cast<const uint4 *>(a.kinds + r.first);
-        r.dp = *reinterpret_cast<const uint4 *>(a.depth8 + r.first);
-    } else {
-        uint8_t k[16], d[16];
-#pragma unroll
-        for (int i = 0; i < 16; i++) {
-            bool in = r.first + i < a.L;
-            k[i] = in ? a.kinds[r.first + i] : (uint8_t)KIND_BLANK;  // past the end: blank
-            d[i] = in ? a.depth8[r.first + i] : (uint8_t)0;
+template <uint32_t RUN>
+__device__ __forceinline__ Run<RUN> load_run(const TreeArgs &a, uint32_t tile, uint32_t tid) {
+    Run<RUN> r;
+    r.first = ((uint64_t)tile * TR_THREADS + tid) * RUN;
+    uint32_t kd[RUN / 4], dp[RUN / 4];
+    if (r.first + RUN <= a.L) {
+        if (RUN == 16) {
+            *reinterpret_cast<uint4 *>(kd) = *reinterpret_cast<const uint4 *>(a.kinds + r.first);
+            *reinterpret_cast<uint4 *>(dp) = *reinterpret_cast<const uint4 *>(a.depth8 + r.first);
+        } else {
+            kd[0] = *reinterpret_cast<const uint32_t *>(a.kinds + r.first);
+            dp[0] = *reinterpret_cast<const uint32_t *>(a.depth8 + r.first);
         }
-        r.kd = *reinterpret_cast<uint4 *>(k);
-        r.dp = *reinterpret_cast<uint4 *>(d);
+    } else {
+#pragma unroll
+        for (uint32_t w = 0; w < RUN / 4; w++) {
+            kd[w] = dp[w] = 0;  // past the end: blank
+            for (uint32_t i = 0; i < 4; i++) {
+                if (r.first + 4 * w + i >= a.L) break;
+                kd[w] |= (uint32_t)a.kinds[r.first + 4 * w + i] << (8 * i);
+                dp[w] |= (uint32_t)a.depth8[r.first + 4 * w + i] << (8 * i);
+            }
+        }
     }
+    static_assert(KIND_BLANK == 0, "a blank line's kind byte is zero");
+    const uint32_t top = (a.levels - 1) * 0x01010101u;
+#pragma unroll
+    for (uint32_t w = 0; w < RUN / 4; w++) r.lv[w] = __vminu4(dp[w], top) | ((zero_bytes(kd[w]) >> 7) * 0xFFu);
     return r;
 }
 
-__device__ __forceinline__ uint32_t byte_of(const uint4 &v, int i) {
-    uint32_t w = i < 4 ? v.x : i < 8 ? v.y : i < 12 ? v.z : v.w;
-    return (w >> (8 * (i & 3))) & 0xFF;
-}
-
-// Level of a line for the tree, or 0xFF for a blank line. Depths >= levels
-// cannot reach this path (the host picks the any-depth path for them).
-__device__ __forceinline__ uint32_t level_of(const Run &r, int i, uint32_t levels) {
-    if (byte_of(r.kd, i) == KIND_BLANK) return 0xFF;
-    return min(byte_of(r.dp, i), levels - 1);
+template <uint32_t RUN>
+__device__ __forceinline__ uint32_t level_of(const Run<RUN> &r, int i) {
+    return (r.lv[i >> 2] >> (8 * (i & 3))) & 0xFFu;
 }
 
 // Dynamic shared memory of the summary and resolve kernels: D levels x 256
@@ -99,23 +109,24 @@ __device__ __forceinline__ TreeSmem tree_smem(uint32_t D) {
 }
 
 // Pass 1: per tile and level, the last line (+1) and the first line of that depth.
+template <uint32_t RUN>
 __global__ void __launch_bounds__(TR_THREADS) tree_summary_kernel(TreeArgs a) {
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tile = blockIdx.x;
     const uint32_t D = a.levels;
     TreeSmem sm = tree_smem(D);
-    Run r = load_run(a, tile, tid);
+    const Run<RUN> r = load_run<RUN>(a, tile, tid);
     for (uint32_t k = 0; k < D; k++) {
         sm.a(k, tid) = 0;
         sm.b(k, tid) = NONE;
     }
 #pragma unroll
-    for (int i = 0; i < 16; i++) {
-        uint32_t d = level_of(r, i, D);
+    for (int i = 0; i < (int)RUN; i++) {
+        uint32_t d = level_of(r, i);
         if (d != 0xFF) sm.a(d, tid) = (uint32_t)(r.first + i + 1);
     }
 #pragma unroll
-    for (int i = 15; i >= 0; i--) {
-        uint32_t d = level_of(r, i, D);
+    for (int i = RUN - 1; i >= 0; i--) {
+        uint32_t d = level_of(r, i);
         if (d != 0xFF) sm.b(d, tid) = (uint32_t)(r.first + i);
     }
     __syncthreads();
@@ -216,27 +227,51 @@ __global__ void __launch_bounds__(1024) tree_scan_kernel(TreeArgs a) {
     }
 }
 
+// v to p[at .. at + W), W lines of which those below L exist; at is a multiple of
+// W and the arrays are 256-byte aligned.
+template <uint32_t W>
+__device__ __forceinline__ void put_words(uint32_t *p, uint64_t at, uint32_t L, const uint32_t (&v)[W]) {
+    if (at + W <= L) {
+        if constexpr (W == 8)
+            asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p + at), "r"(v[0]), "r"(v[1]),
+                         "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                         : "memory");
+        else
+            *reinterpret_cast<uint4 *>(p + at) = make_uint4(v[0], v[1], v[2], v[3]);
+    } else {
+        for (uint32_t q = 0; q < W; q++)
+            if (at + q < L) p[at + q] = v[q];
+    }
+}
+
 // Pass 3: every thread rebuilds the ancestor stack before its 16 lines and
 // the stack of the lines after them, walks forward for parent (and the
 // parent's depth, kept in registers) and backward for subtree_end,
 // first_child and next_sibling.
-__global__ void __launch_bounds__(TR_THREADS, 5) tree_resolve_kernel(TreeArgs a) {
+// What bounds it is the serial chain of a thread's lines, and the stores: with 16
+// bytes at a time every 32-byte sector was written in two halves; whole sectors
+// at a time, and four blocks an SM without spills instead of five, took 72
+// against 93 us for 11 M lines.
+// FEW: at most kTreeFewTiles tiles, whose summaries are scanned here.
+template <uint32_t RUN, bool FEW>
+__global__ void __launch_bounds__(TR_THREADS, 4) tree_resolve_kernel(TreeArgs a) {
+    constexpr uint32_t W = RUN < 8 ? RUN : 8;  // lines stored at a time
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, tile = blockIdx.x;
     const uint32_t D = a.levels;
     TreeSmem sm = tree_smem(D);
-    Run r = load_run(a, tile, tid);
+    const Run<RUN> r = load_run<RUN>(a, tile, tid);
     for (uint32_t k = 0; k < D; k++) {
         sm.a(k, tid) = 0;
         sm.b(k, tid) = NONE;
     }
 #pragma unroll
-    for (int i = 0; i < 16; i++) {
-        uint32_t d = level_of(r, i, D);
+    for (int i = 0; i < (int)RUN; i++) {
+        uint32_t d = level_of(r, i);
         if (d != 0xFF) sm.a(d, tid) = (uint32_t)(r.first + i + 1);
     }
 #pragma unroll
-    for (int i = 15; i >= 0; i--) {
-        uint32_t d = level_of(r, i, D);
+    for (int i = RUN - 1; i >= 0; i--) {
+        uint32_t d = level_of(r, i);
         if (d != 0xFF) sm.b(d, tid) = (uint32_t)(r.first + i);
     }
     __syncthreads();
@@ -247,6 +282,22 @@ __global__ void __launch_bounds__(TR_THREADS, 5) tree_resolve_kernel(TreeArgs a)
     // 16-byte loads), reduces them, and one warp scan of the 32 lane values
     // gives each lane its seed.
     for (uint32_t k = warp; k < D; k += 8) {
+        uint32_t in_last, in_first;
+        if (!FEW) {
+            in_last = a.in_last[(size_t)tile * kTreeLevels + k];
+            in_first = a.in_first[(size_t)tile * kTreeLevels + k];
+        } else {  // (a single tile has no summaries)
+            in_last = 0;
+            in_first = NONE;
+#pragma unroll
+            for (uint32_t i = 0; i < kTreeFewTiles / 32; i++) {
+                const uint32_t t = i * 32 + lane;
+                if (t < tile) in_last = max(in_last, a.tile_last[(size_t)t * kTreeLevels + k]);
+                if (t > tile && t < a.n_tiles) in_first = min(in_first, a.tile_first[(size_t)t * kTreeLevels + k]);
+            }
+            in_last = __reduce_max_sync(0xFFFFFFFFu, in_last);
+            in_first = __reduce_min_sync(0xFFFFFFFFu, in_first);
+        }
         uint4 *ra = reinterpret_cast<uint4 *>(&sm.a(k, 8 * lane));
         uint4 *rb = reinterpret_cast<uint4 *>(&sm.b(k, 8 * lane));
         {
@@ -261,7 +312,7 @@ __global__ void __launch_bounds__(TR_THREADS, 5) tree_resolve_kernel(TreeArgs a)
                 if ((int)lane >= o) inc = max(inc, t);
             }
             const uint32_t prev = __shfl_up_sync(0xFFFFFFFFu, inc, 1);
-            uint32_t run = max(a.in_last[(size_t)tile * kTreeLevels + k], lane == 0 ? 0u : prev);
+            uint32_t run = max(in_last, lane == 0 ? 0u : prev);
 #pragma unroll
             for (int i = 0; i < 8; i++) {
                 const uint32_t t = v[i];
@@ -283,7 +334,7 @@ __global__ void __launch_bounds__(TR_THREADS, 5) tree_resolve_kernel(TreeArgs a)
                 if (lane + o < 32) inc = min(inc, t);
             }
             const uint32_t next = __shfl_down_sync(0xFFFFFFFFu, inc, 1);
-            uint32_t run = min(a.in_first[(size_t)tile * kTreeLevels + k], lane == 31 ? NONE : next);
+            uint32_t run = min(in_first, lane == 31 ? NONE : next);
 #pragma unroll
             for (int i = 7; i >= 0; i--) {
                 const uint32_t t = v[i];
@@ -306,11 +357,13 @@ __global__ void __launch_bounds__(TR_THREADS, 5) tree_resolve_kernel(TreeArgs a)
             runmax = v;
         }
     }
-    uint32_t pdw[4] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu};  // parent depth bytes, 0xFF = none
-    uint32_t par[4];
+    uint32_t pdw[RUN / 4];  // parent depth bytes, 0xFF = none
 #pragma unroll
-    for (int i = 0; i < 16; i++) {
-        uint32_t d = level_of(r, i, D);
+    for (uint32_t w = 0; w < RUN / 4; w++) pdw[w] = 0xFFFFFFFFu;
+    uint32_t par[W];
+#pragma unroll
+    for (int i = 0; i < (int)RUN; i++) {
+        uint32_t d = level_of(r, i);
         uint32_t pv = NONE;
         if (d != 0xFF) {
             uint32_t low = M & mask_below(d);
@@ -322,14 +375,8 @@ __global__ void __launch_bounds__(TR_THREADS, 5) tree_resolve_kernel(TreeArgs a)
             M = low | (1u << d);
             sm.a(d, tid) = (uint32_t)(r.first + i + 1);
         }
-        par[i & 3] = pv;
-        if ((i & 3) == 3) {
-            uint64_t at = r.first + (i - 3);
-            if (at + 4 <= a.L) *reinterpret_cast<uint4 *>(a.parent + at) = make_uint4(par[0], par[1], par[2], par[3]);
-            else
-                for (int q = 0; q < 4; q++)
-                    if (at + q < a.L) a.parent[at + q] = par[q];
-        }
+        par[i % W] = pv;
+        if (i % W == W - 1) put_words<W>(a.parent, r.first + i + 1 - W, a.L, par);
     }
 
     // Backward: level k is on the stack of following lines iff its first line
@@ -344,11 +391,11 @@ __global__ void __launch_bounds__(TR_THREADS, 5) tree_resolve_kernel(TreeArgs a)
             runmin = v;
         }
     }
-    uint32_t se[4], fc[4], ns[4];
+    uint32_t se[W], fc[W], ns[W];
 #pragma unroll
-    for (int i = 15; i >= 0; i--) {
+    for (int i = RUN - 1; i >= 0; i--) {
         uint64_t line = r.first + i;
-        uint32_t d = level_of(r, i, D);
+        uint32_t d = level_of(r, i);
         uint32_t vse = (uint32_t)(line + 1), vfc = NONE, vns = NONE;
         if (d != 0xFF) {
             if (M) {
@@ -368,40 +415,44 @@ __global__ void __launch_bounds__(TR_THREADS, 5) tree_resolve_kernel(TreeArgs a)
             M = (M & mask_below(d)) | (1u << d);
             sm.b(d, tid) = (uint32_t)line;
         }
-        se[i & 3] = vse;
-        fc[i & 3] = vfc;
-        ns[i & 3] = vns;
-        if ((i & 3) == 0) {
-            uint64_t at = line;
-            if (at + 4 <= a.L) {
-                if (a.subtree_end) *reinterpret_cast<uint4 *>(a.subtree_end + at) = make_uint4(se[0], se[1], se[2], se[3]);
-                *reinterpret_cast<uint4 *>(a.first_child + at) = make_uint4(fc[0], fc[1], fc[2], fc[3]);
-                *reinterpret_cast<uint4 *>(a.next_sibling + at) = make_uint4(ns[0], ns[1], ns[2], ns[3]);
-            } else {
-                for (int q = 0; q < 4; q++) {
-                    if (at + q >= a.L) continue;
-                    if (a.subtree_end) a.subtree_end[at + q] = se[q];
-                    a.first_child[at + q] = fc[q];
-                    a.next_sibling[at + q] = ns[q];
-                }
-            }
+        se[i % W] = vse;
+        fc[i % W] = vfc;
+        ns[i % W] = vns;
+        if (i % W == 0) {
+            if (a.subtree_end) put_words<W>(a.subtree_end, line, a.L, se);
+            put_words<W>(a.first_child, line, a.L, fc);
+            put_words<W>(a.next_sibling, line, a.L, ns);
         }
     }
 }
 
-cudaError_t launch_tree_fast(const TreeArgs &a, cudaStream_t st) {
-    if (a.n_tiles == 0) return cudaSuccess;
+uint32_t tree_tile_lines(uint32_t L) { return L <= kTreeFewTiles * kTreeSmallTile ? kTreeSmallTile : kTreeTile; }
+
+template <uint32_t RUN, bool FEW>
+static cudaError_t launch_tree_run(const TreeArgs &a, cudaStream_t st) {
     size_t smem = (size_t)a.levels * TR_THREADS * 4 * 2;
     if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(tree_summary_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = cudaFuncSetAttribute(tree_summary_kernel<RUN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(tree_resolve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            e = cudaFuncSetAttribute(tree_resolve_kernel<RUN, FEW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
     }
-    tree_summary_kernel<<<a.n_tiles, TR_THREADS, smem, st>>>(a); OL_LAUNCHED();
-    tree_scan_kernel<<<a.levels, 1024, 0, st>>>(a); OL_LAUNCHED();
-    tree_resolve_kernel<<<a.n_tiles, TR_THREADS, smem, st>>>(a); OL_LAUNCHED();
+    if (a.n_tiles > 1) {
+        tree_summary_kernel<RUN><<<a.n_tiles, TR_THREADS, smem, st>>>(a); OL_LAUNCHED();
+    }
+    if (!FEW) {
+        tree_scan_kernel<<<a.levels, 1024, 0, st>>>(a); OL_LAUNCHED();
+    }
+    tree_resolve_kernel<RUN, FEW><<<a.n_tiles, TR_THREADS, smem, st>>>(a); OL_LAUNCHED();
     return cudaGetLastError();
+}
+
+// 1 MiB (21,000 lines, 17 levels) took 21.5 us in three kernels of 16 lines a
+// thread: 10.9 us in two of 4.
+cudaError_t launch_tree_fast(const TreeArgs &a, cudaStream_t st) {
+    if (a.n_tiles == 0) return cudaSuccess;
+    if (tree_tile_lines(a.L) == kTreeSmallTile) return launch_tree_run<4, true>(a, st);
+    return a.n_tiles <= kTreeFewTiles ? launch_tree_run<16, true>(a, st) : launch_tree_run<16, false>(a, st);
 }
 
 // ------------------------------------------------------------ any depth ----
