@@ -87,11 +87,13 @@ cudaError_t launch_tree_fast(const TreeArgs &a, cudaStream_t st);
 
 // Any-depth path (content lines deeper than kTreeLevels-1).
 struct TreeDeepArgs {
-    const uint32_t *keys;    // depth of content lines, NONE for blank lines
+    const uint8_t *kinds;
+    const uint8_t *depth8;
+    const uint32_t *keys;    // depth of content lines, NONE for blank lines; nullptr: depth8 holds every depth
     uint32_t L;
-    uint32_t *levels[8];     // levels[0] = keys, levels[k] = min over 32 of levels[k-1]
+    uint32_t *levels[8];     // minima: levels[0] of every 32 lines, levels[k] of 32 of levels[k-1]
     uint32_t level_len[8];
-    uint32_t n_levels;
+    uint32_t n_levels;       // at least 2; the last one has at most 32 entries
     uint32_t *parent;
     uint32_t *subtree_end;
     uint32_t *first_child;

@@ -56,33 +56,33 @@ cudaError_t enqueue_tree_fast(ol_ctx *ctx, const ol_doc *d, ol_tree *t) {
     return launch_tree_fast(a, st);
 }
 
-// Any-depth path: exact depths, 32-ary min tree, per-line searches.
+// Any-depth path: the minima of a 32-ary tree over the depths (exact ones from
+// the text where depth8 is clamped), per-line searches.
 cudaError_t enqueue_tree_deep(ol_ctx *ctx, const ol_doc *d, ol_tree *t) {
     cudaStream_t st = ctx->stream;
-    uint32_t L = d->line_count;
+    const uint32_t L = d->line_count;
     TreeDeepArgs a{};
+    a.kinds = d->kinds;
+    a.depth8 = d->depth8;
     a.L = L;
-    size_t total = 0;
-    uint32_t len = L, n_levels = 0;
-    uint32_t lens[8];
-    while (true) {
-        lens[n_levels++] = len;
-        total += (size_t)len * 4;
-        if (len <= 1 || n_levels == 8) break;
-        len = (len + 31) / 32;
-    }
-    cudaError_t e = ctx->scratch_c.reserve(total, st);
+    const size_t key_words = d->max_depth >= 255 ? L : 0;
+    size_t total = key_words;
+    size_t at[8];
+    uint32_t len = L;
+    do {
+        len = (uint32_t)(((uint64_t)len + 31) / 32);
+        a.level_len[a.n_levels] = len;
+        at[a.n_levels++] = total;
+        total += len;
+    } while (a.n_levels < 2 || len > 32);
+    cudaError_t e = ctx->scratch_c.reserve(total * 4, st);
     if (e != cudaSuccess) return e;
-    size_t at = 0;
-    for (uint32_t l = 0; l < n_levels; l++) {
-        a.levels[l] = (uint32_t *)((uint8_t *)ctx->scratch_c.ptr + at);
-        a.level_len[l] = lens[l];
-        at += (size_t)lens[l] * 4;
+    for (uint32_t l = 0; l < a.n_levels; l++) a.levels[l] = (uint32_t *)ctx->scratch_c.ptr + at[l];
+    if (key_words) {
+        a.keys = (uint32_t *)ctx->scratch_c.ptr;
+        e = launch_classify_lines(d->text, d->text_len, d->offsets, L, nullptr, (uint32_t *)ctx->scratch_c.ptr, st);
+        if (e != cudaSuccess) return e;
     }
-    a.n_levels = n_levels;
-    a.keys = a.levels[0];
-    e = launch_classify_lines(d->text, d->text_len, d->offsets, L, nullptr, a.levels[0], st);
-    if (e != cudaSuccess) return e;
     a.parent = (uint32_t *)t->parent_buf.ptr;
     a.subtree_end = (uint32_t *)t->end_buf.ptr;
     a.first_child = (uint32_t *)t->fc_buf.ptr;
