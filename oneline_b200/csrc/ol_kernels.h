@@ -174,15 +174,19 @@ struct QueryArgs {
     const FlatNode *nodes;   // ... or materialised nodes (then the four above are unused)
     uint32_t lines;          // lines in the document
     uint32_t lo, hi;         // range [lo, hi) of lines considered
+    const uint32_t *hi_dev;  // its end on the device (at most hi), or nullptr
     uint32_t target_kind;    // 0: any
     uint32_t target_depth;   // NONE: any
+    uint16_t *masks;         // kQueryMasks per block
     uint32_t *counts;        // per block of 4096 lines, 16-byte aligned
     uint32_t *bases;         // same size, 16-byte aligned
     uint32_t *total;         // device
     uint32_t *out;           // ascending line indices, first max_out of them
     uint32_t max_out;
 };
-uint32_t query_blocks(uint32_t lines);
+constexpr uint32_t kQueryMasks = 256;
+constexpr uint32_t kQuerySelfScan = 8192;  // blocks (33 M lines) whose counts the writing blocks add up themselves
+uint32_t query_blocks(uint32_t lo, uint32_t hi);
 cudaError_t launch_query(const QueryArgs &a, cudaStream_t st);
 
 // ------------------------------------------------------------ dictionary --

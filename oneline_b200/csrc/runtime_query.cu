@@ -5,6 +5,8 @@
 // matching line indices, ascending.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <cstring>
 #include <string>
 
 #include "runtime.h"
@@ -13,16 +15,22 @@ using namespace ol;
 
 namespace {
 
+// Matches that come back together with their number; more take a second copy.
+constexpr uint32_t kQueryFirst = 16384;
+
 // Runs the filter over lines [lo, hi) of a resident document (or over `nodes`
-// when given) and downloads the result.
+// when given; hi_dev: the range's end on the device, at most hi) and downloads
+// the result.
 ol_status run_query(ol_ctx *ctx, const ol_doc *d, const FlatNode *nodes, uint32_t lines, uint32_t lo, uint32_t hi,
-                    uint32_t kind, uint32_t depth, uint32_t max_matches, uint32_t *total, uint32_t *out) {
+                    const uint32_t *hi_dev, uint32_t kind, uint32_t depth, uint32_t max_matches, uint32_t *total,
+                    uint32_t *out) {
     cudaStream_t st = ctx->stream;
     *total = 0;
     if (hi <= lo) return OL_OK;
-    const uint32_t blocks = query_blocks(hi - lo), ld = scan_ld(blocks);
-    const size_t small = ((size_t)2 * ld + 4) * 4;
-    cudaError_t e = ctx->search_out.reserve(small + (size_t)std::max<uint32_t>(max_matches, 1) * 4, st);
+    const uint32_t blocks = query_blocks(lo, hi), ld = scan_ld(blocks), first = std::min(max_matches, kQueryFirst);
+    const size_t small = ((size_t)2 * ld + 4) * 4, masks = (size_t)blocks * kQueryMasks * 2;
+    cudaError_t e = ctx->search_out.reserve(small + masks + (size_t)std::max<uint32_t>(max_matches, 1) * 4, st);
+    if (e == cudaSuccess) e = ctx->host_words.reserve((4 + (size_t)first) * 4);
     if (e != cudaSuccess) return ctx_cuda(ctx, e, "query");
     uint32_t *w = (uint32_t *)ctx->search_out.ptr;
     QueryArgs a{};
@@ -37,26 +45,34 @@ ol_status run_query(ol_ctx *ctx, const ol_doc *d, const FlatNode *nodes, uint32_
     a.lines = lines;
     a.lo = lo;
     a.hi = hi;
+    a.hi_dev = hi_dev;
     a.target_kind = kind;
     a.target_depth = depth;
+    a.masks = (uint16_t *)w;
+    w += masks / 4;
     a.counts = w;
     a.bases = w + ld;
-    a.total = w + 2 * ld;
+    a.total = w + 2 * ld;  // the total, then (16 bytes on) the matches: one copy brings both
     a.out = w + 2 * ld + 4;
     a.max_out = max_matches;
     {
         GpuPass pass(ctx, "query");
         e = launch_query(a, st);
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(total, a.total, 4, cudaMemcpyDeviceToHost, st);
+    const uint32_t *back = (const uint32_t *)ctx->host_words.ptr;
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(ctx->host_words.ptr, a.total, (4 + (size_t)first) * 4, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     prof_mark(ctx, "query: wait for the count");
-    const uint32_t k = std::min(*total, max_matches);
-    if (e == cudaSuccess && k) {
+    if (e != cudaSuccess) return ctx_cuda(ctx, e, "query");
+    *total = back[0];
+    const uint32_t k = std::min(*total, max_matches), k0 = std::min(k, first);
+    if (k0) memcpy(out, back + 4, (size_t)k0 * 4);
+    if (k > k0) {
         GpuPass pass(ctx, "download");
-        e = cudaMemcpyAsync(out, a.out, (size_t)k * 4, cudaMemcpyDeviceToHost, st);
+        e = cudaMemcpyAsync(out + k0, a.out + k0, (size_t)(k - k0) * 4, cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     prof_mark(ctx, "query: download matches");
     return ctx_cuda(ctx, e, "query");
 }
@@ -68,7 +84,8 @@ extern "C" ol_status ol_query_document(ol_ctx *ctx, const ol_doc *d, uint32_t ki
     if (!ctx || !d || !total || (max_matches && !out)) return OL_ERR_INVALID_ARG;
     std::lock_guard<std::recursive_mutex> g(ctx->mu);
     cudaSetDevice(ctx->device);
-    return run_query(ctx, d, nullptr, d->line_count, 0, d->line_count, kind, depth, max_matches, total, out);
+    return run_query(ctx, d, nullptr, d->line_count, 0, d->line_count, nullptr, kind, depth, max_matches, total,
+                     out);
 }
 
 extern "C" ol_status ol_query_subtree(ol_ctx *ctx, const ol_doc *d, const ol_tree *t, uint64_t root, uint32_t kind,
@@ -80,11 +97,9 @@ extern "C" ol_status ol_query_subtree(ol_ctx *ctx, const ol_doc *d, const ol_tre
                             std::to_string(d->line_count) + " lines, tree has " + std::to_string(t->line_count) + ")");
     std::lock_guard<std::recursive_mutex> g(ctx->mu);
     cudaSetDevice(ctx->device);
-    uint32_t end = 0;
-    cudaError_t e = cudaMemcpyAsync(&end, (const uint32_t *)t->end_buf.ptr + root, 4, cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    if (e != cudaSuccess) return ctx_cuda(ctx, e, "query_subtree");
-    return run_query(ctx, d, nullptr, d->line_count, (uint32_t)root, end, kind, depth, max_matches, total, out);
+    // the subtree's end stays on the device: blocks past it have nothing to do
+    return run_query(ctx, d, nullptr, d->line_count, (uint32_t)root, d->line_count, (const uint32_t *)t->end_buf.ptr + root, kind,
+                     depth, max_matches, total, out);
 }
 
 extern "C" ol_status ol_query_raw(ol_ctx *ctx, const uint8_t *text, uint64_t len, uint32_t kind, uint32_t depth,
@@ -122,8 +137,8 @@ extern "C" ol_status ol_query(ol_ctx *ctx, const uint8_t *text, uint64_t len, co
                                   (FlatNode *)ctx->scratch_c.ptr, nullptr, st);
     s = ctx_cuda(ctx, e, "query");
     if (s == OL_OK)
-        s = run_query(ctx, d, (const FlatNode *)ctx->scratch_c.ptr, (uint32_t)n_lines, 0, (uint32_t)n_lines, kind, depth,
-                      max_matches, total, out);
+        s = run_query(ctx, d, (const FlatNode *)ctx->scratch_c.ptr, (uint32_t)n_lines, 0, (uint32_t)n_lines, nullptr, kind,
+                      depth, max_matches, total, out);
     ol_doc_free(d);
     return s;
 }
