@@ -125,9 +125,24 @@ __global__ void batch_split_kernel(const BatchSplitDoc *__restrict__ docs, const
     if ((threadIdx.x & 31) == 0 && deepest) atomicMax(max_depth + lo, deepest);
 }
 
+// 16 bytes from src + sh, 16 * i bytes further on, for the threads' pieces i < n
+// of an aligned destination: two aligned loads (the second one's bytes are the
+// next thread's first), words Q .. Q + 4 of them shifted by sh bits.
+template <uint32_t Q>
+__device__ __forceinline__ void pack_pieces(const uint4 *src, uint4 *dst, uint32_t n, uint32_t sh) {
+    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+        const uint4 a = __ldg(src + i), b = Q || sh ? __ldg(src + i + 1) : a;
+        const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        dst[i] = make_uint4(__funnelshift_r(w[Q], w[Q + 1], sh), __funnelshift_r(w[Q + 1], w[Q + 2], sh),
+                            __funnelshift_r(w[Q + 2], w[Q + 3], sh), __funnelshift_r(w[Q + 3], w[Q + 4], sh));
+    }
+}
+
 // Item `blockIdx.x` of the documents' items (item_start: the prefix sum of
 // batch_pack_items): the document's bytes [64 KiB k, 64 KiB (k + 1)), and its
-// separator in its last item.
+// separator in its last item. Bound by memory: byte by byte it took 190 us for
+// 126 MB, 16 bytes at a time 48 us (`in` is readable for 32 bytes past its
+// end).
 __global__ void batch_pack_kernel(const BatchPackDoc *__restrict__ docs, const uint32_t *__restrict__ item_start,
                                   uint32_t n, const uint8_t *__restrict__ in, uint8_t *__restrict__ text) {
     const uint32_t item = blockIdx.x;
@@ -144,7 +159,20 @@ __global__ void batch_pack_kernel(const BatchPackDoc *__restrict__ docs, const u
     const uint64_t b1 = min(d.len, b0 + kBatchPackBytes);
     const uint8_t *src = in + d.src;
     uint8_t *dst = text + d.dst;
-    for (uint64_t j = b0 + threadIdx.x; j < b1; j += blockDim.x) dst[j] = src[j];
+    const uint64_t head = b0 + min(b1 - b0, (uint64_t)(-(uintptr_t)(dst + b0) & 15));  // up to an aligned destination
+    const uint32_t pieces = (uint32_t)((b1 - head) / 16);
+    for (uint64_t j = b0 + threadIdx.x; j < head; j += blockDim.x) dst[j] = src[j];
+    for (uint64_t j = head + (uint64_t)pieces * 16 + threadIdx.x; j < b1; j += blockDim.x) dst[j] = src[j];
+    const uintptr_t from = (uintptr_t)(src + head);
+    const uint4 *s16 = reinterpret_cast<const uint4 *>(from & ~(uintptr_t)15);
+    uint4 *d16 = reinterpret_cast<uint4 *>(dst + head);
+    const uint32_t sh = (from & 3) * 8;
+    switch ((from & 15) >> 2) {  // uniform
+        case 0: pack_pieces<0>(s16, d16, pieces, sh); break;
+        case 1: pack_pieces<1>(s16, d16, pieces, sh); break;
+        case 2: pack_pieces<2>(s16, d16, pieces, sh); break;
+        default: pack_pieces<3>(s16, d16, pieces, sh); break;
+    }
     if (d.sep && threadIdx.x == 0 && b0 + kBatchPackBytes >= d.len) dst[d.len] = '\n';
 }
 

@@ -119,7 +119,7 @@ cudaError_t batch_fill_pinned(ol_ctx *ctx, ol_batch *b, const uint8_t *data, con
     if (items > 0x7FFFFFFFull) return cudaErrorInvalidValue;
     const size_t table = ((size_t)n * sizeof(BatchPackDoc) + (size_t)(n + 1) * 4 + 255) & ~(size_t)255;
     DevBuf tmp;
-    cudaError_t e = tmp.reserve(table + std::max<uint64_t>(in_bytes, 16), st);
+    cudaError_t e = tmp.reserve(table + in_bytes + 32, st);
     uint8_t *base = (uint8_t *)tmp.ptr;
     if (e == cudaSuccess) e = cudaMemcpyAsync(base, docs.data(), (size_t)n * sizeof(BatchPackDoc), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess)
