@@ -63,6 +63,14 @@ __device__ __forceinline__ uint4 ld_stream16(const void *p) {
     return v;
 }
 
+// 16 bytes from device to shared memory without registers in between (both
+// aligned); cp_async_wait waits for all of this thread's.
+__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // ------------------------------------------------------------ byte SWAR ----
 
 // High bit of each byte of x set exactly where that byte is zero.
@@ -71,25 +79,18 @@ __device__ __forceinline__ uint32_t zero_bytes(uint32_t x) {
     return ~(y | x | 0x7F7F7F7Fu);
 }
 
-// 4-bit mask (bit i = byte i) of bytes of w equal to c4's byte.
-__device__ __forceinline__ uint32_t eq_mask4(uint32_t w, uint32_t c4) {
-    uint32_t z = zero_bytes(w ^ c4);  // bits 7,15,23,31
-    // gather bits 7,15,23,31 into 0..3
-    return ((z >> 7) & 1u) | ((z >> 14) & 2u) | ((z >> 21) & 4u) | ((z >> 28) & 8u);
+// 16-bit mask (bit i = byte i) from the high bits of four SWAR words (nothing
+// but high bits set): the bytes, each 0 or 128, times their places' weights, in
+// one four-way dot product a word.
+__device__ __forceinline__ uint32_t gather16(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3) {
+    const uint32_t lo = __dp4a(c0, 0x08040201u, __dp4a(c1, 0x80402010u, 0u));
+    const uint32_t hi = __dp4a(c2, 0x08040201u, __dp4a(c3, 0x80402010u, 0u));
+    return (lo >> 7) | (hi << 1);
 }
 
 // 16-bit mask of the bytes of a 16-byte vector equal to byte c.
 __device__ __forceinline__ uint32_t eq_mask16(uint4 v, uint32_t c4) {
-    return eq_mask4(v.x, c4) | (eq_mask4(v.y, c4) << 4) | (eq_mask4(v.z, c4) << 8) | (eq_mask4(v.w, c4) << 12);
-}
-
-// 16-bit mask (bit i = byte i) from the high bits of four SWAR words. One
-// multiply gathers two words: the high bits of c0 (moved to bits 0, 8, 16,
-// 24) and of c1 (bits 4, 12, 20, 28) land, shifted by 21, 14, 7 and 0, on bits
-// 21..28 in byte order; no two partial products meet, so nothing carries.
-__device__ __forceinline__ uint32_t gather16(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3) {
-    auto g2 = [](uint32_t lo, uint32_t hi) { return ((((lo >> 7) | (hi >> 3)) * 0x00204081u) >> 21) & 0xFFu; };
-    return g2(c0, c1) | (g2(c2, c3) << 8);
+    return gather16(zero_bytes(v.x ^ c4), zero_bytes(v.y ^ c4), zero_bytes(v.z ^ c4), zero_bytes(v.w ^ c4));
 }
 
 __device__ __forceinline__ bool is_blank(uint8_t b) { return b == ' ' || b == '\t'; }

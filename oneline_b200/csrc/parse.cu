@@ -1,8 +1,8 @@
 // Kernel (a)+(b): newline scan fused with per-line classification.
 //
 // The text is read once and no block ever waits on another:
-//   1. parse_stage_kernel: per 16 KiB tile, the newline count (16-byte
-//      coalesced vector loads, exact byte SWAR, popc, warp scans), the
+//   1. parse_stage_kernel: per 16 KiB tile, the newline count (asynchronous
+//      16-byte copies, exact byte SWAR, popc, warp scans), the
 //      newline positions in order, and the classification of every line
 //      starting in the tile from shared memory, staged as one word per line
 //      in the tile's slot; also the tile's first newline and deepest line;
@@ -32,6 +32,7 @@
 namespace ol {
 
 constexpr uint32_t PT_THREADS = 256;
+constexpr uint32_t PT_WARPS = PT_THREADS / 32;
 constexpr uint32_t PT_STEPS = 4;                          // 16-byte pieces per thread
 constexpr uint32_t PT_TILE = PT_THREADS * 16 * PT_STEPS;  // 16384
 constexpr uint32_t PT_HALO = 256;
@@ -41,13 +42,11 @@ static_assert(PT_TILE == kParseTile && PT_HALO == kParseHalo, "tile geometry");
 static_assert(PT_LIST == kParseSlotCap && kParseFinishTiles % PT_THREADS == 0, "slot and finish geometry");
 
 struct ParseSmem {
-    alignas(16) uint8_t text[PT_TILE + PT_HALO + 16];  // +16: word reads may run 3 bytes past
-    uint16_t nl[PT_LIST + 1];        // newline positions of the current round, ascending
-    uint32_t warp_tot[PT_STEPS][8];  // newline count per (step, warp)
-    uint32_t warp_base[PT_STEPS][8];
-    uint32_t halo_first;             // first newline in the halo (local), or NONE
-    uint32_t tile_nl;                // newlines in the tile
-    uint32_t long_idx, long_start;   // the line left to classify_long (long_start: tile-local), or NONE
+    alignas(16) uint8_t text[PT_TILE + PT_HALO + 32];  // +32: reads of 16 unaligned bytes may run past
+    uint16_t nl[PT_LIST + 1];                 // newline positions of the current round, ascending
+    uint32_t warp_tot[PT_WARPS];              // newlines of each warp's 2 KiB
+    uint32_t halo_first;                      // first newline in the halo (local), or NONE
+    uint32_t long_idx, long_start;  // the line left to classify_long (long_start: tile-local), or NONE
 };
 
 // Staged form: a tile's lines as one word each, (start, kind, depth8) or a
@@ -65,67 +64,71 @@ __device__ __forceinline__ uint32_t lds4(const uint8_t *base, uint32_t off) {
     return __funnelshift_r(w[0], w[1], (off & 3) * 8);
 }
 
-// High bit of every byte of w equal to '|'.
-__device__ __forceinline__ uint32_t pipe_bits(uint32_t w) { return zero_bytes(w ^ 0x7C7C7C7Cu); }
-
 // parse_line (crates/oneline-simd/src/line.rs:8-44) for a line held in shared
 // memory at tile-local [s, e), e = its '\n' or the text end; the bytes from e
 // to e+3 are readable. The prefix is read as alternating runs: a run of '|'
-// four bytes per step (byte SWAR), then a run of blanks; it continues only
-// while another '|' follows the blanks.
+// sixteen bytes per step, then a run of blanks; it continues only while another
+// '|' follows the blanks. The usual line, one blank or none before its content,
+// needs no look at single bytes.
 __device__ __forceinline__ uint32_t classify_smem(const uint8_t *t, uint32_t s, uint32_t e, uint32_t &depth_out) {
     uint32_t eff = e;
     while (eff > s && t[eff - 1] == '\r') eff--;
     uint32_t c = s, depth = 0;
-    if (s < eff && t[s] == '|') {
+    uint32_t w = lds4(t, c);
+    if (s < eff && (w & 0xFFu) == '|') {
         for (;;) {
             // run of '|' (stops at a non-'|' byte, at the latest at eff)
             for (;;) {
-                uint32_t other = ~pipe_bits(lds4(t, c)) & 0x80808080u;
-                if (other) {
-                    uint32_t nb = (__ffs(other) - 8) >> 3;
-                    depth += nb;
-                    c += nb;
-                    break;
-                }
-                depth += 4;
-                c += 4;
+                const uint32_t *q = reinterpret_cast<const uint32_t *>(t) + (c >> 2);
+                const uint32_t sh = (c & 3) * 8, a0 = q[0], a1 = q[1], a2 = q[2], a3 = q[3], a4 = q[4];
+                uint32_t x = __funnelshift_r(a0, a1, sh) ^ 0x7C7C7C7Cu, at = 0;
+                if (!x) x = __funnelshift_r(a1, a2, sh) ^ 0x7C7C7C7Cu, at = 4;
+                if (!x) x = __funnelshift_r(a2, a3, sh) ^ 0x7C7C7C7Cu, at = 8;
+                if (!x) x = __funnelshift_r(a3, a4, sh) ^ 0x7C7C7C7Cu, at = 12;
+                if (x) at += (__ffs(x) - 1) >> 3;
+                else at = 16;
+                depth += at;
+                c += at;
+                if (at < 16) break;
             }
             // run of blanks; the prefix goes on only if a '|' follows it
-            uint32_t b = c;
-            while (b < eff && is_blank(t[b])) b++;
-            if (b < eff && t[b] == '|') {
-                c = b;
-                continue;
+            w = lds4(t, c);
+            if (c >= eff || !is_blank((uint8_t)w)) break;
+            const uint8_t next = (uint8_t)(w >> 8);
+            if (c + 1 < eff && next != '|' && !is_blank(next)) {
+                c++;
+                w >>= 8;
+                break;
             }
+            uint32_t b = c + 1;
+            while (b < eff && is_blank(t[b])) b++;
             c = b;
+            if (b < eff && t[b] == '|') continue;
+            w = lds4(t, c);
             break;
         }
-    } else {
+    } else if (s < eff && is_blank((uint8_t)w)) {
         while (c < eff && is_blank(t[c])) c++;
+        w = lds4(t, c);
     }
     depth_out = depth;
     if (c >= eff) return KIND_BLANK;
-    uint32_t w = lds4(t, c);
     return classify3((uint8_t)w, (uint8_t)(w >> 8), (uint8_t)(w >> 16), eff - c);
 }
 
-// Exact '\n' bits (high bit of each byte) of a 16-byte piece at tile-local lo;
-// bytes at or past `valid` are cleared.
-__device__ __forceinline__ void newline_bits(const uint4 &v, uint32_t lo, uint32_t valid, uint32_t z[4]) {
-    const uint32_t NL4 = 0x0A0A0A0Au;
-    z[0] = zero_bytes(v.x ^ NL4);
-    z[1] = zero_bytes(v.y ^ NL4);
-    z[2] = zero_bytes(v.z ^ NL4);
-    z[3] = zero_bytes(v.w ^ NL4);
-    if (lo + 16 > valid) {
-#pragma unroll
-        for (uint32_t i = 0; i < 4; i++) {
-            uint32_t b0 = lo + 4 * i;  // bytes b0..b0+3; keep those < valid
-            uint32_t keep = b0 >= valid ? 0u : (valid - b0 >= 4 ? 4u : valid - b0);
-            z[i] &= keep == 4 ? 0xFFFFFFFFu : ((1u << (8 * keep)) - 1u);
-        }
-    }
+// 32-bit mask of the positions lo .. lo + 31 below n.
+__device__ __forceinline__ uint32_t below32(uint32_t n, uint32_t lo) {
+    return n <= lo ? 0u : n - lo >= 32 ? 0xFFFFFFFFu : (1u << (n - lo)) - 1u;
+}
+
+// Exact newline mask of a 16-byte piece: bit b = byte b. ('\n' is below 0x80, so
+// three operations a word tell it from every byte.)
+__device__ __forceinline__ uint32_t newline_mask(const uint4 &v) {
+    auto bits = [](uint32_t w) {  // high bit of every newline byte
+        const uint32_t y = ((w ^ 0x0A0A0A0Au) & 0x7F7F7F7Fu) + 0x7F7F7F7Fu;
+        return ~(y | w) & 0x80808080u;
+    };
+    return gather16(bits(v.x), bits(v.y), bits(v.z), bits(v.w));
 }
 
 // The first newline at or past tile t0, or N: the whole warp scans the tiles'
@@ -186,77 +189,57 @@ __device__ __forceinline__ void parse_tile(const ParseArgs &a, ParseSmem &sm, ui
     // bytes of this tile (and halo) that belong to the text
     const uint32_t valid = N - t0 >= PT_TILE + PT_HALO ? PT_TILE + PT_HALO : (uint32_t)(N - t0);
 
-    // 1. Coalesced 16-byte loads: step k covers [t0 + k*4096, +4096), lane-major.
-    uint4 v[PT_STEPS];
+    // 1. The tile and its halo into shared memory, 16 bytes a copy, without a stop
+    //    in registers: the pass needs 32 of them and runs eight blocks an SM
+    //    (through registers six: 113 against 101 us per 256 MiB).
 #pragma unroll
-    for (uint32_t k = 0; k < PT_STEPS; k++) v[k] = ld_stream16(a.text + t0 + k * 4096 + tid * 16);
-    uint4 vh = make_uint4(0, 0, 0, 0);
-    if (tid < PT_HALO / 16) vh = ld_stream16(a.text + t0 + PT_TILE + tid * 16);
+    for (uint32_t k = 0; k < PT_STEPS; k++) cp_async16(&sm.text[k * 4096 + tid * 16], a.text + t0 + k * 4096 + tid * 16);
+    if (tid < PT_HALO / 16) cp_async16(&sm.text[PT_TILE + tid * 16], a.text + t0 + PT_TILE + tid * 16);
     if (tid == 0) {
-        sm.halo_first = NONE;
         sm.long_idx = NONE;
         *reinterpret_cast<uint4 *>(&sm.text[PT_TILE + PT_HALO]) = make_uint4(0, 0, 0, 0);
+        *reinterpret_cast<uint4 *>(&sm.text[PT_TILE + PT_HALO + 16]) = make_uint4(0, 0, 0, 0);
     }
-#pragma unroll
-    for (uint32_t k = 0; k < PT_STEPS; k++) *reinterpret_cast<uint4 *>(&sm.text[k * 4096 + tid * 16]) = v[k];
-    if (tid < PT_HALO / 16) *reinterpret_cast<uint4 *>(&sm.text[PT_TILE + tid * 16]) = vh;
+    cp_async_wait();
+    __syncthreads();  // (a) text in shared memory
 
-    // 2. Newline bits and their ranks within the warp: steps (0,1) and (2,3)
-    //    packed in 16-bit fields.
-    uint32_t nlm[PT_STEPS];  // bit b: byte b of the thread's piece in step k is a newline
-    uint32_t cnt[PT_STEPS];
-#pragma unroll
-    for (uint32_t k = 0; k < PT_STEPS; k++) {
-        uint32_t z[4];
-        newline_bits(v[k], k * 4096 + tid * 16, valid, z);
-        nlm[k] = gather16(z[0], z[1], z[2], z[3]);
-        cnt[k] = __popc(nlm[k]);
+    // 2. Newlines of the thread's 64 consecutive bytes, and their rank: one count
+    //    and one scan per thread, and ranks in thread order. (Four strided pieces
+    //    a thread, straight from the loads, took twice the instructions: a scan
+    //    each, and a list of 32 totals.)
+    const uint32_t mine = tid * 64;
+    uint32_t m0, m1;  // bit b: byte mine + b, mine + 32 + b
+    {
+        const uint4 *own = reinterpret_cast<const uint4 *>(&sm.text[mine]);
+        m0 = newline_mask(own[0]) | (newline_mask(own[1]) << 16);
+        m1 = newline_mask(own[2]) | (newline_mask(own[3]) << 16);
     }
-    uint32_t c01 = cnt[0] | (cnt[1] << 16), c23 = cnt[2] | (cnt[3] << 16);
-    uint32_t i01 = c01, i23 = c23;
+    if (valid < PT_TILE) {  // uniform: the last tile
+        m0 &= below32(valid, mine);
+        m1 &= below32(valid, mine + 32);
+    }
+    const uint32_t cnt = __popc(m0) + __popc(m1);
+    uint32_t rank = cnt;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        uint32_t t1 = __shfl_up_sync(0xFFFFFFFFu, i01, o);
-        uint32_t t2 = __shfl_up_sync(0xFFFFFFFFu, i23, o);
-        if ((int)lane >= o) {
-            i01 += t1;
-            i23 += t2;
-        }
+        const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, rank, o);
+        if ((int)lane >= o) rank += t;
     }
-    const uint32_t r01 = i01 - c01, r23 = i23 - c23;
-    if (lane == 31) {
-        sm.warp_tot[0][warp] = i01 & 0xFFFF;
-        sm.warp_tot[1][warp] = i01 >> 16;
-        sm.warp_tot[2][warp] = i23 & 0xFFFF;
-        sm.warp_tot[3][warp] = i23 >> 16;
-    }
-    __syncthreads();  // (a) halo_first initialised, warp totals visible
-    if (tid < PT_HALO / 16) {
+    if (lane == 31) sm.warp_tot[warp] = rank;
+    rank -= cnt;
+    if (warp == 0) {  // the halo's first newline
+        uint32_t m = tid < PT_HALO / 16 ? newline_mask(*reinterpret_cast<const uint4 *>(&sm.text[PT_TILE + tid * 16])) : 0u;
         const uint32_t lo = PT_TILE + tid * 16;
-        uint32_t first = NONE;
-        uint32_t zh[4];
-        newline_bits(vh, lo, valid, zh);
-#pragma unroll
-        for (int i = 3; i >= 0; i--)
-            if (zh[i]) first = lo + 4 * i + ((__ffs(zh[i]) - 8) >> 3);
-        for (int o = 8; o > 0; o >>= 1) first = min(first, __shfl_xor_sync(0x0000FFFFu, first, o));
+        if (valid < PT_TILE + PT_HALO) m &= below32(valid, lo);
+        const uint32_t first = __reduce_min_sync(0xFFFFFFFFu, m ? lo + __ffs(m) - 1 : NONE);
         if (tid == 0) sm.halo_first = first;
     }
-    if (warp == 1) {
-        // 32 (step, warp) totals in position order: index = k*8 + w.
-        uint32_t c = sm.warp_tot[lane >> 3][lane & 7], inc = c;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            uint32_t t = __shfl_up_sync(0xFFFFFFFFu, inc, o);
-            if ((int)lane >= o) inc += t;
-        }
-        sm.warp_base[lane >> 3][lane & 7] = inc - c;
-        if (lane == 31) sm.tile_nl = inc;
-    }
-    __syncthreads();  // (b) bases and halo_first visible
+    __syncthreads();  // (b) totals and halo_first visible
+    const uint32_t t8 = lane < PT_WARPS ? sm.warp_tot[lane] : 0u;
+    const uint32_t n_nl = __reduce_add_sync(0xFFFFFFFFu, t8);
+    rank += __reduce_add_sync(0xFFFFFFFFu, lane < warp ? t8 : 0u);
 
     const uint32_t off = tile == 0 ? 1u : 0u;
-    const uint32_t n_nl = sm.tile_nl;
     const uint32_t n_lines = n_nl + off;
     if (STAGE) {
         const bool over = n_lines > a.slot_cap;
@@ -276,23 +259,17 @@ __device__ __forceinline__ void parse_tile(const ParseArgs &a, ParseSmem &sm, ui
     // classify and write the round's lines.
     for (uint32_t r0 = 0; r0 < n_lines; r0 += PT_LIST) {
         const int32_t w0 = (int32_t)r0 - (int32_t)off;  // rank of nl[0]
-#pragma unroll
-        for (uint32_t k = 0; k < PT_STEPS; k++) {
-            uint32_t rr = (k & 1) ? ((k < 2 ? r01 : r23) >> 16) : ((k < 2 ? r01 : r23) & 0xFFFF);
-            int32_t rk = (int32_t)(sm.warp_base[k][warp] + rr) - w0;
-            if (rk > (int32_t)PT_LIST) continue;
-            // one loop over the piece's 16-bit newline mask: the warp runs as
-            // many rounds as its busiest lane has newlines in this piece
-            uint32_t m = nlm[k];
-            while (m) {
-                const uint32_t b = __ffs(m) - 1;
-                m &= m - 1;
-                if (rk >= 0 && rk <= (int32_t)PT_LIST) sm.nl[rk] = (uint16_t)(k * 4096 + tid * 16 + b);
-                rk++;
-            }
+        int32_t rk = (int32_t)rank - w0;
+        if (rk <= (int32_t)PT_LIST) {
+            auto list = [&](uint32_t m, uint32_t lo) {  // the warp runs as many rounds as its busiest lane has newlines
+                for (; m; m &= m - 1, rk++)
+                    if (STAGE || (rk >= 0 && rk <= (int32_t)PT_LIST)) sm.nl[rk] = (uint16_t)(lo + __ffs(m) - 1);
+            };
+            list(m0, mine);
+            list(m1, mine + 32);
         }
         __syncthreads();  // (c) list ready
-        if (STAGE && tid == 0) a.tile_first[tile] = n_nl ? sm.nl[0] : NONE;
+        if (STAGE && tid == 0) a.tile_first[tile] = n_nl ? sm.nl[off] : NONE;
 
         const uint32_t r_end = min(n_lines, r0 + PT_LIST);
         for (uint32_t j = r0 + tid; j < r_end; j += PT_THREADS) {
@@ -334,7 +311,8 @@ __device__ __forceinline__ void parse_tile(const ParseArgs &a, ParseSmem &sm, ui
             }
             if (kind != KIND_BLANK) my_max = max(my_max, depth);
         }
-        __syncthreads();  // (d) the next round may overwrite the list
+        // (d) the next round overwrites the list; in place, long_idx and long_start are complete
+        if (!STAGE || r0 + PT_LIST < n_lines) __syncthreads();
     }
     my_max = __reduce_max_sync(0xFFFFFFFFu, my_max);
     if (STAGE) {
@@ -349,7 +327,7 @@ __device__ __forceinline__ void parse_tile(const ParseArgs &a, ParseSmem &sm, ui
 // tile 0 resets the document's counters, which only pass 2 adds to. Block b
 // first asks L2 to prefetch the tile kPrefetchTilesAhead further on (when this
 // launch covers it), which a block that starts soon will read.
-__global__ void __launch_bounds__(PT_THREADS, 6) parse_stage_kernel(ParseArgs a) {
+__global__ void __launch_bounds__(PT_THREADS, 8) parse_stage_kernel(ParseArgs a) {
     __shared__ ParseSmem sm;
     const uint32_t tile = a.first_tile + blockIdx.x;
     if (threadIdx.x == 0 && blockIdx.x + kPrefetchTilesAhead < gridDim.x)  // inside this launch's tiles
