@@ -2,7 +2,7 @@
 //
 // Up to eight patterns are searched in one pass over the text; CTA b owns the
 // 16 KiB tile b and stages it, plus a halo of (longest pattern - 1) bytes, in
-// shared memory with 16-byte coalesced loads (in the stage pass, after asking
+// shared memory with asynchronous 16-byte copies (in the stage pass, after asking
 // L2 to prefetch the tile kPrefetchTilesAhead further on, which a block that
 // starts soon will read). Every 16-byte piece is compared with each pattern of
 // up to 7 bytes at all sixteen starts at once (byte SWAR on the piece shifted by
@@ -132,14 +132,11 @@ __device__ __forceinline__ bool verify_start(const SearchArgs &a, const SearchSm
 __device__ __forceinline__ void load_tile(const SearchArgs &a, SearchSmem &sm, uint64_t t0) {
     const uint32_t tid = threadIdx.x;
     const bool staged = a.halo <= kSearchMaxStagedPattern;
-    uint4 v[SR_STEPS];
 #pragma unroll
-    for (uint32_t k = 0; k < SR_STEPS; k++) v[k] = ld_stream16(a.text + t0 + k * 4096 + tid * 16);
-#pragma unroll
-    for (uint32_t k = 0; k < SR_STEPS; k++) *reinterpret_cast<uint4 *>(&sm.text[k * 4096 + tid * 16]) = v[k];
+    for (uint32_t k = 0; k < SR_STEPS; k++) cp_async16(&sm.text[k * 4096 + tid * 16], a.text + t0 + k * 4096 + tid * 16);
     const uint32_t halo = staged ? a.halo : 0u;
     for (uint32_t o = tid * 16; o < halo; o += SR_THREADS * 16)
-        *reinterpret_cast<uint4 *>(&sm.text[kSearchTile + o]) = ld_stream16(a.text + t0 + kSearchTile + o);
+        cp_async16(&sm.text[kSearchTile + o], a.text + t0 + kSearchTile + o);
     // 16 bytes past the halo: zeros when staged; unstaged, the bytes right
     // after the tile (the filter looks 3 bytes ahead; the text is padded)
     if (tid == 0)
@@ -167,6 +164,7 @@ __device__ __forceinline__ void load_tile(const SearchArgs &a, SearchSmem &sm, u
         }
         if (tid < SR_THREADS / 32) sm.queued[tid] = 0;
     }
+    cp_async_wait();
 }
 
 // Adds the match at tile start `start` to a pattern's masks, 16 starts each
