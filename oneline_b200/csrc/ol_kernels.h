@@ -63,7 +63,7 @@ cudaError_t launch_scan_columns(const uint32_t *in, uint32_t *out, uint32_t *tot
 // Column stride for per-tile count columns: rows rounded up to a multiple of 4.
 inline uint32_t scan_ld(uint32_t rows) { return (rows + 3u) & ~3u; }
 cudaError_t launch_classify_lines(const uint8_t *text, uint64_t N, const uint32_t *offsets, uint32_t L, FlatNode *nodes,
-                                  uint32_t *depth32, cudaStream_t st);
+                                  uint32_t *depth32, cudaStream_t st, const uint32_t *count = nullptr);
 
 struct TreeArgs {
     const uint8_t *kinds;

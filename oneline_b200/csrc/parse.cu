@@ -482,9 +482,12 @@ __global__ void __launch_bounds__(PT_THREADS, 6) parse_redo_kernel(ParseArgs a) 
 // FlatNode of every line from the text and a complete offsets array (used for
 // GpuParser::parse(input, offsets) and to materialise nodes of a resident
 // document). One thread per line, bytes from global memory (read-only path).
+// With `count`, there are *count lines, at most L.
 __global__ void classify_lines_kernel(const uint8_t *__restrict__ text, uint64_t N, const uint32_t *__restrict__ offsets,
-                                      uint32_t L, FlatNode *__restrict__ nodes, uint32_t *__restrict__ depth32) {
+                                      uint32_t L, const uint32_t *__restrict__ count, FlatNode *__restrict__ nodes,
+                                      uint32_t *__restrict__ depth32) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (count) L = min(L, *count);
     if (i >= L) return;
     uint32_t s = offsets[i];
     uint32_t last_end = text[N - 1] == '\n' ? (uint32_t)(N - 1) : (uint32_t)N;
@@ -526,9 +529,9 @@ cudaError_t launch_parse_end(const ParseArgs &a, cudaStream_t st) {
 }
 
 cudaError_t launch_classify_lines(const uint8_t *text, uint64_t N, const uint32_t *offsets, uint32_t L, FlatNode *nodes,
-                                  uint32_t *depth32, cudaStream_t st) {
+                                  uint32_t *depth32, cudaStream_t st, const uint32_t *count) {
     if (L == 0) return cudaSuccess;
-    classify_lines_kernel<<<(L + 255) / 256, 256, 0, st>>>(text, N, offsets, L, nodes, depth32); OL_LAUNCHED();
+    classify_lines_kernel<<<(L + 255) / 256, 256, 0, st>>>(text, N, offsets, L, count, nodes, depth32); OL_LAUNCHED();
     return cudaGetLastError();
 }
 

@@ -64,6 +64,19 @@ def _check_len(n: int) -> None:
                               "(32-bit offsets)")
 
 
+def _line_guess(text) -> int:
+    """Room for the lines of `text`: a one-shot parse into it needs one call, and a
+    second one only where the lines turn out to be more. One line in 16 bytes for a
+    short text (most have fewer); else from four samples, with head room."""
+    n, w = len(text), 16 << 10  # `text`: bytes or a uint8 array
+    if n <= 64 * w:
+        return n // 16 + 64
+    text = np.frombuffer(text, np.uint8)
+    span = (n - w) // 3
+    found = sum(np.count_nonzero(text[i * span : i * span + w] == 10) for i in range(4))
+    return min(n + 1, int((found + 4) / (4 * w) * n * 1.25) + 4096)
+
+
 class _ProfileStep(ctypes.Structure):
     _fields_ = [("label", ctypes.c_char * 40), ("ns", ctypes.c_uint64)]
 
@@ -401,12 +414,15 @@ class GpuParser:
         _check_len(n)
         L = _lib.load()
         cnt = ctypes.c_uint64()
-        check(L.ol_parse_raw(self._ctx, p, n, None, None, 0, ctypes.byref(cnt)), self._ctx)
-        lines = cnt.value
-        offs = np.zeros(max(lines, 1), np.uint32)
-        nodes = np.zeros(max(lines, 1), NODE_DTYPE)
-        if lines:
-            check(L.ol_parse_raw(self._ctx, p, n, offs.ctypes.data, nodes.ctypes.data, lines, ctypes.byref(cnt)), self._ctx)
+        cap = _line_guess(keep)
+        while True:
+            offs = np.empty(cap, np.uint32)
+            nodes = np.empty(cap, NODE_DTYPE)
+            check(L.ol_parse_raw(self._ctx, p, n, offs.ctypes.data, nodes.ctypes.data, cap, ctypes.byref(cnt)), self._ctx)
+            lines = cnt.value
+            if lines <= cap:
+                break
+            cap = lines  # nothing was written
         return FlatTree(src if isinstance(src, bytes) else bytes(src), nodes[:lines], offs[:lines])
 
     def parse(self, text, line_offsets) -> FlatTree:
@@ -424,11 +440,13 @@ class GpuParser:
         _check_len(n)
         L = _lib.load()
         cnt = ctypes.c_uint64()
-        check(L.ol_scan_line_offsets(self._ctx, p, n, None, 0, ctypes.byref(cnt)), self._ctx)
-        out = np.zeros(max(cnt.value, 1), np.uint32)
-        if cnt.value:
-            check(L.ol_scan_line_offsets(self._ctx, p, n, out.ctypes.data, out.size, ctypes.byref(cnt)), self._ctx)
-        return out[: cnt.value]
+        cap = _line_guess(keep)
+        while True:
+            out = np.empty(cap, np.uint32)
+            check(L.ol_scan_line_offsets(self._ctx, p, n, out.ctypes.data, cap, ctypes.byref(cnt)), self._ctx)
+            if cnt.value <= cap:
+                return out[: cnt.value]
+            cap = cnt.value  # nothing was written
 
     # ----------------------------------------------------------------- tree
 
