@@ -109,12 +109,13 @@ constexpr uint32_t kSearchMaxPatterns = 8;  // patterns per launch
 // Per-pattern constants of a search launch, computed on the host from the
 // pattern bytes (search_add_pattern) and read by every block as kernel
 // parameters.
-struct SearchPatMeta {
+struct alignas(16) SearchPatMeta {
     uint32_t pre[4];  // bytes 0..3 (found by its rarest four bytes: r0..r0 + 3), each replicated into a word (0 past the end)
     uint32_t anc[4];  // anchor words: bytes [r, r + 4) little-endian, r = r0 + 1 .. r0 + 4
     uint32_t len;
     uint32_t r0;
     uint32_t last4;   // the last four bytes (len >= 4)
+    uint32_t pad;
 };
 constexpr uint32_t kSearchPatBytes = 512;       // pattern bytes passed as kernel parameters
 constexpr uint32_t kSearchFinishTiles = 256;    // texts up to this size are finished in one launch

@@ -68,21 +68,22 @@ __host__ __device__ __forceinline__ uint32_t anchor_hash(uint32_t w) {
     return (w * 0x9E3779B1u) >> (32 - kAnchorBits);
 }
 
-struct alignas(16) PatMeta {
+struct alignas(16) PatMeta {  // a SearchPatMeta, copied from the kernel parameters 16 bytes a lane
     uint4 pre;  // bytes 0..3 of the pattern (window patterns: r0..r0 + 3), each replicated into a word (unused ones 0)
     uint4 anc;  // anchor words r = r0 + 1 .. r0 + 4
-    const uint8_t *ptr;
     uint32_t len;
     uint32_t r0;
     uint32_t last4;  // the last four bytes (len >= 4)
+    uint32_t pad;
 };
+static_assert(sizeof(PatMeta) == 48 && sizeof(SearchPatMeta) == 48, "copied as three 16-byte pieces");
 
 struct SearchSmem {
     alignas(16) uint8_t text[kSearchTile + kSearchMaxStagedPattern + 16];  // stage pass: output staging after use
     uint32_t anchor_map[(1u << kAnchorBits) / 32];
     uint32_t queue[SR_THREADS / 32][SR_QCAP];  // (pattern << 16) | start, per warp
-    uint32_t queued[SR_THREADS / 32];
     PatMeta pat[kSearchMaxPatterns];
+    const uint8_t *ptr[kSearchMaxPatterns];
     uint32_t count[kSearchMaxPatterns];
     uint32_t active;  // stage pass: patterns with matches in this tile (bit mask)
 };
@@ -115,20 +116,23 @@ __device__ __forceinline__ void keep_valid_starts(uint64_t N, uint32_t m, uint64
 // Whether pattern pm (at least eight bytes) occurs at tile start s: its last
 // four bytes first (patterns that begin with a run match a long way into
 // another run), then four at a time.
-__device__ __forceinline__ bool verify_start(const SearchArgs &a, const SearchSmem &sm, const PatMeta &pm, uint32_t s,
+__device__ __forceinline__ bool verify_start(const SearchArgs &a, const SearchSmem &sm, uint32_t p, uint32_t s,
                                              bool staged, uint64_t t0) {
+    const PatMeta &pm = sm.pat[p];
     const uint32_t m = pm.len;
     if (t0 + s + m > a.text_len) return false;
     if (text4(a, sm, s + m - 4, staged, t0) != pm.last4) return false;
-    const uint32_t *pw = reinterpret_cast<const uint32_t *>(pm.ptr);  // 16-byte aligned
+    const uint32_t *pw = reinterpret_cast<const uint32_t *>(sm.ptr[p]);  // 16-byte aligned
     for (uint32_t j = 0; j + 4 < m; j += 4)
         if (text4(a, sm, s + j, staged, t0) != pw[j >> 2]) return false;
     return true;
 }
 
-// Loads tile b (plus the halo) into shared memory, and (warp 0) the pattern
-// table and the anchor map from the kernel parameters; the caller's
-// __syncthreads publishes them.
+// Loads tile b (plus the halo) into shared memory, and from the kernel
+// parameters the anchor map (warp 0), the pattern table (warp 1) and the pattern
+// pointers (warp 2): one warp with all three, eight lanes each copying a table
+// entry word by word, kept the block waiting (256 MiB, 8 patterns: 119.8 against
+// 116.5 us). The caller's __syncthreads publishes them.
 __device__ __forceinline__ void load_tile(const SearchArgs &a, SearchSmem &sm, uint64_t t0) {
     const uint32_t tid = threadIdx.x;
     const bool staged = a.halo <= kSearchMaxStagedPattern;
@@ -150,19 +154,15 @@ __device__ __forceinline__ void load_tile(const SearchArgs &a, SearchSmem &sm, u
             const uint32_t h = a.anchor_hash[tid];
             atomicOr(&sm.anchor_map[h >> 5], 1u << (h & 31));
         }
-        if (tid < a.np) {
-            const SearchPatMeta &m = a.meta[tid];
-            PatMeta pm;
-            pm.ptr = a.pat[tid] ? a.pat[tid] : a.pat_bytes + a.pat_at[tid];
-            pm.len = m.len;
-            pm.r0 = m.r0;
-            pm.last4 = m.last4;
-            pm.pre = make_uint4(m.pre[0], m.pre[1], m.pre[2], m.pre[3]);
-            pm.anc = make_uint4(m.anc[0], m.anc[1], m.anc[2], m.anc[3]);
-            sm.pat[tid] = pm;
-            sm.count[tid] = 0;
+    } else if (tid < 64) {
+        const uint32_t i = tid - 32;
+        if (i < a.np * 3) reinterpret_cast<uint4 *>(sm.pat)[i] = reinterpret_cast<const uint4 *>(a.meta)[i];
+    } else if (tid < 96) {
+        const uint32_t i = tid - 64;
+        if (i < a.np) {
+            sm.ptr[i] = a.pat[i] ? a.pat[i] : a.pat_bytes + a.pat_at[i];
+            sm.count[i] = 0;
         }
-        if (tid < SR_THREADS / 32) sm.queued[tid] = 0;
     }
     cp_async_wait();
 }
@@ -283,14 +283,13 @@ __device__ __forceinline__ uint32_t filter_tile(const SearchArgs &a, SearchSmem 
     const bool staged = a.halo <= kSearchMaxStagedPattern;
     uint32_t found = 0;
     uint32_t *queue = sm.queue[warp];
-    // Verifies the queued starts when there are at least `least`.
-    auto drain = [&](uint32_t least) {
+    uint32_t queued = 0;  // the same in all lanes
+    // Verifies the queued starts.
+    auto drain = [&]() {
         __syncwarp();
-        const uint32_t n = sm.queued[warp];
-        if (n < least) return;  // uniform
-        for (uint32_t i = lane; i < n; i += 32) {
+        for (uint32_t i = lane; i < queued; i += 32) {
             const uint32_t e = queue[i], p = e >> 16, start = e & 0xFFFFu;
-            if (!verify_start(a, sm, sm.pat[p], start, staged, t0)) continue;
+            if (!verify_start(a, sm, p, start, staged, t0)) continue;
             found |= 1u << p;
             if (COUNT)
                 atomicAdd(&sm.count[p], 1u);
@@ -298,30 +297,49 @@ __device__ __forceinline__ uint32_t filter_tile(const SearchArgs &a, SearchSmem 
                 set_match(match[p], start);
         }
         __syncwarp();
-        if (lane == 0) sm.queued[warp] = 0;
-        __syncwarp();
+        queued = 0;
     };
-    // Queues pattern p's starts first + bit, for the set bits of each lane's g,
-    // that lie in the tile.
+    // Queues each lane's (p, start) if `ok` and the start lies in the tile (one before it has wrapped).
+    auto queue_start = [&](uint32_t p, uint32_t start, bool ok) {
+        ok = ok && start < kSearchTile;
+        const uint32_t who = __ballot_sync(0xFFFFFFFFu, ok);
+        if (ok) queue[queued + __popc(who & ((1u << lane) - 1u))] = (p << 16) | start;
+        queued += __popc(who);
+        if (queued > SR_QCAP - 32) drain();
+    };
+    // Queues pattern p's starts first + bit, for the set bits of each lane's g.
     auto queue_starts = [&](uint32_t p, uint32_t g, uint32_t first) {
         while (__any_sync(0xFFFFFFFFu, g != 0)) {
-            const uint32_t start = first + __ffs(g) - 1;
-            if (g && start < kSearchTile)  // (before the tile: wrapped)
-                queue[atomicAdd(&sm.queued[warp], 1u)] = (p << 16) | start;
+            queue_start(p, first + __ffs(g) - 1, g != 0);
             g &= g - 1;
-            drain(SR_QCAP - 31);
         }
     };
-    // Words in the map, each against every pattern's anchors: those of the lane's
+    // Words in the map, against every pattern's anchors: those of the lane's
     // pieces, then (a round more) of the words past the tile, of starts in it.
+    // Most often one lane or two have one; then the warp takes a word at a time
+    // and each lane compares it with one anchor. Only where more lanes have one
+    // than there are patterns does each lane take its own through all patterns
+    // (always so: 116 us for 256 MiB and 8 patterns, 106 for 100 MB of nested text
+    // with longer ones; now 103 and 88).
     if (anchored) {
+        const uint32_t anchor = reinterpret_cast<const uint32_t *>(&sm.pat[lane >> 2].anc)[lane & 3];
+        const uint32_t anchor_r = sm.pat[lane >> 2].r0 + 1 + (lane & 3);
+        const bool mine = (anchored >> (lane >> 2)) & 1u;
 #pragma unroll 1
         for (uint32_t past = 0; past < 2; past++) {
             if (past) {
                 if ((tid & ~31u) >= a.anchor_words) break;  // whole warps
                 flagged = tid < a.anchor_words && in_map(*reinterpret_cast<const uint32_t *>(&sm.text[kSearchTile + tid * 4]));
             }
-            while (__any_sync(0xFFFFFFFFu, flagged != 0)) {
+            while (const uint32_t with = __ballot_sync(0xFFFFFFFFu, flagged != 0)) {
+                if (__popc(with) <= __popc(anchored)) {  // one word, lane 4p + i for anchor i of pattern p
+                    const uint32_t from = __ffs(with) - 1, b = __ffs(__shfl_sync(0xFFFFFFFFu, flagged, from)) - 1;
+                    const uint32_t t = (tid & ~31u) + from;
+                    const uint32_t at = past ? kSearchTile + t * 4 : ((b >> 2) * SR_THREADS + t) * 16 + (b & 3) * 4;
+                    queue_start(lane >> 2, at - anchor_r, *reinterpret_cast<const uint32_t *>(&sm.text[at]) == anchor && mine);
+                    if (lane == from) flagged &= flagged - 1;
+                    continue;
+                }
                 const uint32_t b = __ffs(flagged) - 1;  // (NONE without one)
                 const uint32_t at = !flagged ? 0u : past ? kSearchTile + tid * 4 : ((b >> 2) * SR_THREADS + tid) * 16 + (b & 3) * 4;
                 const uint32_t x = *reinterpret_cast<const uint32_t *>(&sm.text[at]);
@@ -368,7 +386,7 @@ __device__ __forceinline__ uint32_t filter_tile(const SearchArgs &a, SearchSmem 
             queue_starts(p, g, piece * 16 - r0);
         }
     }
-    drain(1);
+    if (queued) drain();
     return found;
 }
 
