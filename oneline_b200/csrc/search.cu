@@ -492,6 +492,21 @@ __global__ void __launch_bounds__(SR_THREADS) search_write_kernel(const __grid_c
 // copies them to their final slots. A tile with more hits than its staging slot
 // holds is flagged and left to search_write_kernel, which recomputes it.
 
+// Lists the starts at + bit of the set bits, ascending, from both ends at once:
+// half the rounds of the lane that has most (256 MiB with 28 M hits of "||||":
+// 181 us one at a time, 159 so; run by run 158, all 64 positions of a lane in one
+// loop 174).
+__device__ __forceinline__ void list_starts(uint16_t *out, uint32_t bits, uint32_t at) {
+    uint16_t *end = out + __popc(bits);
+    while (bits) {
+        const uint32_t lo = __ffs(bits) - 1, hi = 31 - __clz(bits);
+        *out++ = (uint16_t)(at + lo);
+        *--end = (uint16_t)(at + hi);
+        bits &= bits - 1;
+        bits &= ~(1u << hi);
+    }
+}
+
 template <uint32_t NP>
 __global__ void __launch_bounds__(SR_THREADS, 5) search_stage_kernel(const __grid_constant__ SearchArgs a) {
     constexpr uint32_t NQ = (NP + 1) / 2;  // packed count words, two patterns each
@@ -554,12 +569,8 @@ __global__ void __launch_bounds__(SR_THREADS, 5) search_stage_kernel(const __gri
         const uint32_t mm[2] = {m.x, m.y};
 #pragma unroll
         for (uint32_t h = 0; h < 2; h++) {
-            uint32_t bits = mm[h];
-            while (bits) {
-                const uint32_t b = __ffs(bits) - 1;
-                bits &= bits - 1;
-                stage[r++] = (uint16_t)((4 * tid + 2 * h + (b >> 4)) * 16 + (b & 15));
-            }
+            list_starts(stage + r, mm[h], 64 * tid + 32 * h);
+            r += __popc(mm[h]);
         }
         __syncthreads();
         uint4 *dst = reinterpret_cast<uint4 *>(a.stage + (size_t)tile * a.stage_cap);
@@ -619,12 +630,8 @@ __global__ void __launch_bounds__(SR_THREADS, 5) search_stage_kernel(const __gri
             const uint32_t mm[2] = {m4[p].x, m4[p].y};
 #pragma unroll
             for (uint32_t h = 0; h < 2; h++) {
-                uint32_t bits = mm[h];
-                while (bits) {
-                    const uint32_t b = __ffs(bits) - 1;
-                    bits &= bits - 1;
-                    stage[r++] = (uint16_t)((4 * tid + 2 * h + (b >> 4)) * 16 + (b & 15));
-                }
+                list_starts(stage + r, mm[h], 64 * tid + 32 * h);
+                r += __popc(mm[h]);
             }
         }
         if (tid == 0) a.counts[(size_t)p * a.ld + tile] = tot;
