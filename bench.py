@@ -533,7 +533,7 @@ def run_ours(args, world, rank, local):
     peak, peak_kind = hbm_peak()
     hits = sum(totals)
     # algorithmic bytes: text read once per launch + every output byte once
-    groups = {"parse pass (newline_count, scan, parse_tiles, fixup)": (t_parse, N + 6 * lines),
+    groups = {"parse pass (parse_stage, scan, parse_copy, parse_redo)": (t_parse, N + 6 * lines),
               "tree pass (summary, scan, resolve)": (t_tree, 2 * lines + 16 * lines),
               "8-pattern search pass (search_stage, scan, search_copy, search_write)": (t_search, N + 4 * hits)}
     dom = max(groups, key=lambda k: groups[k][0])

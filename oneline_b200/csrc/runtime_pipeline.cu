@@ -1,5 +1,5 @@
 // The parse-then-search pipeline of a resident document as one CUDA graph:
-// re-parse (newline count, column scan, tile parse, fix-up), tree links and a
+// re-parse (stage and finish, or scan, copy and redo passes), tree links and a
 // multi-pattern search, captured once and replayed with a single launch. The
 // graph has two branches: the parse and the tree on one private context's
 // stream, the search (which reads only the text) on a second one, so the
