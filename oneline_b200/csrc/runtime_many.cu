@@ -433,15 +433,31 @@ ol_status ol::many_run(ol_ctx *ctx, const ol_doc *d, const ol_patset *set, uint6
     if (e == cudaSuccess) e = launch_dict_plan(pa, st);
     uint32_t H = kDictMaxHeavy;
     uint64_t cap = std::max<uint64_t>(N / 16, 65536);
-    if (e == cudaSuccess && n_tiles > kPlanTiles) {
-        e = read_meta();
+    auto read_plan = [&]() -> ol_status {  // as many heavy patterns and light hits as the sample promises
+        cudaError_t r = read_meta();
         prof_mark(ctx, "dictionary: wait for the sample");
-        if (e != cudaSuccess) return ctx_cuda(ctx, e, "search_many sample");
+        if (r != cudaSuccess) return ctx_cuda(ctx, r, "search_many sample");
         if (hm->error & OL_DEVERR_TIMEOUT) return ctx_fail(ctx, OL_ERR_TIMEOUT, "search_many: a bounded wait ran out");
         H = hm->plan.n_heavy;
         cap = std::min<uint64_t>(0xFFFFFFF0ull, (uint64_t)((double)hm->plan.light_sample * scale * 1.25) + 65536);
+        return OL_OK;
+    };
+    auto reserve_hits = [&]() -> cudaError_t {  // the bitmaps and the first attempt's keys
+        cudaError_t r = H ? ctx->dict_bitmap.reserve((size_t)H * n_words * 4, st) : cudaSuccess;
+        return r == cudaSuccess ? ctx->dict_keys.reserve((size_t)cap * 16, st) : r;
+    };
+    ol_status ps = OL_OK;
+    if (e == cudaSuccess && n_tiles > kPlanTiles) ps = read_plan();
+    if (ps != OL_OK) return ps;
+    if (e == cudaSuccess) e = reserve_hits();
+    if (e == cudaErrorMemoryAllocation && n_tiles <= kPlanTiles) {
+        // no memory for all there can be (at most 5 bytes a text byte): what the sample promises may fit
+        cudaGetLastError();
+        ctx->dict_bitmap.release(st);
+        ctx->dict_keys.release(st);
+        if ((ps = read_plan()) != OL_OK) return ps;
+        e = reserve_hits();
     }
-    if (e == cudaSuccess && H) e = ctx->dict_bitmap.reserve((size_t)H * n_words * 4, st);
     if (e != cudaSuccess) return ctx_cuda(ctx, e, "search_many");
 
     // 2. The match pass; 3. heavy ranks, light order, per-id slots; 4. hits.
