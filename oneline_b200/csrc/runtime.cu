@@ -62,8 +62,10 @@ void DevBuf::release(cudaStream_t st) {
 
 cudaError_t HostBuf::reserve(size_t need) {
     if (need <= bytes) return cudaSuccess;
+    // at least twice as much each time: callers ask for the size of an answer, and a
+    // page-lock and unlock cost more than the copies through it save
+    need = std::max({need, 2 * bytes, (size_t)64 << 10});
     release();
-    need = std::max<size_t>(need, 4096);
     cudaError_t e = cudaMallocHost((void **)&ptr, need);
     if (e != cudaSuccess) {
         ptr = nullptr;

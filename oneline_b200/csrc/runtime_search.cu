@@ -187,8 +187,8 @@ ol_status search_multi_host(ol_ctx *ctx, const ol_doc *d, const uint8_t *const *
             totals[idx[c + j]] = tot_h[j];
             found += std::min(tot_h[j], m2[c + j]) * (size_t)4;
         }
-        const bool staged = found <= kStagedResult;
-        if (staged && (e = ctx->host_words.reserve(found)) != cudaSuccess) return ctx_cuda(ctx, e, "search download");
+        const bool staged = found <= kStagedResult && ctx->host_words.reserve(found) == cudaSuccess;
+        if (!staged) cudaGetLastError();  // (nothing page-locked left for it)
         {
             GpuPass pass(ctx, "download");
             size_t at = 0;
