@@ -364,10 +364,8 @@ ol_status alloc_lines(ol_ctx *ctx, ol_doc *d, uint64_t cap_lines) {
 }
 
 // Runs the parse (when the estimate was too low, the line arrays are written
-// once more at the exact size),
-// waits, and records the line count. With nodes_out, the 16-byte nodes are
-// materialised into ctx->scratch_c as well.
-ol_status parse_doc(ol_ctx *ctx, ol_doc *d, uint64_t est_lines, FlatNode **nodes_out, const uint8_t *host_text) {
+// once more at the exact size), waits, and records the line count.
+ol_status parse_doc(ol_ctx *ctx, ol_doc *d, uint64_t est_lines, const uint8_t *host_text) {
     cudaStream_t st = ctx->stream;
     for (int attempt = 0; attempt < 2; attempt++) {
         ol_status s = alloc_lines(ctx, d, est_lines);
@@ -387,14 +385,6 @@ ol_status parse_doc(ol_ctx *ctx, ol_doc *d, uint64_t est_lines, FlatNode **nodes
         }
         d->line_count = hs.line_count;
         d->max_depth = hs.max_content_depth;
-        if (nodes_out) {
-            e = ctx->scratch_c.reserve((size_t)d->line_cap * sizeof(FlatNode), st);
-            if (e == cudaSuccess)
-                e = launch_classify_lines(d->text, d->text_len, d->offsets, d->line_count, (FlatNode *)ctx->scratch_c.ptr,
-                                          nullptr, st);
-            if (e != cudaSuccess) return ctx_cuda(ctx, e, "materialise nodes");
-            *nodes_out = (FlatNode *)ctx->scratch_c.ptr;
-        }
         return OL_OK;
     }
     return ctx_fail(ctx, OL_ERR_CUDA, "parse: line capacity retry failed");
@@ -454,7 +444,7 @@ static ol_status upload_common(ol_ctx *ctx, const uint8_t *text, uint64_t len, b
         ol_doc_free(d);
         return ctx_cuda(ctx, e, "upload");
     }
-    s = parse_doc(ctx, d, est, nullptr, device_src ? nullptr : text);
+    s = parse_doc(ctx, d, est, device_src ? nullptr : text);
     prof_mark(ctx, "upload: wait for parse");
     if (s != OL_OK) {
         ol_doc_free(d);
@@ -565,7 +555,9 @@ static ol_status parse_short(ol_ctx *ctx, const uint8_t *text, uint64_t len, uin
                              uint64_t cap, uint64_t *line_count, bool *done) {
     *done = false;
     cudaStream_t st = ctx->stream;
-    const uint32_t room = (uint32_t)((estimate_lines(text, len) + 63) / 64 * 64);
+    const uint64_t est = estimate_lines(text, len);  // the lines, or one more
+    if (est - 1 > cap) offsets = nullptr, nodes = nullptr;  // the caller's room is too small
+    const uint32_t room = (uint32_t)((est + 63) / 64 * 64);
     const size_t o_stats = (text_alloc_bytes(len) + 255) / 256 * 256, o_offs = o_stats + 256;
     const size_t o_nodes = o_offs + (size_t)room * 4, o_kinds = o_nodes + (size_t)room * sizeof(FlatNode);
     const size_t o_depth = o_kinds + room, total = o_depth + room;
@@ -629,14 +621,18 @@ extern "C" ol_status ol_parse_raw(ol_ctx *ctx, const uint8_t *text, uint64_t len
         if (s != OL_OK) return s;
         if (len > 0) {
             cudaError_t e = cudaSuccess;
-            FlatNode *dn = nullptr;
-            s = parse_doc(ctx, d, estimate_lines(text, len), nodes ? &dn : nullptr, text);  // upload overlapped
+            s = parse_doc(ctx, d, estimate_lines(text, len), text);  // upload overlapped
             *line_count = d->line_count;
             if (s == OL_OK && d->line_count <= cap && d->line_count > 0) {
                 cudaStream_t st = ctx->stream;
-                if (offsets) e = cudaMemcpyAsync(offsets, d->offsets, (size_t)d->line_count * 4, cudaMemcpyDeviceToHost, st);
+                const size_t node_bytes = (size_t)d->line_count * sizeof(FlatNode);
+                if (nodes) e = ctx->scratch_c.reserve(node_bytes, st);
+                FlatNode *dn = (FlatNode *)ctx->scratch_c.ptr;
                 if (e == cudaSuccess && nodes)
-                    e = cudaMemcpyAsync(nodes, dn, (size_t)d->line_count * sizeof(FlatNode), cudaMemcpyDeviceToHost, st);
+                    e = launch_classify_lines(d->text, len, d->offsets, d->line_count, dn, nullptr, st);
+                if (e == cudaSuccess && offsets)
+                    e = cudaMemcpyAsync(offsets, d->offsets, (size_t)d->line_count * 4, cudaMemcpyDeviceToHost, st);
+                if (e == cudaSuccess && nodes) e = cudaMemcpyAsync(nodes, dn, node_bytes, cudaMemcpyDeviceToHost, st);
                 if (e == cudaSuccess) e = cudaStreamSynchronize(st);
                 if (e != cudaSuccess) s = ctx_cuda(ctx, e, "download");
             }

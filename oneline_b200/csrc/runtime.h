@@ -132,8 +132,7 @@ ol_status new_doc(ol_ctx *ctx, uint64_t len, ol_doc **out);
 // Parses doc's text and waits (one retry with the exact line count when the
 // estimate was low). With host_text, the text is uploaded first, overlapped
 // with the parse.
-ol_status parse_doc(ol_ctx *ctx, ol_doc *d, uint64_t est_lines, FlatNode **nodes_out,
-                    const uint8_t *host_text = nullptr);
+ol_status parse_doc(ol_ctx *ctx, ol_doc *d, uint64_t est_lines, const uint8_t *host_text = nullptr);
 cudaError_t enqueue_parse(ol_ctx *ctx, ol_doc *d);
 // Copies host bytes to device memory on the context stream (pinned: one DMA;
 // pageable: through the pinned staging ring).
