@@ -289,7 +289,7 @@ __device__ __forceinline__ void dict_walk(const DictMatchArgs &a, DictWarp<SLICE
         const uint32_t back = hi != 0xFFFFFFFFu ? __clz(~hi) : 32 + __clz(~lo);  // (__clz(0) = 32)
         e = p + 3;
         t = 1;
-        r0 = e > SLICE + 2 ? e - SLICE + 1 : 3u;
+        r0 = e > SLICE + 2 ? e - SLICE + 1 : 3u;  // at most 63: see the candidates past the slice
         starts = (~0ull >> (kDictMaxLen - 1 - min(3 + back, kDictMaxLen - 1))) & (~0ull << r0);
         v = __ldg(a.set.dense + (size_t)a.set.run_root[j] * 256 + (key >> 24));
     } else {
@@ -492,7 +492,8 @@ __global__ void __launch_bounds__(DM_THREADS, 2) dict_match_kernel(const __grid_
         for (uint32_t j = 0; j < n_runs; j++) {
             if (!(w.run[j][Warp::kWords + 1] >> 31)) continue;  // uniform, and so is what follows
             const uint32_t f = dict_run_from(w, j, SLICE);
-            if (f >= 3 && f < kDictMaxLen) tail = SLICE + f - 3;  // of one run byte at most
+            // (f = 63: a start in the slice would need a pattern of 64 run bytes and a rest)
+            if (f >= 3 && f + 1 < kDictMaxLen) tail = SLICE + f - 3;  // of one run byte at most
         }
         for (uint32_t qn = 0, at = 0, last = 0; !last;) {
             while (qn < 32 && !last) {  // each lane's lowest candidate, until the queue holds a full round
