@@ -117,7 +117,9 @@ struct alignas(16) SearchPatMeta {
     uint32_t last4;   // the last four bytes (len >= 4)
     uint32_t pad;
 };
-constexpr uint32_t kSearchPatBytes = 512;       // pattern bytes passed as kernel parameters
+constexpr uint32_t kSearchInlinePattern = 64;   // patterns of up to this length travel in a launch's parameters
+constexpr uint32_t kSearchPatBytes = kSearchInlinePattern * kSearchMaxPatterns;  // room for as many as a launch takes
+static_assert(kSearchInlinePattern % 16 == 0, "each pattern's bytes begin on a 16-byte boundary");
 constexpr uint32_t kSearchFinishTiles = 256;    // texts up to this size are finished in one launch
 
 struct SearchArgs {
@@ -156,10 +158,9 @@ struct SearchArgs {
 };
 constexpr uint32_t kSearchStageCap = 8192;  // staged hits per tile (all patterns of a launch)
 
-// Appends a pattern to a launch (slot a.np): its device copy (nullptr: its
-// bytes go into the launch's parameters, which search_takes_pattern_bytes tells
-// have room), and the constants the kernels take from its host bytes.
-bool search_takes_pattern_bytes(const SearchArgs &a, uint32_t len);
+// Appends a pattern to a launch (slot a.np): its device copy (nullptr: at most
+// kSearchInlinePattern bytes, which go into the launch's parameters), and the
+// constants the kernels take from its host bytes.
 void search_add_pattern(SearchArgs &a, const uint8_t *host, const uint8_t *dev, uint32_t len, uint32_t *out,
                         uint32_t max_out);
 cudaError_t launch_search(const SearchArgs &a, cudaStream_t st);

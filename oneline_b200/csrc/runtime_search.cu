@@ -17,10 +17,6 @@ static uint32_t halo_for(uint32_t m) { return ((m > 0 ? m - 1 : 0) + 15u) & ~15u
 
 namespace {
 
-// Patterns of up to this length travel in the launch's parameters (eight of
-// them fit), longer ones through device memory.
-constexpr uint32_t kInlinePattern = kSearchPatBytes / kSearchMaxPatterns;
-
 // Enqueues searches of n patterns over doc, at most 8 per launch (longer than
 // the staged limit: one per launch). Results stay on the device: d_totals[i]
 // and d_outs[i]. The bytes of long patterns are copied to device memory first.
@@ -30,7 +26,7 @@ cudaError_t enqueue_multi(ol_ctx *ctx, const ol_doc *d, const uint8_t *const *pa
     uint32_t n_tiles = (uint32_t)((d->text_len + kSearchTile - 1) / kSearchTile);
     size_t total_bytes = 0;
     for (uint32_t i = 0; i < n; i++)
-        if (lens[i] > kInlinePattern) total_bytes += (lens[i] + 15) & ~15u;
+        if (lens[i] > kSearchInlinePattern) total_bytes += (lens[i] + 15) & ~15u;
     cudaError_t e = ctx->scratch_a.reserve((size_t)scan_ld(n_tiles) * kSearchMaxPatterns * 4 * 2, st);
     std::vector<const uint8_t *> dp(n, nullptr);
     if (e == cudaSuccess && total_bytes == 0) return ol::launch_multi(ctx, d, pats, dp.data(), lens, n, max_out, d_totals, d_outs);
@@ -54,7 +50,7 @@ cudaError_t enqueue_multi(ol_ctx *ctx, const ol_doc *d, const uint8_t *const *pa
     std::vector<size_t> at(n);
     size_t w = 0;
     for (uint32_t i = 0; i < n; i++) {
-        if (lens[i] <= kInlinePattern) continue;
+        if (lens[i] <= kSearchInlinePattern) continue;
         at[i] = w;
         memcpy(ctx->pat_host + w, pats[i], lens[i]);
         w += (lens[i] + 15) & ~15u;
@@ -63,14 +59,14 @@ cudaError_t enqueue_multi(ol_ctx *ctx, const ol_doc *d, const uint8_t *const *pa
     if ((e = cudaMemcpyAsync(dpat, ctx->pat_host, w, cudaMemcpyHostToDevice, st)) != cudaSuccess) return e;
     if ((e = cudaEventRecord(ctx->pat_done, st)) != cudaSuccess) return e;
     for (uint32_t i = 0; i < n; i++)
-        if (lens[i] > kInlinePattern) dp[i] = dpat + at[i];
+        if (lens[i] > kSearchInlinePattern) dp[i] = dpat + at[i];
     return ol::launch_multi(ctx, d, pats, dp.data(), lens, n, max_out, d_totals, d_outs);
 }
 
 }  // namespace
 
 // Launches the searches of n patterns (hpats[i]; those longer than
-// kInlinePattern also in device memory, dpats[i]) over doc, at most 8 per launch
+// kSearchInlinePattern also in device memory, dpats[i]) over doc, at most 8 per launch
 // (longer than the staged limit: one per launch). Only stream operations: a CUDA
 // graph can capture it once the context's scratch is large enough.
 cudaError_t ol::launch_multi(ol_ctx *ctx, const ol_doc *d, const uint8_t *const *hpats, const uint8_t *const *dpats,
@@ -108,7 +104,7 @@ cudaError_t ol::launch_multi(ol_ctx *ctx, const ol_doc *d, const uint8_t *const 
         while (i < n && a.np < kSearchMaxPatterns) {
             bool long_pat = halo_for(lens[i]) > kSearchMaxStagedPattern;
             if (a.np > 0 && (alone || long_pat)) break;
-            search_add_pattern(a, hpats[i], lens[i] <= kInlinePattern ? nullptr : dpats[i], lens[i], d_outs[i], max_out[i]);
+            search_add_pattern(a, hpats[i], lens[i] <= kSearchInlinePattern ? nullptr : dpats[i], lens[i], d_outs[i], max_out[i]);
             halo = std::max(halo, halo_for(lens[i]));
             i++;
             if (alone) break;

@@ -784,10 +784,6 @@ static uint32_t rarest_place(const uint8_t *pat, uint32_t len, uint32_t first, u
     return best;
 }
 
-bool search_takes_pattern_bytes(const SearchArgs &a, uint32_t len) {
-    return a.n_pat_bytes + ((len + 15) & ~15u) <= kSearchPatBytes;
-}
-
 void search_add_pattern(SearchArgs &a, const uint8_t *host, const uint8_t *dev, uint32_t len, uint32_t *out,
                         uint32_t max_out) {
     const uint32_t p = a.np++;
