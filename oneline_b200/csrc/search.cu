@@ -62,7 +62,7 @@ constexpr uint32_t kAnchorMin = 8;
 constexpr uint32_t kAnchorBits = 15;
 constexpr uint32_t kAnchorReach = 240;  // largest r0 (or window offset): at most 16 pieces past the tile
 constexpr uint32_t kPoorAnchor = 20;    // anchor_place: a word of this weight is mostly one byte repeated
-constexpr uint32_t kRunMask = 48;       // runs of up to this length are decided from the masks
+constexpr uint32_t kRunMask = 48;       // runs of up to this length are decided from the masks of four pieces
 
 __host__ __device__ __forceinline__ uint32_t anchor_hash(uint32_t w) {
     return (w * 0x9E3779B1u) >> (32 - kAnchorBits);
@@ -173,14 +173,16 @@ __device__ __forceinline__ void set_match(uint16_t *masks, uint32_t start) {
     atomicOr(reinterpret_cast<uint32_t *>(masks) + (start >> 5), 1u << (start & 31));
 }
 
-// The starts of run pattern p (one byte m times) in a lane's piece v: the mask
-// of the sixteen; for runs longer than the masks decide, of the candidates.
+// The starts of run pattern p (one byte m times) in a lane's piece: the mask of
+// the sixteen, from e, the piece's mask of the byte. Longer runs than the masks
+// of four pieces show: their candidates are next to each other and in one run,
+// whose end is looked for once for all of them, sixteen bytes at a time.
 __device__ __forceinline__ uint32_t run_starts(const SearchArgs &a, const SearchSmem &sm, uint32_t p, uint32_t e, uint32_t piece,
                                             uint64_t t0) {
-    const uint32_t lane = threadIdx.x & 31, m = sm.pat[p].len;
+    const uint32_t lane = threadIdx.x & 31, m = sm.pat[p].len, c = sm.pat[p].pre.x;
     // the masks of the three pieces after mine (lanes 0..2 have those after the warp's)
     uint32_t more = 0;
-    if (lane < 3) more = eq_mask16(*reinterpret_cast<const uint4 *>(&sm.text[(piece + 32) * 16]), sm.pat[p].pre.x);
+    if (lane < 3) more = eq_mask16(*reinterpret_cast<const uint4 *>(&sm.text[(piece + 32) * 16]), c);
     unsigned long long x = e;
 #pragma unroll
     for (uint32_t j = 1; j < 4; j++) {
@@ -192,8 +194,26 @@ __device__ __forceinline__ uint32_t run_starts(const SearchArgs &a, const Search
     uint32_t have = 1;
     for (; have * 2 <= n; have *= 2) x &= x >> have;
     x &= x >> (n - have);
+    uint32_t g = (uint32_t)x & 0xFFFFu;
+    if (m > kRunMask && g) {
+        // where the run ends, from the piece on, as far as it matters to the sixteen
+        const uint32_t last = 31 - __clz(g);
+        uint32_t end = last + kRunMask;
+        if (last == 15) {
+            const uint32_t far = m + 15;
+            for (end = kRunMask; end < far; end += 16) {
+                const uint32_t ne = 0xFFFFu ^ eq_mask16(*reinterpret_cast<const uint4 *>(&sm.text[piece * 16 + end]), c);
+                if (ne) {
+                    end += __ffs(ne) - 1;
+                    break;
+                }
+            }
+        }
+        const uint32_t ok = end < m ? 0u : end - m + 1;  // starts that the run has room for
+        g &= ok >= 16 ? 0xFFFFu : (1u << ok) - 1u;
+    }
     const int64_t room = (int64_t)a.text_len - m - (int64_t)t0 - piece * 16 + 1;  // valid starts from the piece's
-    return (uint32_t)x & (room <= 0 ? 0u : room >= 16 ? 0xFFFFu : (1u << room) - 1u);
+    return g & (room <= 0 ? 0u : room >= 16 ? 0xFFFFu : (1u << room) - 1u);
 }
 
 // Finds every start of the patterns in `mask` in the tile (staged in shared
@@ -366,15 +386,17 @@ __device__ __forceinline__ uint32_t filter_tile(const SearchArgs &a, SearchSmem 
         for (uint32_t base = tid & ~31u; base < n; base += SR_THREADS) {  // whole warps
             const uint32_t piece = base + lane;
             const uint4 v = *reinterpret_cast<const uint4 *>(&sm.text[piece * 16]);  // (past the pieces: not used)
+            if (run) {  // of eight and more: it holds an aligned word of the byte, in the piece or right after it
+                bool word = v.x == pre.x || v.y == pre.x || v.z == pre.x || v.w == pre.x;
+                if (lane == 31) word |= *reinterpret_cast<const uint32_t *>(&sm.text[(piece + 1) * 16]) == pre.x;
+                if (!__any_sync(0xFFFFFFFFu, word)) continue;
+                const uint32_t r = run_starts(a, sm, p, eq_mask16(v, pre.x), piece, t0);
+                if (r) pieces(p, piece, r);
+                continue;
+            }
             uint32_t g = eq_mask16(v, pre.x);
             if (!__any_sync(0xFFFFFFFFu, g != 0)) continue;
-            if (run) {
-                g = run_starts(a, sm, p, g, piece, t0);
-                if (sm.pat[p].len <= kRunMask) {  // uniform
-                    if (g) pieces(p, piece, g);
-                    continue;
-                }
-            } else if (g) {  // the window's first byte: its four bytes
+            if (g) {  // the window's first byte: its four bytes
                 const uint32_t want = (pre.x & 0xFFu) | (pre.y & 0xFF00u) | (pre.z & 0xFF0000u) | (pre.w & 0xFF000000u);
                 uint32_t ok = 0;
                 for (; g; g &= g - 1) {
@@ -808,16 +830,19 @@ void search_add_pattern(SearchArgs &a, const uint8_t *host, const uint8_t *dev, 
         memcpy(a.pat_bytes + a.n_pat_bytes, host, len);
         a.n_pat_bytes += (len + 15) & ~15u;
     }
+    // A run of one byte, however rare the byte: its four anchor words are the same,
+    // and in text that is such a run every word has four candidates (64 MiB of "Z",
+    // eight of them looked for: 340 us by anchors, 71 by masks).
+    if (len <= kSearchMaxStagedPattern && std::all_of(host, host + len, [&](uint8_t c) { return c == host[0]; })) {
+        a.len_class[3] |= 1u << p;
+        return;
+    }
     uint32_t weight;
     m.r0 = rarest_place(host, len, 1, 4, weight);
     if (weight >= kPoorAnchor) {
-        if (len <= kSearchMaxStagedPattern && std::all_of(host, host + len, [&](uint8_t c) { return c == host[0]; })) {
-            a.len_class[3] |= 1u << p;
-        } else {
-            m.r0 = rarest_place(host, len, 0, 1, weight);
-            for (uint32_t j = 0; j < 4; j++) m.pre[j] = host[m.r0 + j] * 0x01010101u;
-            a.len_class[2] |= 1u << p;
-        }
+        m.r0 = rarest_place(host, len, 0, 1, weight);
+        for (uint32_t j = 0; j < 4; j++) m.pre[j] = host[m.r0 + j] * 0x01010101u;
+        a.len_class[2] |= 1u << p;
         return;
     }
     a.len_class[1] |= 1u << p;
