@@ -110,12 +110,13 @@ constexpr uint32_t kSearchMaxPatterns = 8;  // patterns per launch
 // pattern bytes (search_add_pattern) and read by every block as kernel
 // parameters.
 struct alignas(16) SearchPatMeta {
-    uint32_t pre[4];  // bytes 0..3 (found by its rarest four bytes: r0..r0 + 3), each replicated into a word (0 past the end)
+    uint32_t pre[4];  // bytes 0..3, each replicated into a word (0 past the end); of a pattern found by its rarest
+                      // four bytes, the rarest two of those so, and the four, r0..r0 + 3, as a word
     uint32_t anc[4];  // anchor words: bytes [r, r + 4) little-endian, r = r0 + 1 .. r0 + 4
     uint32_t len;
     uint32_t r0;
     uint32_t last4;   // the last four bytes (len >= 4)
-    uint32_t pad;
+    uint32_t pair;    // the place of the rarest two in r0..r0 + 3
 };
 constexpr uint32_t kSearchInlinePattern = 64;   // patterns of up to this length travel in a launch's parameters
 constexpr uint32_t kSearchPatBytes = kSearchInlinePattern * kSearchMaxPatterns;  // room for as many as a launch takes
@@ -148,6 +149,7 @@ struct SearchArgs {
     uint32_t anchor_hash[kSearchMaxPatterns * 4];  // anchor-map bits of the patterns of >= 8 bytes
     uint32_t n_anchor;
     uint32_t anchor_words;  // aligned text words past a tile that may be anchors of starts in it
+    uint32_t window_pieces; // 16-byte pieces to look for the other patterns in
     // bit p: pattern p is decided whole (up to 7 bytes); found by its anchors, by
     // its rarest four bytes, or as a run of one byte (search_add_pattern)
     uint32_t len_class[4];

@@ -14,10 +14,10 @@
 // together; a word found there gives the one start it can belong to, which is
 // queued per warp and verified word by word, 32 at a time, one per lane. Where
 // in the pattern the anchor words lie is chosen by how rare such words are in
-// text. Where they cannot but be runs of one byte (which made nearly every piece
-// of indented text a candidate), a run c^m is decided from the masks of c at 64
-// positions, and any other pattern is looked for by its rarest four bytes, at
-// all starts like a short one. An occurrence must end inside the text (the
+// text. A run c^m is decided from the masks of c at 64 positions; any other
+// pattern whose anchor words cannot but be runs of one byte (which made nearly
+// every piece of indented text a candidate) is looked for by its rarest four
+// bytes, at all starts like a short one. An occurrence must end inside the text (the
 // buffer is zero padded: a pattern ending in NUL must not match the padding).
 // Recomputing form, three launches, no block waits on another:
 //   1. search_count_kernel: matches per (tile, pattern);
@@ -69,12 +69,13 @@ __host__ __device__ __forceinline__ uint32_t anchor_hash(uint32_t w) {
 }
 
 struct alignas(16) PatMeta {  // a SearchPatMeta, copied from the kernel parameters 16 bytes a lane
-    uint4 pre;  // bytes 0..3 of the pattern (window patterns: r0..r0 + 3), each replicated into a word (unused ones 0)
+    uint4 pre;  // bytes 0..3 of the pattern, each replicated into a word (unused ones 0); of a window pattern: its
+                // rarest two so, and the window r0..r0 + 3 as a word
     uint4 anc;  // anchor words r = r0 + 1 .. r0 + 4
     uint32_t len;
     uint32_t r0;
     uint32_t last4;  // the last four bytes (len >= 4)
-    uint32_t pad;
+    uint32_t pair;   // window patterns: the place of those two in the window
 };
 static_assert(sizeof(PatMeta) == 48 && sizeof(SearchPatMeta) == 48, "copied as three 16-byte pieces");
 
@@ -375,37 +376,48 @@ __device__ __forceinline__ uint32_t filter_tile(const SearchArgs &a, SearchSmem 
             }
         }
     }
-    // The other patterns, piece by piece (windows: the pieces past the tile too).
+    // The other patterns, piece by piece (windows: the pieces past the tile too). A
+    // window is looked for by its rarest two bytes: by its first byte, which is
+    // most often the common one, a pattern like "||||||||a" took 102 us in 64 MiB of
+    // "|" and 70 in outline text; now 41 and 41.
+    if (const uint32_t others = windows | runs) {
 #pragma unroll 1
-    for (uint32_t bits = windows | runs; bits; bits &= bits - 1) {
-        const uint32_t p = __ffs(bits) - 1, r0 = sm.pat[p].r0;
-        const uint4 pre = sm.pat[p].pre;
-        const bool run = (runs >> p) & 1u;
-        const uint32_t n = SR_PIECES + (run ? 0 : (r0 + 15) / 16);
-#pragma unroll 1
-        for (uint32_t base = tid & ~31u; base < n; base += SR_THREADS) {  // whole warps
+        for (uint32_t base = tid & ~31u; base < a.window_pieces; base += SR_THREADS) {  // whole warps
             const uint32_t piece = base + lane;
-            const uint4 v = *reinterpret_cast<const uint4 *>(&sm.text[piece * 16]);  // (past the pieces: not used)
-            if (run) {  // of eight and more: it holds an aligned word of the byte, in the piece or right after it
-                bool word = v.x == pre.x || v.y == pre.x || v.z == pre.x || v.w == pre.x;
-                if (lane == 31) word |= *reinterpret_cast<const uint32_t *>(&sm.text[(piece + 1) * 16]) == pre.x;
-                if (!__any_sync(0xFFFFFFFFu, word)) continue;
-                const uint32_t r = run_starts(a, sm, p, eq_mask16(v, pre.x), piece, t0);
-                if (r) pieces(p, piece, r);
-                continue;
-            }
-            uint32_t g = eq_mask16(v, pre.x);
-            if (!__any_sync(0xFFFFFFFFu, g != 0)) continue;
-            if (g) {  // the window's first byte: its four bytes
-                const uint32_t want = (pre.x & 0xFFu) | (pre.y & 0xFF00u) | (pre.z & 0xFF0000u) | (pre.w & 0xFF000000u);
-                uint32_t ok = 0;
-                for (; g; g &= g - 1) {
-                    const uint32_t b = __ffs(g) - 1;
-                    if (text4(a, sm, piece * 16 + b, true, t0) == want) ok |= 1u << b;
+            const uint4 v = *reinterpret_cast<const uint4 *>(&sm.text[piece * 16]);
+            uint32_t w4 = __shfl_down_sync(0xFFFFFFFFu, v.x, 1);
+            if (lane == 31) w4 = *reinterpret_cast<const uint32_t *>(&sm.text[(piece + 1) * 16]);
+#pragma unroll 1
+            for (uint32_t bits = others; bits; bits &= bits - 1) {
+                const uint32_t p = __ffs(bits) - 1;
+                const uint4 pre = sm.pat[p].pre;
+                if ((runs >> p) & 1u) {  // of eight and more: it holds an aligned word of it, in the piece or right after
+                    if (base >= SR_PIECES ||
+                        !__any_sync(0xFFFFFFFFu, v.x == pre.x || v.y == pre.x || v.z == pre.x || v.w == pre.x || w4 == pre.x))
+                        continue;
+                    const uint32_t g = run_starts(a, sm, p, eq_mask16(v, pre.x), piece, t0);
+                    if (g) pieces(p, piece, g);
+                    continue;
                 }
-                g = piece < n ? ok : 0u;
+                // the window's rarest two bytes, in any of the sixteen places: a zero byte in one of four words
+                const uint32_t x[4] = {(v.x ^ pre.x) | (__funnelshift_r(v.x, v.y, 8) ^ pre.y),
+                                       (v.y ^ pre.x) | (__funnelshift_r(v.y, v.z, 8) ^ pre.y),
+                                       (v.z ^ pre.x) | (__funnelshift_r(v.z, v.w, 8) ^ pre.y),
+                                       (v.w ^ pre.x) | (__funnelshift_r(v.w, w4, 8) ^ pre.y)};
+                uint32_t z = 0;
+#pragma unroll
+                for (int i = 0; i < 4; i++) z |= (x[i] - 0x01010101u) & ~x[i];
+                if (!__any_sync(0xFFFFFFFFu, (z & 0x80808080u) != 0)) continue;
+                const uint32_t r0 = sm.pat[p].r0, pair = sm.pat[p].pair;
+                uint32_t ok = 0;
+                if (piece < SR_PIECES + (r0 + pair + 15) / 16) {  // where they are: the window's four bytes
+                    for (uint32_t g = gather16(zero_bytes(x[0]), zero_bytes(x[1]), zero_bytes(x[2]), zero_bytes(x[3])); g; g &= g - 1) {
+                        const uint32_t b = __ffs(g) - 1, off = piece * 16 + b - pair;
+                        if (off < kSearchTile + 512 && text4(a, sm, off, true, t0) == pre.z) ok |= 1u << b;
+                    }
+                }
+                queue_starts(p, ok, piece * 16 - pair - r0);
             }
-            queue_starts(p, g, piece * 16 - r0);
         }
     }
     if (queued) drain();
@@ -835,14 +847,22 @@ void search_add_pattern(SearchArgs &a, const uint8_t *host, const uint8_t *dev, 
     // eight of them looked for: 340 us by anchors, 71 by masks).
     if (len <= kSearchMaxStagedPattern && std::all_of(host, host + len, [&](uint8_t c) { return c == host[0]; })) {
         a.len_class[3] |= 1u << p;
+        a.window_pieces = std::max(a.window_pieces, SR_PIECES);
         return;
     }
     uint32_t weight;
     m.r0 = rarest_place(host, len, 1, 4, weight);
     if (weight >= kPoorAnchor) {
         m.r0 = rarest_place(host, len, 0, 1, weight);
-        for (uint32_t j = 0; j < 4; j++) m.pre[j] = host[m.r0 + j] * 0x01010101u;
+        const uint8_t *w = host + m.r0;
+        auto pair_weight = [&](uint32_t j) { return byte_weight(w[j]) + byte_weight(w[j + 1]) + (w[j] == w[j + 1] ? 4 : 0); };
+        for (uint32_t j = 1; j < 3; j++)
+            if (pair_weight(j) < pair_weight(m.pair)) m.pair = j;
+        m.pre[0] = w[m.pair] * 0x01010101u;
+        m.pre[1] = w[m.pair + 1] * 0x01010101u;
+        m.pre[2] = word(m.r0);
         a.len_class[2] |= 1u << p;
+        a.window_pieces = std::max(a.window_pieces, SR_PIECES + (m.r0 + m.pair + 15) / 16);
         return;
     }
     a.len_class[1] |= 1u << p;
