@@ -280,7 +280,7 @@ __device__ __forceinline__ void parse_tile(const ParseArgs &a, ParseSmem &sm, ui
     for (uint32_t r0 = 0; r0 < n_lines; r0 += PT_LIST) {
         const int32_t w0 = (int32_t)r0 - (int32_t)off;  // rank of nl[0]
         int32_t rk = (int32_t)rank - w0;
-        if (rk <= (int32_t)PT_LIST) {
+        if (rk <= (int32_t)PT_LIST && rk + (int32_t)cnt > 0) {  // some of the thread's are in the round
             auto list = [&](uint32_t m, uint32_t lo) {  // the warp runs as many rounds as its busiest lane has newlines
                 for (; m; m &= m - 1, rk++)
                     if (STAGE || (rk >= 0 && rk <= (int32_t)PT_LIST)) sm.nl[rk] = (uint16_t)(lo + __ffs(m) - 1);
@@ -472,7 +472,10 @@ __global__ void __launch_bounds__(256) parse_copy_kernel(ParseArgs a) {
 // deepest line. Block b looks through tiles b, b + grid, ...: one atomic a
 // block. (One a warp and tile of the stage pass, all on one address, made that
 // pass 438 us per GiB in some processes and 704 us in others, on one box; it
-// now takes 457 us in all.)
+// now takes 457 us in all.) The grid is as many blocks as run at a time: a dense
+// tile is a long chain of rounds (32 MiB of newlines: 360 us with 512 blocks, 282
+// so; of two-byte lines 164 and 132).
+constexpr uint32_t kRedoGrid = 148 * 6;
 __global__ void __launch_bounds__(PT_THREADS, 6) parse_redo_kernel(ParseArgs a) {
     __shared__ ParseSmem sm;
     __shared__ uint32_t list[PT_THREADS], n_list, deepest;
@@ -544,7 +547,7 @@ cudaError_t launch_parse_end(const ParseArgs &a, cudaStream_t st) {
     cudaError_t e = launch_scan_columns(a.tile_count, a.tile_base, nullptr, a.n_tiles, 1, scan_ld(a.n_tiles), st);
     if (e != cudaSuccess) return e;
     parse_copy_kernel<<<(a.n_tiles + PC_TILES - 1) / PC_TILES, 256, 0, st>>>(a); OL_LAUNCHED();
-    parse_redo_kernel<<<std::min(a.n_tiles, 512u), PT_THREADS, 0, st>>>(a); OL_LAUNCHED();
+    parse_redo_kernel<<<std::min(a.n_tiles, kRedoGrid), PT_THREADS, 0, st>>>(a); OL_LAUNCHED();
     return cudaGetLastError();
 }
 
