@@ -35,9 +35,8 @@ constexpr uint32_t OL_DEVERR_CAPACITY = 1u << 1;  // an output buffer was too sm
 struct DocStats {
     uint32_t line_count;        // lines in the document
     uint32_t max_content_depth; // deepest non-blank line (saturates at 0xFFFFFFFF)
-    uint32_t reserved;
     uint32_t error;             // OL_DEVERR_* bits
-    uint32_t pad[12];
+    uint32_t pad[13];
 };
 
 // ---------------------------------------------------------- memory access --

@@ -75,7 +75,6 @@ struct TreeArgs {
     uint32_t *tile_first;    // n_tiles * kTreeLevels: first content line of each depth in the tile (NONE: none)
     uint32_t *in_last;       // exclusive prefix max of tile_last over the tiles
     uint32_t *in_first;      // exclusive suffix min of tile_first over the tiles
-    DocStats *stats;
     uint32_t *parent;
     uint32_t *subtree_end;   // optional
     uint32_t *first_child;
@@ -130,7 +129,6 @@ struct SearchArgs {
     uint32_t np;                                // patterns in this launch (1..8)
     uint32_t halo;                              // round_up(longest - 1, 16); > 4096 only when np == 1
     const uint8_t *pat[kSearchMaxPatterns];     // device copies (16-byte aligned), or nullptr: in pat_bytes
-    uint32_t pat_len[kSearchMaxPatterns];
     uint32_t *out[kSearchMaxPatterns];          // ascending offsets, first max_out[p] of them
     uint32_t max_out[kSearchMaxPatterns];
     uint32_t ld;             // column stride of counts and bases: scan_ld(n_tiles)
@@ -279,7 +277,6 @@ struct DictMatchArgs {
     uint32_t tile_stride;    // tiles 0, s, 2s, ... (count mode samples)
     uint32_t count_only;     // 1: counts[u] += every hit; 0: heavy bitmaps + light keys
     uint32_t *counts;        // per unique pattern (count mode: all hits; else light hits)
-    const uint8_t *heavy_of_u;  // heavy index or 0xFF
     const DictPlan *plan;    // (not in count mode)
     uint32_t *bitmap;        // [n_heavy][n_tiles * kDictWordsPerTile]
     uint32_t *heavy_counts;  // [n_heavy][heavy_ld]: += hits per tile

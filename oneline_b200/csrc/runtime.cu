@@ -138,9 +138,8 @@ extern "C" ol_status ol_ctx_create(int32_t device, ol_ctx **out) {
         uint64_t thr = UINT64_MAX;
         cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr);
     }
-    e = cudaMallocAsync((void **)&c->counters, sizeof(CtxCounters), c->stream);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->pat_done, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaMallocHost((void **)&c->host_counters, sizeof(CtxCounters));
+    e = cudaEventCreateWithFlags(&c->pat_done, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaMallocHost((void **)&c->host_stats, sizeof(DocStats));
     for (int i = 0; i < kRingSlots && e == cudaSuccess; i++) {
         e = cudaMallocHost((void **)&c->ring[i], kRingBytes);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ring_done[i], cudaEventDisableTiming);
@@ -174,9 +173,8 @@ extern "C" void ol_ctx_destroy(ol_ctx *ctx) {
     ctx->dict_hits.release(ctx->stream);
     ctx->dict_sort.release(ctx->stream);
     ctx->host_words.release();
-    if (ctx->counters) cudaFreeAsync(ctx->counters, ctx->stream);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-    if (ctx->host_counters) cudaFreeHost(ctx->host_counters);
+    if (ctx->host_stats) cudaFreeHost(ctx->host_stats);
     if (ctx->pat_host) cudaFreeHost(ctx->pat_host);
     if (ctx->pat_done) cudaEventDestroy(ctx->pat_done);
     for (int i = 0; i < kRingSlots; i++) {
@@ -373,7 +371,7 @@ ol_status parse_doc(ol_ctx *ctx, ol_doc *d, uint64_t est_lines, const uint8_t *h
         // the first attempt uploads the text as it parses; a retry finds every tile staged
         cudaError_t e = attempt ? enqueue_parse_end(ctx, d)
                                 : host_text ? upload_parse_overlapped(ctx, d, host_text, d->text_len) : enqueue_parse(ctx, d);
-        DocStats *pinned = &ctx->host_counters->doc;
+        DocStats *pinned = ctx->host_stats;
         if (e == cudaSuccess) e = cudaMemcpyAsync(pinned, d->stats, sizeof(DocStats), cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         if (e != cudaSuccess) return ctx_cuda(ctx, e, "parse");

@@ -36,14 +36,6 @@ struct HostBuf {
 
 struct Prof;
 
-// Small per-context words in device memory, and their page-locked copy on the
-// host: short results are read back through the latter.
-struct CtxCounters {
-    uint32_t error;
-    uint32_t pad[15];
-    DocStats doc;  // a parse's counters
-};
-
 }  // namespace ol
 
 struct ol_ctx {
@@ -73,8 +65,7 @@ struct ol_ctx {
     ol::DevBuf dict_sort;    // the light-hit sort's histograms
     ol::HostBuf host_words;  // short results read back (page-locked)
     ol::DevBuf dict_hits;    // hits of the blocking search before the download
-    ol::CtxCounters *counters = nullptr;
-    ol::CtxCounters *host_counters = nullptr;  // pinned
+    ol::DocStats *host_stats = nullptr;  // a parse's counters read back (page-locked)
     uint8_t *pat_host = nullptr;  // pinned staging for pattern bytes
     size_t pat_host_bytes = 0;
     cudaEvent_t pat_done = nullptr;

@@ -497,7 +497,6 @@ ol_status ol::many_run(ol_ctx *ctx, const ol_doc *d, const ol_patset *set, uint6
         ma.tile_stride = 1;
         ma.count_only = 0;
         ma.counts = light_count;
-        ma.heavy_of_u = pa.heavy_of_u;
         ma.plan = pa.plan;
         ma.bitmap = (uint32_t *)ctx->dict_bitmap.ptr;
         ma.heavy_counts = heavy_counts;

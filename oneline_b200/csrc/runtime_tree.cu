@@ -48,7 +48,6 @@ cudaError_t enqueue_tree_fast(ol_ctx *ctx, const ol_doc *d, ol_tree *t) {
     a.tile_first = w + words;
     a.in_last = w + 2 * words;
     a.in_first = w + 3 * words;
-    a.stats = d->stats;
     a.parent = (uint32_t *)t->parent_buf.ptr;
     a.subtree_end = (uint32_t *)t->end_buf.ptr;
     a.first_child = (uint32_t *)t->fc_buf.ptr;

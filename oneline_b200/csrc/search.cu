@@ -832,7 +832,6 @@ void search_add_pattern(SearchArgs &a, const uint8_t *host, const uint8_t *dev, 
                         uint32_t max_out) {
     const uint32_t p = a.np++;
     a.pat[p] = dev;
-    a.pat_len[p] = len;
     a.out[p] = out;
     a.max_out[p] = max_out;
     SearchPatMeta &m = a.meta[p];

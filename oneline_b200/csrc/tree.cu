@@ -503,7 +503,6 @@ __global__ void __launch_bounds__(TD_LINES) deep_top_kernel(TreeDeepArgs a) {
 }
 
 __device__ __forceinline__ uint32_t umin(uint32_t a, uint32_t b) { return a < b ? a : b; }
-__device__ __forceinline__ uint64_t umin64(uint64_t a, uint64_t b) { return a < b ? a : b; }
 
 // Entry i of level l (lines: -1), or NONE past its end.
 __device__ __forceinline__ uint32_t deep_value(const TreeDeepArgs &a, int32_t l, uint64_t i) {
