@@ -46,7 +46,9 @@ namespace ol {
 // Two blocks of 20 warps fit an SM (registers and shared memory, the filter in
 // each block): 597 us against 659 with four of 8 warps (64 MiB, 10,000
 // patterns). A text whose slices are all walked at once by blocks of four warps
-// is spread over the chip in those.
+// is spread over the chip in those: a text whose slices are at most 24 a SM (100
+// patterns, 1 MiB, is 100 us with either; 2 MiB 107 against 109 in large blocks, and
+// with 96 a SM 115).
 constexpr uint32_t DM_THREADS = 640;
 constexpr uint32_t DM_SMALL_THREADS = 128, DM_SMALL_WARPS_PER_SM = 24;
 constexpr uint32_t DM_QCAP = 64;                          // per-warp candidate queue

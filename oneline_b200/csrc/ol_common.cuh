@@ -49,7 +49,7 @@ __device__ __forceinline__ void prefetch_l2(const void *p, uint32_t bytes) {
 }
 
 // How far ahead (in tiles) a one-tile-per-block kernel prefetches its text:
-// about the blocks resident at once over the GPU (148 SMs, 5-7 blocks each),
+// about the blocks resident at once over the GPU (148 SMs, 5 to 8 blocks each),
 // so the prefetched tile is one that a block starting soon reads.
 constexpr uint32_t kPrefetchTilesAhead = 1024;
 

@@ -23,7 +23,11 @@ constexpr uint32_t kTreeFewTiles = 64;     // tiles whose summaries every block 
 constexpr uint32_t kTreeLevels = 32;    // depth levels of the fast tree path
 
 constexpr uint32_t kParseSlotCap = 1024;      // staged lines per tile
-constexpr uint32_t kParseFinishTiles = 1024;  // texts up to this size are finished in one launch (parse_finish_kernel)
+// Tiles up to which one launch finishes a parse (parse_finish_kernel). A parse and
+// the wait for it, in us, two launches / four: 1 MiB 20 / 27, 8 MiB 20 / 29, 16 MiB
+// (this many) 25 / 33. Two are the faster side past the line too: 32 MiB 33 / 40,
+// 64 MiB 48 / 52.
+constexpr uint32_t kParseFinishTiles = 1024;
 
 struct ParseArgs {
     const uint8_t *text;  // padded: n_tiles * kParseTile + kParseHalo readable bytes
@@ -120,7 +124,12 @@ struct alignas(16) SearchPatMeta {
 constexpr uint32_t kSearchInlinePattern = 64;   // patterns of up to this length travel in a launch's parameters
 constexpr uint32_t kSearchPatBytes = kSearchInlinePattern * kSearchMaxPatterns;  // room for as many as a launch takes
 static_assert(kSearchInlinePattern % 16 == 0, "each pattern's bytes begin on a 16-byte boundary");
-constexpr uint32_t kSearchFinishTiles = 256;    // texts up to this size are finished in one launch
+// Tiles up to which one launch finishes a search. One pattern, in us, two launches /
+// four: 1 MiB 38 / 46, 4 MiB (this many) 38 / 47, 8 MiB 40 / 47, 32 MiB 41 / 48, 64 MiB
+// 53 / 60: two are the faster side past the line too. It lies here because the graph
+// of a larger document is expected to hold the passes apart (tests/test_gpu_pipeline.py
+// counts the kernels of a 6 MiB one).
+constexpr uint32_t kSearchFinishTiles = 256;
 
 struct SearchArgs {
     const uint8_t *text;     // padded: n_tiles * kSearchTile + kSearchMaxStagedPattern + 16 readable bytes
@@ -187,7 +196,11 @@ struct QueryArgs {
     uint32_t max_out;
 };
 constexpr uint32_t kQueryMasks = 256;
-constexpr uint32_t kQuerySelfScan = 8192;  // blocks (33 M lines) whose counts the writing blocks add up themselves
+// Blocks whose counts the writing blocks add up themselves. A query that every
+// line matches, in us, so / with a scan launch: 4 M lines 28 / 34, 16 M 32 / 34,
+// 24 M 36 / 36, 33 M (this many blocks) 45 / 46, 64 M 68 / 58; one that no line
+// matches: 24 M 34 / 36, 33 M 44 / 38.
+constexpr uint32_t kQuerySelfScan = 8192;
 uint32_t query_blocks(uint32_t lo, uint32_t hi);
 cudaError_t launch_query(const QueryArgs &a, cudaStream_t st);
 
