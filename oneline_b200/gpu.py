@@ -79,23 +79,23 @@ def _line_guess(text) -> int:
     return min(n + 1, int((found + 4) / (4 * w) * n * 1.25) + 4096)
 
 
-def _line_arrays(text, dtypes, call) -> list[np.ndarray]:
-    """Arrays with an entry for every line of `text`, which call(pointers, room,
-    &count) fills when there is room."""
+def _line_arrays(ctx, call, ptr: int, text, dtypes) -> list[np.ndarray]:
+    """The results of a one-shot ``call`` on `text` (at ptr): arrays with an entry for every line."""
     cnt, cap, guess = ctypes.c_uint64(), _line_guess(text), True
     while True:
         try:
-            arrays, room = [np.empty(cap, t) for t in dtypes], cap
+            arrays = [np.empty(cap, t) for t in dtypes]
+            to, room = [a.ctypes.data for a in arrays], cap
         except MemoryError:  # the guess is more than this host gives: count first
             if not guess:
                 raise
-            arrays, room = None, 0
-        call([a.ctypes.data for a in arrays] if arrays else [None] * len(dtypes), room, ctypes.byref(cnt))
-        if arrays and cnt.value <= room:
+            to, room = [None] * len(dtypes), -1
+        check(call(ctx, ptr, len(text), *to, max(room, 0), ctypes.byref(cnt)), ctx)
+        lines = cnt.value
+        if lines <= room:
             break
-        cap, guess = cnt.value, False  # nothing was written
-    lines = cnt.value
-    if lines < cap // 2:  # give back what the guess had too much
+        cap, guess = lines, False  # nothing was written
+    if lines < cap // 2 and cap > 4096:  # give back what the guess had too much
         for a in arrays:
             a.resize(lines, refcheck=False)
         return arrays
@@ -438,9 +438,7 @@ class GpuParser:
     def parse_raw(self, text) -> FlatTree:
         p, n, keep, src = _as_bytes_view(text)
         _check_len(n)
-        L = _lib.load()
-        offs, nodes = _line_arrays(keep, (np.uint32, NODE_DTYPE), lambda ptrs, cap, cnt: check(
-            L.ol_parse_raw(self._ctx, p, n, *ptrs, cap, cnt), self._ctx))
+        offs, nodes = _line_arrays(self._ctx, _lib.load().ol_parse_raw, p, keep, (np.uint32, NODE_DTYPE))
         return FlatTree(src if isinstance(src, bytes) else bytes(src), nodes, offs)
 
     def parse(self, text, line_offsets) -> FlatTree:
@@ -456,9 +454,7 @@ class GpuParser:
     def scan_line_offsets(self, text) -> np.ndarray:
         p, n, keep, src = _as_bytes_view(text)
         _check_len(n)
-        L = _lib.load()
-        return _line_arrays(keep, (np.uint32,), lambda ptrs, cap, cnt: check(
-            L.ol_scan_line_offsets(self._ctx, p, n, *ptrs, cap, cnt), self._ctx))[0]
+        return _line_arrays(self._ctx, _lib.load().ol_scan_line_offsets, p, keep, (np.uint32,))[0]
 
     # ----------------------------------------------------------------- tree
 
