@@ -439,7 +439,7 @@ ol_status ol::many_run(ol_ctx *ctx, const ol_doc *d, const ol_patset *set, uint6
     pa.outs = (uint32_t *)(b + o_outs);
     pa.plan = &meta->plan;
     if (e == cudaSuccess) e = launch_dict_plan(pa, st);
-    uint32_t H = kDictMaxHeavy;
+    uint32_t H = std::min(kDictMaxHeavy, U);  // as many as there can be
     uint64_t cap = std::max<uint64_t>(N / 16, 65536);
     auto read_plan = [&]() -> ol_status {  // as many heavy patterns and light hits as the sample promises
         cudaError_t r = read_meta();
