@@ -123,7 +123,8 @@ constexpr size_t kWholeResult = 64 << 10;
 // Matches (of up to 64 patterns) up to this size are read back through
 // page-locked memory: copies that only have to be enqueued, and one wait, where
 // each copy to pageable memory waits for itself (11.7 us against 1 and a wait of
-// 6). 100 MB, five patterns, three with matches: 212 us before, 173 now.
+// 6). 100 MB, five patterns, three with matches: 205 to 230 us before, 171 to 200
+// now, by process.
 constexpr size_t kStagedResult = 1 << 20;
 
 // Blocking multi-pattern search into host buffers.
