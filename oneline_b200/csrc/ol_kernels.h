@@ -157,9 +157,10 @@ struct SearchArgs {
     uint32_t n_anchor;
     uint32_t anchor_words;  // aligned text words past a tile that may be anchors of starts in it
     uint32_t window_pieces; // 16-byte pieces to look for the other patterns in
-    // bit p: pattern p is decided whole (up to 7 bytes); found by its anchors, by
-    // its rarest four bytes, or as a run of one byte (search_add_pattern)
-    uint32_t len_class[4];
+    // bit p: pattern p is decided whole (up to 4 bytes); found by its anchors, by
+    // its rarest four bytes, as a run of one byte, or (5 to 7 bytes) by its first
+    // two (search_add_pattern)
+    uint32_t len_class[5];
     // The bytes of patterns without a device copy, each from a 16-byte boundary.
     uint32_t n_pat_bytes;
     uint32_t pat_at[kSearchMaxPatterns];

@@ -168,6 +168,33 @@ __device__ __forceinline__ void load_tile(const SearchArgs &a, SearchSmem &sm, u
     cp_async_wait();
 }
 
+// Whether one of the sixteen bytes is zero, without telling which.
+__device__ __forceinline__ bool any_zero_byte(const uint32_t (&x)[4]) {
+    uint32_t z = 0;
+#pragma unroll
+    for (int i = 0; i < 4; i++) z |= (x[i] - 0x01010101u) & ~x[i];
+    return (z & 0x80808080u) != 0;
+}
+
+// The starts of pattern p (5 to 7 bytes) in a piece, whole: its first four bytes at
+// the sixteen starts at once, then the last four at the starts that are left.
+__device__ __forceinline__ uint32_t mid_starts(const SearchArgs &a, const SearchSmem &sm, uint32_t p, uint32_t piece,
+                                            bool tail_tile, uint64_t t0) {
+    const uint32_t *t = reinterpret_cast<const uint32_t *>(&sm.text[piece * 16]), m = sm.pat[p].len;
+    const uint4 pre = sm.pat[p].pre;
+    uint32_t c[4], g, ok = 0;
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+        c[i] = zero_bytes((t[i] ^ pre.x) | (__funnelshift_r(t[i], t[i + 1], 8) ^ pre.y) |
+                          (__funnelshift_r(t[i], t[i + 1], 16) ^ pre.z) | (__funnelshift_r(t[i], t[i + 1], 24) ^ pre.w));
+    if (tail_tile) keep_valid_starts(a.text_len, m, t0, piece * 16, c[0], c[1], c[2], c[3]);
+    for (g = gather16(c[0], c[1], c[2], c[3]); g; g &= g - 1) {
+        const uint32_t b = __ffs(g) - 1;
+        if (text4(a, sm, piece * 16 + b + m - 4, true, t0) == sm.pat[p].last4) ok |= 1u << b;
+    }
+    return ok;
+}
+
 // Adds the match at tile start `start` to a pattern's masks, 16 starts each
 // (verified starts of one piece may come from several lanes).
 __device__ __forceinline__ void set_match(uint16_t *masks, uint32_t start) {
@@ -238,20 +265,21 @@ __device__ __forceinline__ uint32_t filter_tile(const SearchArgs &a, SearchSmem 
                                                 uint16_t (*match)[SR_PIECES], Pieces pieces) {
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const bool tail_tile = t0 + kSearchTile + a.halo + 16 > a.text_len;
-    // patterns in `mask` by how they are found: whole (up to 7 bytes), by anchors,
-    // by their rarest four bytes, as runs
+    // patterns in `mask` by how they are found: whole (up to 4 bytes), by anchors, by
+    // their rarest four bytes, as runs, by their first two bytes (5 to 7 bytes)
     const uint32_t shorts = a.len_class[0] & mask, anchored = a.len_class[1] & mask, windows = a.len_class[2] & mask,
-                   runs = a.len_class[3] & mask;
+                   runs = a.len_class[3] & mask, mids = a.len_class[4] & mask;
     auto in_map = [&](uint32_t x) {
         const uint32_t h = anchor_hash(x);
         return (sm.anchor_map[h >> 5] >> (h & 31)) & 1u;
     };
     uint32_t flagged = 0;  // bit 4k + i: word i of my piece of step k is in the map
+    uint32_t begun = 0;    // bit 4p + k: my piece of step k has pattern p's first two bytes (mids)
 #pragma unroll
     for (uint32_t k = 0; k < SR_STEPS; k++) {
         const uint32_t piece = k * SR_THREADS + tid;
         const uint4 vk = *reinterpret_cast<const uint4 *>(&sm.text[piece * 16]);
-        if (shorts) {  // uniform
+        if (shorts | mids) {  // uniform
             uint32_t w4 = __shfl_down_sync(0xFFFFFFFFu, vk.x, 1);
             if (lane == 31) w4 = *reinterpret_cast<const uint32_t *>(&sm.text[(piece + 1) * 16]);
             const uint32_t w[5] = {vk.x, vk.y, vk.z, vk.w, w4};
@@ -281,25 +309,22 @@ __device__ __forceinline__ uint32_t filter_tile(const SearchArgs &a, SearchSmem 
                     for (int i = 0; i < 4; i++) x[i] |= s3[i] ^ pre.w;
                 uint32_t c0 = zero_bytes(x[0]), c1 = zero_bytes(x[1]), c2 = zero_bytes(x[2]), c3 = zero_bytes(x[3]);
                 if (tail_tile) keep_valid_starts(a.text_len, m, t0, piece * 16, c0, c1, c2, c3);
-                if (c0 | c1 | c2 | c3) {
-                    uint32_t g = gather16(c0, c1, c2, c3);
-                    if (m > 4) {  // the last four bytes, at the starts still in question, one by one
-                        uint32_t ok = 0;
-                        for (; g; g &= g - 1) {
-                            const uint32_t b = __ffs(g) - 1, off = piece * 16 + b + m - 4;
-                            const uint32_t *tw = reinterpret_cast<const uint32_t *>(sm.text) + (off >> 2);
-                            if (__funnelshift_r(tw[0], tw[1], (off & 3) * 8) == sm.pat[p].last4) ok |= 1u << b;
-                        }
-                        g = ok;
-                    }
-                    if (g) pieces(p, piece, g);
-                }
+                if (c0 | c1 | c2 | c3) pieces(p, piece, gather16(c0, c1, c2, c3));
+            }
+#pragma unroll 1
+            for (uint32_t bits = mids; bits; bits &= bits - 1) {
+                const uint32_t p = __ffs(bits) - 1;
+                const uint2 pre = *reinterpret_cast<const uint2 *>(&sm.pat[p].pre);
+                uint32_t x[4];
+#pragma unroll
+                for (int i = 0; i < 4; i++) x[i] = (w[i] ^ pre.x) | (s1[i] ^ pre.y);
+                begun |= (any_zero_byte(x) ? 1u : 0u) << (4 * p + k);
             }
         }
         if (anchored)  // uniform
             flagged |= (in_map(vk.x) | (in_map(vk.y) << 1) | (in_map(vk.z) << 2) | (in_map(vk.w) << 3)) << (4 * k);
     }
-    if (!(anchored | windows | runs)) return 0;  // uniform
+    if (!(anchored | windows | runs | mids)) return 0;  // uniform
 
     const bool staged = a.halo <= kSearchMaxStagedPattern;
     uint32_t found = 0;
@@ -310,6 +335,11 @@ __device__ __forceinline__ uint32_t filter_tile(const SearchArgs &a, SearchSmem 
         __syncwarp();
         for (uint32_t i = lane; i < queued; i += 32) {
             const uint32_t e = queue[i], p = e >> 16, start = e & 0xFFFFu;
+            if ((mids >> p) & 1u) {  // a piece
+                const uint32_t g = mid_starts(a, sm, p, start, tail_tile, t0);
+                if (g) pieces(p, start, g);
+                continue;
+            }
             if (!verify_start(a, sm, p, start, staged, t0)) continue;
             found |= 1u << p;
             if (COUNT)
@@ -335,6 +365,14 @@ __device__ __forceinline__ uint32_t filter_tile(const SearchArgs &a, SearchSmem 
             g &= g - 1;
         }
     };
+    // Pieces with the first two bytes of a pattern of 5 to 7.
+#pragma unroll 1
+    for (uint32_t bits = mids; bits; bits &= bits - 1) {
+        const uint32_t p = __ffs(bits) - 1, mine = (begun >> (4 * p)) & 15u;
+        if (!__any_sync(0xFFFFFFFFu, mine != 0)) continue;
+#pragma unroll 1
+        for (uint32_t k = 0; k < SR_STEPS; k++) queue_start(p, k * SR_THREADS + tid, (mine >> k) & 1u);
+    }
     // Words in the map, against every pattern's anchors: those of the lane's
     // pieces, then (a round more) of the words past the tile, of starts in it.
     // Most often one lane or two have one; then the warp takes a word at a time
@@ -404,10 +442,7 @@ __device__ __forceinline__ uint32_t filter_tile(const SearchArgs &a, SearchSmem 
                                        (v.y ^ pre.x) | (__funnelshift_r(v.y, v.z, 8) ^ pre.y),
                                        (v.z ^ pre.x) | (__funnelshift_r(v.z, v.w, 8) ^ pre.y),
                                        (v.w ^ pre.x) | (__funnelshift_r(v.w, w4, 8) ^ pre.y)};
-                uint32_t z = 0;
-#pragma unroll
-                for (int i = 0; i < 4; i++) z |= (x[i] - 0x01010101u) & ~x[i];
-                if (!__any_sync(0xFFFFFFFFu, (z & 0x80808080u) != 0)) continue;
+                if (!__any_sync(0xFFFFFFFFu, any_zero_byte(x))) continue;
                 const uint32_t r0 = sm.pat[p].r0, pair = sm.pat[p].pair;
                 uint32_t ok = 0;
                 if (piece < SR_PIECES + (r0 + pair + 15) / 16) {  // where they are: the window's four bytes
@@ -843,7 +878,7 @@ void search_add_pattern(SearchArgs &a, const uint8_t *host, const uint8_t *dev, 
     };
     if (len >= 4) m.last4 = word(len - 4);
     if (len < kAnchorMin) {  // decided from these constants alone
-        a.len_class[0] |= 1u << p;
+        a.len_class[len > 4 ? 4 : 0] |= 1u << p;
         return;
     }
     if (!dev) {
