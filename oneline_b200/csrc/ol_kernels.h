@@ -161,6 +161,7 @@ struct SearchArgs {
     // its rarest four bytes, as a run of one byte, or (5 to 7 bytes) by its first
     // two (search_add_pattern)
     uint32_t len_class[5];
+    uint32_t rare_runs;     // those of the runs whose word is in the anchor map
     // The bytes of patterns without a device copy, each from a 16-byte boundary.
     uint32_t n_pat_bytes;
     uint32_t pat_at[kSearchMaxPatterns];

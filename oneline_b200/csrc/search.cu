@@ -5,16 +5,16 @@
 // shared memory with asynchronous 16-byte copies (in the stage pass, after asking
 // L2 to prefetch the tile kPrefetchTilesAhead further on, which a block that
 // starts soon will read). Every 16-byte piece is compared with each pattern of
-// up to 7 bytes at all sixteen starts at once (byte SWAR on the piece shifted by
-// 1, 2 and 3 bytes, built once for all patterns; of 5 to 7 bytes the last four
-// only where the first four occur), which decides it. Longer patterns are looked for
-// by their anchor words: four consecutive 4-byte words of the pattern, one of
-// which lies on a 4-byte boundary of the text in every occurrence. A shared hash
-// map of those words is tested once per aligned text word, for all patterns
-// together; a word found there gives the one start it can belong to, which is
-// queued per warp and verified word by word, 32 at a time, one per lane. Where
-// in the pattern the anchor words lie is chosen by how rare such words are in
-// text. A run c^m is decided from the masks of c at 64 positions; any other
+// up to 4 bytes at all sixteen starts at once (byte SWAR on the piece shifted by
+// 1, 2 and 3 bytes, built once for all patterns), which decides it; of 5 to 7 bytes
+// the first two are looked for like that, and the pieces that have them are queued
+// and compared whole. Longer patterns are looked for by their anchor words: four
+// consecutive 4-byte words of the pattern, one of which lies on a 4-byte boundary
+// of the text in every occurrence. A shared hash map of those words is tested once
+// per aligned text word, for all patterns together; a word found there gives the
+// one start it can belong to, which is queued per warp and verified word by word,
+// 32 at a time, one per lane. Where in the pattern the anchor words lie is chosen
+// by how rare such words are in text. A run c^m is decided from the masks of c at 64 positions; any other
 // pattern whose anchor words cannot but be runs of one byte (which made nearly
 // every piece of indented text a candidate) is looked for by its rarest four
 // bytes, at all starts like a short one. An occurrence must end inside the text (the
@@ -248,15 +248,16 @@ __device__ __forceinline__ uint32_t run_starts(const SearchArgs &a, const Search
 // memory). Every lane takes its four pieces, one per step, and builds once for
 // all patterns the windows of the piece shifted by 1, 2 and 3 bytes (the word
 // after the piece comes from the next lane, or from shared memory for lane 31).
-// Patterns of at most 7 bytes are decided at all sixteen starts at once; their
-// matches go to pieces(p, piece, 16-bit mask). Longer patterns share one test of
-// the piece's four aligned words against the anchor map, whose cost does not
-// grow with the number of patterns. What needs more than that comes after the
+// Patterns of at most 4 bytes are decided at all sixteen starts at once; their
+// matches go to pieces(p, piece, 16-bit mask). Patterns of 8 bytes and more share
+// one test of the piece's four aligned words against the anchor map, whose cost
+// does not grow with the number of patterns. What needs more than that comes after the
 // steps, in loops that are not unrolled (inside the steps, where everything is
 // there four times, it made the stage pass 680 us per GiB instead of 480): words
-// found in the map, the patterns without good anchors (runs, decided from masks
-// of 64 positions, and those compared by four bytes). Their starts are queued
-// per warp, verified 32 at a time, one per lane, and counted or set in `match`.
+// found in the map, pieces with the first two bytes of a pattern of 5 to 7, the
+// patterns without good anchors (runs, decided from masks of 64 positions, and
+// those compared by four bytes). Their starts, or pieces, are queued per warp,
+// verified 32 at a time, one per lane, and counted or set in `match`.
 // Returns the patterns whose starts the lane verified.
 // The pattern loops are not unrolled (the step loop is): with up to eight
 // patterns a fully unrolled body outgrows the instruction cache.
@@ -268,7 +269,7 @@ __device__ __forceinline__ uint32_t filter_tile(const SearchArgs &a, SearchSmem 
     // patterns in `mask` by how they are found: whole (up to 4 bytes), by anchors, by
     // their rarest four bytes, as runs, by their first two bytes (5 to 7 bytes)
     const uint32_t shorts = a.len_class[0] & mask, anchored = a.len_class[1] & mask, windows = a.len_class[2] & mask,
-                   runs = a.len_class[3] & mask, mids = a.len_class[4] & mask;
+                   runs = a.len_class[3] & mask, mids = a.len_class[4] & mask, rare = a.rare_runs & mask;
     auto in_map = [&](uint32_t x) {
         const uint32_t h = anchor_hash(x);
         return (sm.anchor_map[h >> 5] >> (h & 31)) & 1u;
@@ -321,7 +322,7 @@ __device__ __forceinline__ uint32_t filter_tile(const SearchArgs &a, SearchSmem 
                 begun |= (any_zero_byte(x) ? 1u : 0u) << (4 * p + k);
             }
         }
-        if (anchored)  // uniform
+        if (anchored | rare)  // uniform
             flagged |= (in_map(vk.x) | (in_map(vk.y) << 1) | (in_map(vk.z) << 2) | (in_map(vk.w) << 3)) << (4 * k);
     }
     if (!(anchored | windows | runs | mids)) return 0;  // uniform
@@ -373,6 +374,16 @@ __device__ __forceinline__ uint32_t filter_tile(const SearchArgs &a, SearchSmem 
 #pragma unroll 1
         for (uint32_t k = 0; k < SR_STEPS; k++) queue_start(p, k * SR_THREADS + tid, (mine >> k) & 1u);
     }
+    // Runs of rare bytes are looked for only where the warp's pieces, or the words
+    // right after them, have a word in the map.
+    uint32_t others = windows | runs;
+    if (rare) {  // uniform
+        bool some = flagged != 0;
+        if (lane == 31)
+            for (uint32_t k = 0; k < SR_STEPS; k++)
+                some |= in_map(*reinterpret_cast<const uint32_t *>(&sm.text[(k * SR_THREADS + tid + 1) * 16]));
+        if (!__any_sync(0xFFFFFFFFu, some)) others &= ~rare;
+    }
     // Words in the map, against every pattern's anchors: those of the lane's
     // pieces, then (a round more) of the words past the tile, of starts in it.
     // Most often one lane or two have one; then the warp takes a word at a time
@@ -418,7 +429,7 @@ __device__ __forceinline__ uint32_t filter_tile(const SearchArgs &a, SearchSmem 
     // window is looked for by its rarest two bytes: by its first byte, which is
     // most often the common one, a pattern like "||||||||a" took 102 us in 64 MiB of
     // "|" and 70 in outline text; now 41 and 41.
-    if (const uint32_t others = windows | runs) {
+    if (others) {  // the same in all lanes
 #pragma unroll 1
         for (uint32_t base = tid & ~31u; base < a.window_pieces; base += SR_THREADS) {  // whole warps
             const uint32_t piece = base + lane;
@@ -888,8 +899,14 @@ void search_add_pattern(SearchArgs &a, const uint8_t *host, const uint8_t *dev, 
     }
     // A run of one byte, however rare the byte: its four anchor words are the same,
     // and in text that is such a run every word has four candidates (64 MiB of "Z",
-    // eight of them looked for: 340 us by anchors, 71 by masks).
+    // eight of them looked for: 340 us by anchors, 80 by masks). The word of a
+    // rare byte is in the map all the same, to tell where there is nothing to look
+    // for: eight such patterns in 64 MiB without them 61 us without it, 49 with.
     if (len <= kSearchMaxStagedPattern && std::all_of(host, host + len, [&](uint8_t c) { return c == host[0]; })) {
+        if (word_weight(host) < kPoorAnchor) {
+            a.rare_runs |= 1u << p;
+            a.anchor_hash[a.n_anchor++] = anchor_hash(word(0));
+        }
         a.len_class[3] |= 1u << p;
         a.window_pieces = std::max(a.window_pieces, SR_PIECES);
         return;
