@@ -118,7 +118,10 @@ cudaError_t ol::launch_multi(ol_ctx *ctx, const ol_doc *d, const uint8_t *const 
 
 namespace {
 
-// Results (room for every match asked for) up to this size come back in one copy.
+// Results (room for every match asked for) up to this size are written to
+// page-locked host memory by the kernels. A copy that is enqueued while they run
+// waits about 6 us for them (and does not when the host is late): one pattern in
+// 1 MiB took 26 or 33 us by the pace of the host, 23 so.
 constexpr size_t kWholeResult = 64 << 10;
 // Matches (of up to 64 patterns) up to this size are read back through
 // page-locked memory: copies that only have to be enqueued, and one wait, where
@@ -142,13 +145,13 @@ ol_status search_multi_host(ol_ctx *ctx, const ol_doc *d, const uint8_t *const *
             out_words += std::max<uint32_t>(max_matches[i], 1);
         }
     if (idx.empty()) return OL_OK;
-    cudaError_t e = ctx->search_out.reserve(out_words * 4 + 64 * 4, st);
-    // a small result comes back whole in one copy, totals and room for matches;
-    // else the totals first, then the matches there are
+    // the kernels write a small result, totals and matches, where the host reads it;
+    // else the totals are copied first, then the matches there are
     const bool whole = idx.size() <= 64 && out_words * 4 <= kWholeResult;
+    cudaError_t e = whole ? cudaSuccess : ctx->search_out.reserve(out_words * 4 + 64 * 4, st);
     if (e == cudaSuccess) e = ctx->host_words.reserve(64 * 4 + (whole ? out_words * 4 : 0));
     if (e != cudaSuccess) return ctx_cuda(ctx, e, "search");
-    uint32_t *dev = (uint32_t *)ctx->search_out.ptr;
+    uint32_t *dev = (uint32_t *)(whole ? (void *)ctx->host_words.ptr : ctx->search_out.ptr);
     uint32_t *d_totals = dev;  // 64 slots
     std::vector<const uint8_t *> p2;
     std::vector<uint32_t> l2, m2;
@@ -164,8 +167,8 @@ ol_status search_multi_host(ol_ctx *ctx, const ol_doc *d, const uint8_t *const *
     for (size_t c = 0; c < idx.size(); c += 64) {
         uint32_t cn = (uint32_t)std::min<size_t>(64, idx.size() - c);
         e = enqueue_multi(ctx, d, p2.data() + c, l2.data() + c, cn, m2.data() + c, d_totals, o2.data() + c);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(ctx->host_words.ptr, d_totals, whole ? (64 + out_words) * 4 : cn * 4, cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess && !whole)
+            e = cudaMemcpyAsync(ctx->host_words.ptr, d_totals, cn * 4, cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         prof_mark(ctx, "search: wait for totals");
         if (e != cudaSuccess) return ctx_cuda(ctx, e, "search");
