@@ -79,28 +79,13 @@ def _line_guess(text) -> int:
     return min(n + 1, int((found + 4) / (4 * w) * n * 1.25) + 4096)
 
 
-def _line_arrays(ctx, call, ptr: int, text, dtypes) -> list[np.ndarray]:
-    """The results of a one-shot ``call`` on `text` (at ptr): arrays with an entry for every line."""
-    cnt, cap, guess = ctypes.c_uint64(), _line_guess(text), True
-    while True:
-        try:
-            arrays = [np.empty(cap, t) for t in dtypes]
-            to, room = [a.ctypes.data for a in arrays], cap
-        except MemoryError:  # the guess is more than this host gives: count first
-            if not guess:
-                raise
-            to, room = [None] * len(dtypes), -1
-        check(call(ctx, ptr, len(text), *to, max(room, 0), ctypes.byref(cnt)), ctx)
-        lines = cnt.value
-        if lines <= room:
-            break
-        cap, guess = lines, False  # nothing was written
-    if lines < cap // 2 and cap > 4096:  # give back what the guess had too much
-        for a in arrays:
+def _trim(lines: int, *arrays) -> None:
+    """Gives back what arrays made for a guess have too much, where that is more than
+    half. (Always shrinking costs the next arrays their pages: 8 MiB in lines of 10
+    bytes 4.1 ms, 1.6 so.)"""
+    for a in arrays:
+        if lines < a.size // 2:
             a.resize(lines, refcheck=False)
-        return arrays
-    # (shrinking always costs the next arrays their pages: 8 MiB in lines of 10 bytes 4.1 ms, 1.6 so)
-    return [a[:lines] for a in arrays]
 
 
 class _ProfileStep(ctypes.Structure):
@@ -438,8 +423,25 @@ class GpuParser:
     def parse_raw(self, text) -> FlatTree:
         p, n, keep, src = _as_bytes_view(text)
         _check_len(n)
-        offs, nodes = _line_arrays(self._ctx, _lib.load().ol_parse_raw, p, keep, (np.uint32, NODE_DTYPE))
-        return FlatTree(src if isinstance(src, bytes) else bytes(src), nodes, offs)
+        L = _lib.load()
+        cnt = ctypes.c_uint64()
+        cap = _line_guess(keep)
+        try:
+            offs, nodes = np.empty(cap, np.uint32), np.empty(cap, NODE_DTYPE)
+        except MemoryError:  # the guess is more than this host gives: count first
+            check(L.ol_parse_raw(self._ctx, p, n, None, None, 0, ctypes.byref(cnt)), self._ctx)
+            cap = cnt.value
+            offs, nodes = np.empty(cap, np.uint32), np.empty(cap, NODE_DTYPE)
+        while True:
+            check(L.ol_parse_raw(self._ctx, p, n, offs.ctypes.data, nodes.ctypes.data, cap, ctypes.byref(cnt)), self._ctx)
+            lines = cnt.value
+            if lines <= cap:
+                break
+            cap = lines  # nothing was written
+            offs, nodes = np.empty(cap, np.uint32), np.empty(cap, NODE_DTYPE)
+        if cap > 4096:
+            _trim(lines, offs, nodes)
+        return FlatTree(src if isinstance(src, bytes) else bytes(src), nodes[:lines], offs[:lines])
 
     def parse(self, text, line_offsets) -> FlatTree:
         p, n, keep, src = _as_bytes_view(text)
@@ -454,7 +456,24 @@ class GpuParser:
     def scan_line_offsets(self, text) -> np.ndarray:
         p, n, keep, src = _as_bytes_view(text)
         _check_len(n)
-        return _line_arrays(self._ctx, _lib.load().ol_scan_line_offsets, p, keep, (np.uint32,))[0]
+        L = _lib.load()
+        cnt = ctypes.c_uint64()
+        cap = _line_guess(keep)
+        try:
+            out = np.empty(cap, np.uint32)
+        except MemoryError:  # the guess is more than this host gives: count first
+            check(L.ol_scan_line_offsets(self._ctx, p, n, None, 0, ctypes.byref(cnt)), self._ctx)
+            cap = cnt.value
+            out = np.empty(cap, np.uint32)
+        while True:
+            check(L.ol_scan_line_offsets(self._ctx, p, n, out.ctypes.data, cap, ctypes.byref(cnt)), self._ctx)
+            if cnt.value <= cap:
+                break
+            cap = cnt.value  # nothing was written
+            out = np.empty(cap, np.uint32)
+        if cap > 4096:
+            _trim(cnt.value, out)
+        return out[: cnt.value]
 
     # ----------------------------------------------------------------- tree
 
