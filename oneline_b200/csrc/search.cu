@@ -259,17 +259,22 @@ __device__ __forceinline__ uint32_t run_starts(const SearchArgs &a, const Search
 // those compared by four bytes). Their starts, or pieces, are queued per warp,
 // verified 32 at a time, one per lane, and counted or set in `match`.
 // Returns the patterns whose starts the lane verified.
+// PLAIN: there are patterns of at most 4 bytes and with good anchors only. Without
+// the other kinds' code, though it is not run, the graph of parse, tree and search
+// over 1 GiB takes 1064 and 1325 us for two sets of eight such patterns, 1102 and
+// 1340 with it.
 // The pattern loops are not unrolled (the step loop is): with up to eight
 // patterns a fully unrolled body outgrows the instruction cache.
-template <bool COUNT, class Pieces>
+template <bool COUNT, bool PLAIN, class Pieces>
 __device__ __forceinline__ uint32_t filter_tile(const SearchArgs &a, SearchSmem &sm, uint32_t mask, uint64_t t0,
                                                 uint16_t (*match)[SR_PIECES], Pieces pieces) {
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const bool tail_tile = t0 + kSearchTile + a.halo + 16 > a.text_len;
     // patterns in `mask` by how they are found: whole (up to 4 bytes), by anchors, by
     // their rarest four bytes, as runs, by their first two bytes (5 to 7 bytes)
-    const uint32_t shorts = a.len_class[0] & mask, anchored = a.len_class[1] & mask, windows = a.len_class[2] & mask,
-                   runs = a.len_class[3] & mask, mids = a.len_class[4] & mask, rare = a.rare_runs & mask;
+    const uint32_t shorts = a.len_class[0] & mask, anchored = a.len_class[1] & mask, windows = PLAIN ? 0u : a.len_class[2] & mask,
+                   runs = PLAIN ? 0u : a.len_class[3] & mask, mids = PLAIN ? 0u : a.len_class[4] & mask,
+                   rare = PLAIN ? 0u : a.rare_runs & mask;
     auto in_map = [&](uint32_t x) {
         const uint32_t h = anchor_hash(x);
         return (sm.anchor_map[h >> 5] >> (h & 31)) & 1u;
@@ -480,7 +485,7 @@ __global__ void __launch_bounds__(SR_THREADS) search_count_kernel(const __grid_c
     __syncthreads();
     // Lanes with pieces of the same pattern add up their matches first: one
     // shared-memory atomic per (round, pattern) instead of one per piece.
-    filter_tile<true>(a, sm, 0xFFu, t0, nullptr, [&](uint32_t p, uint32_t piece, uint32_t mk) {
+    filter_tile<true, false>(a, sm, 0xFFu, t0, nullptr, [&](uint32_t p, uint32_t piece, uint32_t mk) {
         const uint32_t group = __match_any_sync(__activemask(), p);
         const uint32_t sum = __reduce_add_sync(group, __popc(mk));
         if ((threadIdx.x & 31) == __ffs(group) - 1 && sum) atomicAdd(&sm.count[p], sum);
@@ -512,7 +517,7 @@ __device__ __forceinline__ void write_tile(const SearchArgs &a, SearchSmem &sm, 
     for (uint32_t o = tid; o < NP * SR_PIECES / 8; o += SR_THREADS)
         reinterpret_cast<uint4 *>(&match[0][0])[o] = make_uint4(0, 0, 0, 0);
     __syncthreads();
-    filter_tile<false>(a, sm, want, t0, match,
+    filter_tile<false, false>(a, sm, want, t0, match,
                        [&](uint32_t p, uint32_t piece, uint32_t mk) { match[p][piece] = (uint16_t)mk; });
     __syncthreads();
     for (uint32_t w = want; w; w &= w - 1) {
@@ -587,7 +592,7 @@ __device__ __forceinline__ void list_starts(uint16_t *out, uint32_t bits, uint32
     }
 }
 
-template <uint32_t NP>
+template <uint32_t NP, bool PLAIN>
 __global__ void __launch_bounds__(SR_THREADS, 5) search_stage_kernel(const __grid_constant__ SearchArgs a) {
     constexpr uint32_t NQ = (NP + 1) / 2;  // packed count words, two patterns each
     __shared__ SearchSmem sm;
@@ -605,7 +610,7 @@ __global__ void __launch_bounds__(SR_THREADS, 5) search_stage_kernel(const __gri
     __syncthreads();
     // the patterns with hits anywhere in the tile, as the filter finds them
     uint32_t found = 0;
-    found |= filter_tile<false>(a, sm, (1u << NP) - 1u, t0, match, [&](uint32_t p, uint32_t piece, uint32_t mk) {
+    found |= filter_tile<false, PLAIN>(a, sm, (1u << NP) - 1u, t0, match, [&](uint32_t p, uint32_t piece, uint32_t mk) {
         match[p][piece] = (uint16_t)mk;
         found |= 1u << p;
     });
@@ -942,13 +947,17 @@ static cudaError_t launch_search_np(const SearchArgs &a, cudaStream_t st) {
         if (a.n_tiles <= kSearchFinishTiles) {
             SearchArgs r = a;
             r.overflow_list = nullptr;  // the flags are enough
-            search_stage_kernel<NP><<<a.n_tiles, SR_THREADS, 0, st>>>(r); OL_LAUNCHED();
+            search_stage_kernel<NP, false><<<a.n_tiles, SR_THREADS, 0, st>>>(r); OL_LAUNCHED();
             search_finish_kernel<NP><<<a.n_tiles, SR_THREADS, 0, st>>>(r); OL_LAUNCHED();
             return cudaGetLastError();
         }
         cudaError_t e0 = cudaMemsetAsync(a.overflow_n, 0, sizeof(uint32_t), st);
         if (e0 != cudaSuccess) return e0;
-        search_stage_kernel<NP><<<a.n_tiles, SR_THREADS, 0, st>>>(a); OL_LAUNCHED();
+        if ((a.len_class[2] | a.len_class[3] | a.len_class[4]) == 0) {
+            search_stage_kernel<NP, true><<<a.n_tiles, SR_THREADS, 0, st>>>(a); OL_LAUNCHED();
+        } else {
+            search_stage_kernel<NP, false><<<a.n_tiles, SR_THREADS, 0, st>>>(a); OL_LAUNCHED();
+        }
         cudaError_t e = launch_scan_columns(a.counts, a.bases, a.totals, a.n_tiles, a.np, a.ld, st);
         if (e != cudaSuccess) return e;
         search_copy_kernel<<<(a.n_tiles + SC_TILES - 1) / SC_TILES, SR_THREADS, 0, st>>>(a); OL_LAUNCHED();
