@@ -941,23 +941,30 @@ void search_add_pattern(SearchArgs &a, const uint8_t *host, const uint8_t *dev, 
 
 constexpr uint32_t kSearchWriteGrid = 512;  // blocks of the staged form's write pass
 
+// The stage pass, without the code for patterns that need more than the steps and
+// the anchors where there are none (filter_tile).
+template <uint32_t NP>
+static void launch_stage(const SearchArgs &a, cudaStream_t st) {
+    if ((a.len_class[2] | a.len_class[3] | a.len_class[4]) == 0) {
+        search_stage_kernel<NP, true><<<a.n_tiles, SR_THREADS, 0, st>>>(a); OL_LAUNCHED();
+    } else {
+        search_stage_kernel<NP, false><<<a.n_tiles, SR_THREADS, 0, st>>>(a); OL_LAUNCHED();
+    }
+}
+
 template <uint32_t NP>
 static cudaError_t launch_search_np(const SearchArgs &a, cudaStream_t st) {
     if (a.stage) {
         if (a.n_tiles <= kSearchFinishTiles) {
             SearchArgs r = a;
             r.overflow_list = nullptr;  // the flags are enough
-            search_stage_kernel<NP, false><<<a.n_tiles, SR_THREADS, 0, st>>>(r); OL_LAUNCHED();
+            launch_stage<NP>(r, st);
             search_finish_kernel<NP><<<a.n_tiles, SR_THREADS, 0, st>>>(r); OL_LAUNCHED();
             return cudaGetLastError();
         }
         cudaError_t e0 = cudaMemsetAsync(a.overflow_n, 0, sizeof(uint32_t), st);
         if (e0 != cudaSuccess) return e0;
-        if ((a.len_class[2] | a.len_class[3] | a.len_class[4]) == 0) {
-            search_stage_kernel<NP, true><<<a.n_tiles, SR_THREADS, 0, st>>>(a); OL_LAUNCHED();
-        } else {
-            search_stage_kernel<NP, false><<<a.n_tiles, SR_THREADS, 0, st>>>(a); OL_LAUNCHED();
-        }
+        launch_stage<NP>(a, st);
         cudaError_t e = launch_scan_columns(a.counts, a.bases, a.totals, a.n_tiles, a.np, a.ld, st);
         if (e != cudaSuccess) return e;
         search_copy_kernel<<<(a.n_tiles + SC_TILES - 1) / SC_TILES, SR_THREADS, 0, st>>>(a); OL_LAUNCHED();

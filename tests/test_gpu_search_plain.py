@@ -1,5 +1,5 @@
 """Sets of short and well-anchored patterns alone, which have a stage kernel of their
-own past 256 tiles, and the same sets with one pattern of each other kind, against
+own, on both sides of 256 tiles (where one launch finishes the search), and the same sets with one pattern of each other kind, against
 the oracle."""
 import numpy as np
 import pytest
